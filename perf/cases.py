@@ -6,7 +6,8 @@ Every case is one call pattern of a user's program, through the public entry poi
   step         a simulation restarted from a stored state, advanced by `steps` global time steps, state read back
   host_step    one step of a caller that keeps its particles in pinned host memory in the reference's default types
   stages       the force stages in place on a caller's device arrays (sphb_dataset_*), reference default types
-  ensemble     independent members of uneven size advanced together (parameter sweep), state read to the host
+  ensemble     independent members of uneven size uploaded from the device, advanced together (parameter sweep), and
+               read to the host
   gradient     kinetic energy after `steps` steps and its gradient with respect to u0 and alphamax
   block_steps  a simulation uploaded from the device and advanced by substeps of the block time-step propagator
   order        SFC keys, key sort, gather and octree on caller-owned arrays
@@ -66,7 +67,7 @@ def listed():
         {"name": "stages63_mixed", "kind": "stages", "side": 63, "precision": "mixed", "radius": 0.2},
         # a parameter sweep: uneven members, differing energies and gammas
         {"name": "ensemble16", "kind": "ensemble", "members": 16, "low": 20, "high": 48, "precision": "mixed",
-         "radius": 0.2, "steps": 40},
+         "radius": 0.2, "steps": 30},
         # gradients of a run (forward, checkpoints, recorded replay, adjoint)
         {"name": "gradient48_mixed", "kind": "gradient", "side": 48, "precision": "mixed", "steps": 20, "every": 5,
          "radius": 0.2},
@@ -210,7 +211,11 @@ def prepare(case, seed):
                 "leaves": torch.zeros(cap, dtype=torch.int64, device="cuda"),
                 "counts": torch.zeros(cap, dtype=torch.int32, device="cuda")}
     if kind == "ensemble":
-        return {"case": case, "ens": Ensemble(members(case, seed), case["precision"])}
+        ics = members(case, seed)
+        start = [([torch.from_numpy(np.ascontiguousarray(ic[f])).cuda() for f in CONSERVED_FIELDS],
+                  torch.from_numpy(ic["id"].astype(np.int64)).cuda()) for ic in ics]
+        tables = [(C.c_void_p * len(fields))(*[a.data_ptr() for a in fields]) for fields, _ in start]
+        return {"case": case, "ens": Ensemble(ics, case["precision"]), "start": start, "tables": tables}
     ic = initial(case, seed)
     if kind == "gradient":
         run = AdjointRun(ic, case["precision"], dt=ic["params"]["minDt"], steps=case["steps"], checkpoint_every=case["every"])
@@ -296,6 +301,9 @@ def run(state):
         return out
     if kind == "ensemble":
         ens = state["ens"]
+        for k, (table, (_, ids)) in enumerate(zip(state["tables"], state["start"])):
+            L.check(ens.lib.sphb_ensemble_upload(ens.h, k, table, L.ptr(ids), 1), "ensemble_upload")
+        L.check(ens.lib.sphb_ensemble_initial_sync(ens.h), "ensemble_initial_sync")
         ens.step(case["steps"])
         return {f: np.concatenate([ens.get(k, f) for k in range(ens.num)])
                 for f in ("x", "y", "z", "vx", "vy", "vz", "temp", "h")}
@@ -364,11 +372,16 @@ def work(case):
 
 
 def tolerance(case):
+    """About four times what the mixed and the all-double form of the same case differ by (1e-6 to 9e-6 for most
+    outputs, 4e-5 with AV cleaning, whose limiter divides nearly cancelling sums, and after the ensemble's many steps;
+    single particles more, where a neighbour count or a switch falls the other way)."""
     if case["kind"] == "order":
         return "exact"
     if case["precision"] == "fp64":
-        return {"rel": 1e-8, "max": 1e-4}
-    return {"rel": 2e-4, "max": 0.5}
+        return {"rel": 1e-9, "max": 1e-6}
+    if case.get("av_clean") or case["kind"] == "ensemble":
+        return {"rel": 1.5e-4, "max": 0.03}
+    return {"rel": 4e-5, "max": 5e-3}
 
 
 # -------------------------------------------------------------------------------------------------------------------
