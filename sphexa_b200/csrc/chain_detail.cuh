@@ -68,6 +68,19 @@ __device__ __forceinline__ float fdiv(float a, float b) { return __fdividef(a, b
 template<class T>
 __device__ __forceinline__ T tableLookup(const T* __restrict__ table, T v)
 {
+    if constexpr (sizeof(T) == 8)
+    {
+        // FP64: the interval and the position in it from one addition of 1.5 * 2^52 (its low word is the rounded
+        // integer), instead of two conversions between FP64 and integers, which run at a quarter of the FP64 rate
+        constexpr double kMagic = 6755399441055744.0;
+        double u = v * (0.5 * (kTableSize - 1));
+        if (!(u < double(kTableSize - 1))) { return 0.0; } // v >= 2, or not a number (coincident particles)
+        double t  = (u - 0.5) + kMagic;
+        int idx   = __double2loint(t);
+        double t0 = __ldg(table + idx);
+        double t1 = __ldg(table + idx + 1);
+        return t0 + (t1 - t0) * (u - (t - kMagic));
+    }
     constexpr int numIntervals = kTableSize - 1;
     constexpr T dx             = T(2.0) / numIntervals;
     constexpr T invDx          = T(1) / dx;
@@ -223,7 +236,11 @@ __device__ __forceinline__ Sep<double> separation(const Pos<double>& pi, const P
                                                   const DevBox& box, const HydroConsts<double>&)
 {
     double rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z;
-    shiftPbc(rx, ry, rz, r, box);
+    // the high words order as the magnitudes do, so a component can exceed r only if its high word reaches that of r:
+    // the six FP64 comparisons of the shift run only for such pairs (across the box, or at the edge of the sphere)
+    int top = max(max(__double2hiint(rx) & 0x7fffffff, __double2hiint(ry) & 0x7fffffff),
+                  __double2hiint(rz) & 0x7fffffff);
+    if (top >= __double2hiint(r)) { shiftPbc(rx, ry, rz, r, box); }
     return {rx, ry, rz};
 }
 

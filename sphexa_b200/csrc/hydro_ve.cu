@@ -3,8 +3,9 @@
 // neighbour lists are read slot-major (one coalesced line per slot). Each J-loop walks the list in stored (ascending)
 // order, like the reference CPU loops, and reads neighbour data through the packed records of hydro.cuh.
 //
-// T = double: the plain FP64 drop-in. Positions are FP64, the periodic shift is the reference's, sums run in list
-// order with the reference's expression order, so results differ from the reference CPU only by FMA contraction.
+// T = double: the plain FP64 drop-in. Positions are FP64, the periodic shift is the reference's and sums run in list
+// order. The pair terms are the reference's up to algebra that keeps FP64 rounding (a reciprocal for a division, a
+// constant factor taken out of a sum), so results differ from the reference CPU by rounding, 1e-15 of a force.
 //
 // T = float: the mixed form. Pair separations come from 32-bit fixed-point coordinates (exact integer differences,
 // periodic wrap by overflow; one unit = L / 2^32), all pair arithmetic is FP32, the kernel W is a degree-12
@@ -193,173 +194,24 @@ __global__ void packVelocityKernel(size_t n, const double* __restrict__ vx, cons
     hrec[i].vz = T(vz[i]);
 }
 
-// ---------------------------------------------------------------------------------------------------------------
-// IAD (sph/include/sph/hydro_ve/iad_kern.hpp:43-110) then divv/curlv with the particle's own c_ij
-// (sph/include/sph/hydro_ve/divv_curlv_kern.hpp:43-123); also the running max of divv for the rho time step.
-// ---------------------------------------------------------------------------------------------------------------
 template<class T>
 __device__ __forceinline__ int expOf(T v)
 {
     return v == T(0) ? 0 : ilogb(v);
 }
 
-template<class T, int kMode>
-__global__ void __launch_bounds__(kChainMaxThreads) iadDivvCurlvKernel(ChainArrays<T> a, HydroConsts<T> k, DevBox box)
-{
-    Target t;
-    bool valid     = chainTarget<kMode>(a, k.ngmax, t);
-    double divvOut = -INFINITY;
-    if (valid)
-    {
-        Pos<T> pi  = posOf(a, t.i);
-        double hiD = a.h[t.i];
-        T hi       = T(hiD);
-        T hiInv    = T(1) / hi;
-
-        BlockSum<T> s11, s12, s13, s22, s23, s33;
-        for (unsigned q0 = 0; q0 < t.count; q0 += kNbChunk)
-        {
-            uint32_t js[kNbChunk];
-            loadChunk(a.nidx, t, t.ngPad, q0, js);
-            unsigned qn = min(kNbChunk, t.count - q0);
-#pragma unroll
-            for (unsigned q = 0; q < kNbChunk; ++q)
-            {
-                if (q >= qn) { break; }
-                uint32_t j = js[q];
-                Pos<T> pj      = posOf(a, j);
-                HydroRec<T> hj = loadHydro(a.hrec + j);
-                Sep<T> r       = separation(pi, pj, 2.0 * hiD, box, k);
-                T dist         = sqrt(r.rx * r.rx + r.ry * r.ry + r.rz * r.rz);
-                T w            = kernelW(a.wh, k, dist * hiInv);
-                T voljW        = hj.vol * w;
-                s11.add(r.rx * r.rx * voljW);
-                s12.add(r.rx * r.ry * voljW);
-                s13.add(r.rx * r.rz * voljW);
-                s22.add(r.ry * r.ry * voljW);
-                s23.add(r.ry * r.rz * voljW);
-                s33.add(r.rz * r.rz * voljW);
-            }
-            s11.flush();
-            s12.flush();
-            s13.flush();
-            s22.flush();
-            s23.flush();
-            s33.flush();
-        }
-        T tau11 = s11.get(), tau12 = s12.get(), tau13 = s13.get();
-        T tau22 = s22.get(), tau23 = s23.get(), tau33 = s33.get();
-        int expSum = expOf(tau11) + expOf(tau12) + expOf(tau13) + expOf(tau22) + expOf(tau23) + expOf(tau33);
-        T norm     = ldexp(T(1), -expSum / 6);
-        tau11 *= norm;
-        tau12 *= norm;
-        tau13 *= norm;
-        tau22 *= norm;
-        tau23 *= norm;
-        tau33 *= norm;
-        T det = tau11 * tau22 * tau33 + T(2) * tau12 * tau23 * tau13 - tau11 * tau23 * tau23 - tau22 * tau13 * tau13 -
-                tau33 * tau12 * tau12;
-        T factor = norm * (hi * hi * hi) / (det * k.K);
-        if (isnan(factor) && t.count == 0) { factor = T(0); }
-        T c11i = (tau22 * tau33 - tau23 * tau23) * factor;
-        T c12i = (tau13 * tau23 - tau33 * tau12) * factor;
-        T c13i = (tau12 * tau23 - tau22 * tau13) * factor;
-        T c22i = (tau11 * tau33 - tau13 * tau13) * factor;
-        T c23i = (tau13 * tau12 - tau11 * tau23) * factor;
-        T c33i = (tau11 * tau22 - tau12 * tau12) * factor;
-
-        HydroRec<T> hrI = a.hrec[t.i];
-        T vxi = hrI.vx, vyi = hrI.vy, vzi = hrI.vz;
-        T kxi = a.kx[t.i];
-        BlockSum<T> dVxx, dVxy, dVxz, dVyx, dVyy, dVyz, dVzx, dVzy, dVzz;
-        for (unsigned q0 = 0; q0 < t.count; q0 += kNbChunk)
-        {
-            uint32_t js[kNbChunk];
-            loadChunk(a.nidx, t, t.ngPad, q0, js);
-            unsigned qn = min(kNbChunk, t.count - q0);
-#pragma unroll
-            for (unsigned q = 0; q < kNbChunk; ++q)
-            {
-                if (q >= qn) { break; }
-                uint32_t j = js[q];
-                Pos<T> pj      = posOf(a, j);
-                HydroRec<T> hj = loadHydro(a.hrec + j);
-                Sep<T> r       = separation(pi, pj, 2.0 * hiD, box, k);
-                T dist         = sqrt(r.rx * r.rx + r.ry * r.ry + r.rz * r.rz);
-                T Wi           = kernelW(a.wh, k, dist * hiInv);
-                T tA0          = -(c11i * r.rx + c12i * r.ry + c13i * r.rz) * Wi;
-                T tA1          = -(c12i * r.rx + c22i * r.ry + c23i * r.rz) * Wi;
-                T tA2          = -(c13i * r.rx + c23i * r.ry + c33i * r.rz) * Wi;
-                T fx           = (hj.vx - vxi) * hj.xm;
-                T fy           = (hj.vy - vyi) * hj.xm;
-                T fz           = (hj.vz - vzi) * hj.xm;
-                dVxx.add(fx * tA0);
-                dVxy.add(fx * tA1);
-                dVxz.add(fx * tA2);
-                dVyx.add(fy * tA0);
-                dVyy.add(fy * tA1);
-                dVyz.add(fy * tA2);
-                dVzx.add(fz * tA0);
-                dVzy.add(fz * tA1);
-                dVzz.add(fz * tA2);
-            }
-            dVxx.flush();
-            dVxy.flush();
-            dVxz.flush();
-            dVyx.flush();
-            dVyy.flush();
-            dVyz.flush();
-            dVzx.flush();
-            dVzy.flush();
-            dVzz.flush();
-        }
-        T hiInv3 = hiInv * hiInv * hiInv;
-        T normKx = k.K * hiInv3 / kxi;
-        T divv   = normKx * (dVxx.get() + dVyy.get() + dVzz.get());
-        T cx     = dVzy.get() - dVyz.get();
-        T cy     = dVxz.get() - dVzx.get();
-        T cz     = dVyx.get() - dVxy.get();
-        T curlv  = normKx * sqrt(cx * cx + cy * cy + cz * cz);
-        if constexpr (kMode & kModeAvClean)
-        {
-            DVRec<T> g{{normKx * dVxx.get(), normKx * (dVxy.get() + dVyx.get()), normKx * (dVxz.get() + dVzx.get()),
-                        normKx * dVyy.get(), normKx * (dVyz.get() + dVzy.get()), normKx * dVzz.get()},
-                       T(0),
-                       T(0)};
-            a.dvrec[t.i] = g;
-#pragma unroll
-            for (int q = 0; q < 6; ++q)
-            {
-                a.dv[q][t.i] = g.dv[q];
-            }
-        }
-
-        a.cij[0][t.i] = c11i;
-        a.cij[1][t.i] = c12i;
-        a.cij[2][t.i] = c13i;
-        a.cij[3][t.i] = c22i;
-        a.cij[4][t.i] = c23i;
-        a.cij[5][t.i] = c33i;
-        a.divv[t.i]   = divv;
-        a.curlv[t.i]  = curlv;
-        a.grec[t.i]   = GradRec<T>{c11i, c12i, c13i, c22i, c23i, c33i, divv, T(a.alpha[t.i])};
-        a.avrec[t.i]  = AVRec<T>{hrI.vx, hrI.vy, hrI.vz, hrI.c, hrI.vol, divv, T(0), T(0)};
-        divvOut       = double(divv);
-    }
-    reduceOrdered<true, (kMode & kModeBatch) != 0>(divvOut, a.n, a.reduce + 0, a.batch, 0);
-}
-
-/*! FP32 IAD + divv/curlv in one pass over the list. The divv/curlv loop of the reference sums, per pair,
+/*! IAD + divv/curlv (sph/include/sph/hydro_ve/iad_kern.hpp:43-110, then divv_curlv_kern.hpp:43-123 with the
+ *  particle's own c_ij) in one pass over the list; also the running max of divv for the rho time step. The divv/curlv loop of the reference sums, per pair,
  *  f_a tA_b with f = (v_j - v_i) xm_j and tA = -(C_i r) W, i.e. dV_ab = -sum_c C_bc M_ac with
  *  M_ac = sum_j f_a r_c W: M is accumulated in the same pass as tau, and C_i, known only after the pass, is applied
  *  to the nine sums at the end. Same quantities, one gather of each neighbour instead of two. */
-// at most 80 registers (three 256-thread blocks per SM), as MomentumEnergy: measured 1.04 -> 0.95 ms at 128^3 against
-// 87 registers
-template<int kMode>
-__global__ void __launch_bounds__(kChainMaxThreads, 3) iadDivvCurlvFusedKernel(ChainArrays<float> a,
-                                                                              HydroConsts<float> k, DevBox box)
+// FP32: at most 80 registers (three 256-thread blocks per SM), as MomentumEnergy: measured 1.04 -> 0.95 ms at 128^3
+// against 87 registers. FP64 ran the two list passes of the reference before, bound by its FP64 pipe and the second
+// gather: 2.10 -> 1.16 ms at 101^3.
+template<class T, int kMode>
+__global__ void __launch_bounds__(kChainMaxThreads, sizeof(T) == 4 ? 3 : 0)
+    iadDivvCurlvFusedKernel(ChainArrays<T> a, HydroConsts<T> k, DevBox box)
 {
-    using T = float;
     Target t;
     bool valid     = chainTarget<kMode>(a, k.ngmax, t);
     double divvOut = -INFINITY;
@@ -541,44 +393,34 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? kAvMaxThreads : kChainMaxThre
             Sep<T> r       = separation(pi, pj, 2.0 * hiD, box, k);
             T r2           = r.rx * r.rx + r.ry * r.ry + r.rz * r.rz;
             T rv           = r.rx * (hr.vx - hj.vx) + r.ry * (hr.vy - hj.vy) + r.rz * (hr.vz - hj.vz);
-            T vsig         = T(0);
+            // 1/r from one rsqrt: 3 r.v / r without a division, and in FP64 r itself for the kernel's table
+            T vsig = T(0);
+            [[maybe_unused]] T rinv = T(0);
+            if constexpr (sizeof(T) == 8) { rinv = rsqrt(r2); }
             if (rv < T(0))
             {
-                // FP32: 3 r.v / r with one rsqrt; FP64: the reference's division
-                if constexpr (sizeof(T) == 4) { vsig = ci + hj.c - T(3) * rv * rsqrtf(r2); }
-                else { vsig = ci + hj.c - fdiv(T(3) * rv, T(sqrt(r2))); }
+                if constexpr (sizeof(T) == 4) { rinv = rsqrtf(r2); }
+                vsig = ci + hj.c - T(3) * rv * rinv;
             }
             if constexpr (kMode & kModeTape)
             {
                 if (!(vijsignalI > vsig)) { vsigJ = int(j); }
             }
             vijsignalI = vijsignalI > vsig ? vijsignalI : vsig;
-            T Wi       = KhiInv3 * kernelWr2(a.wh, k, r2, hiInv, hh);
-            T fac      = hj.vol * (divvI - divvJ);
-            if constexpr (sizeof(T) == 4)
-            {
-                // FP32: sum fac W r and apply -C_i once after the loop (the same vector, 9 FMAs less per pair)
-                T sw = fac * Wi;
-                gx.add(sw * r.rx);
-                gy.add(sw * r.ry);
-                gz.add(sw * r.rz);
-            }
-            else
-            {
-                T tA1 = -(gr.c11 * r.rx + gr.c12 * r.ry + gr.c13 * r.rz) * Wi;
-                T tA2 = -(gr.c12 * r.rx + gr.c22 * r.ry + gr.c23 * r.rz) * Wi;
-                T tA3 = -(gr.c13 * r.rx + gr.c23 * r.ry + gr.c33 * r.rz) * Wi;
-                gx.add(fac * tA1);
-                gy.add(fac * tA2);
-                gz.add(fac * tA3);
-            }
+            T W;
+            if constexpr (sizeof(T) == 4) { W = kernelWr2(a.wh, k, r2, hiInv, hh); }
+            else { W = kernelW(a.wh, k, r2 * rinv * hiInv); }
+            // sum fac W r and apply -C_i once after the loop (the same vector, 9 FMAs less per pair)
+            T sw = hj.vol * (divvI - divvJ) * (KhiInv3 * W);
+            gx.add(sw * r.rx);
+            gy.add(sw * r.ry);
+            gz.add(sw * r.rz);
         }
         gx.flush();
         gy.flush();
         gz.flush();
     }
     T gdx = gx.get(), gdy = gy.get(), gdz = gz.get();
-    if constexpr (sizeof(T) == 4)
     {
         T sx = gdx, sy = gdy, sz = gdz;
         gdx  = -(gr.c11 * sx + gr.c12 * sy + gr.c13 * sz);
@@ -619,6 +461,9 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? kAvMaxThreads : kChainMaxThre
 // artificial_viscosity sph/include/sph/kernels.hpp:71-85) with the Courant time step per particle
 // (tsKCourant, kernels.hpp:10-17) reduced to the minimum.
 // ---------------------------------------------------------------------------------------------------------------
+// FP64 is bound by its FP64 pipe. It ran five divisions and a square root per pair (and four powers on the Atwood
+// ramp); with one rsqrt, the densities compared as |rho_i vol_j - m_j| and the loop rolled it takes 2.12 instead of
+// 3.98 ms at 101^3, the result unchanged to 4e-15.
 // FP32 without AV cleaning: at most 80 registers (three 256-thread blocks per SM) keeps more warps resident for the
 // gathers; measured 2.11 -> 2.05 ms at 128^3 against 96 registers (the AV-cleaning form would spill)
 template<class T, int kMode>
@@ -752,16 +597,13 @@ __global__ void __launch_bounds__(kChainMaxThreads, (sizeof(T) == 4 && !(kMode &
                 GradRec<T> gj  = loadGrad(a.grec + j);
                 Sep<T> r       = separation(pi, pj, 2.0 * hiD, box, k);
                 T r2           = r.rx * r.rx + r.ry * r.ry + r.rz * r.rz;
-                // FP32: 1/r from one rsqrt (r and w_ij = r.v / r without a square root or a division), m_j / rho_j as
-                // vol_j, and the Atwood thresholds compared without a division (1.68 -> 1.58 ms at 128^3; the errors
-                // against FP64 unchanged)
-                T rinv, dist;
-                if constexpr (sizeof(T) == 4)
-                {
-                    rinv = rsqrtf(r2);
-                    dist = r2 * rinv;
-                }
-                else { dist = sqrt(r2); }
+                // 1/r from one rsqrt (r and w_ij = r.v / r without a square root or a division), m_j / rho_j as
+                // vol_j, and the Atwood thresholds compared without a division (FP32: 1.68 -> 1.58 ms at 128^3; the
+                // errors against FP64 unchanged)
+                T rinv;
+                if constexpr (sizeof(T) == 4) { rinv = rsqrtf(r2); }
+                else { rinv = rsqrt(r2); }
+                T dist         = r2 * rinv;
                 T vxij         = hr.vx - hj.vx;
                 T vyij         = hr.vy - hj.vy;
                 T vzij         = hr.vz - hj.vz;
@@ -781,7 +623,6 @@ __global__ void __launch_bounds__(kChainMaxThreads, (sizeof(T) == 4 && !(kMode &
                 T mj     = T(pj.m);
                 T cj     = hj.c;
                 T xmassj = hj.xm;
-                T rhoj   = fdiv(mj, hj.vol);
 
                 T rv   = r.rx * vxij + r.ry * vyij + r.rz * vzij;
                 if constexpr (kMode & kModeAvClean)
@@ -790,9 +631,7 @@ __global__ void __launch_bounds__(kChainMaxThreads, (sizeof(T) == 4 && !(kMode &
                     loadDV(a.dvrec + j, gradVj);
                     rv += avRvCorrection(r.rx, r.ry, r.rz, v1 < v2 ? v1 : v2, etaCrit, gradVi, gradVj);
                 }
-                T wij;
-                if constexpr (sizeof(T) == 4) { wij = rv * rinv; }
-                else { wij = fdiv(rv, dist); }
+                T wij  = rv * rinv;
                 T visc = T(0);
                 if (wij < T(0))
                 {
@@ -802,14 +641,16 @@ __global__ void __launch_bounds__(kChainMaxThreads, (sizeof(T) == 4 && !(kMode &
                 T vijsignal = T(0.5) * (ci + cj) - T(2) * wij;
                 maxvsignalI = vijsignal > maxvsignalI ? vijsignal : maxvsignalI;
 
+                // |rho_i - rho_j| against A (rho_i + rho_j), both times vol_j = m_j / rho_j
                 T aMom, bMom;
-                T dRho = fabs(rhoi - rhoj), sRho = rhoi + rhoj;
-                if (sizeof(T) == 4 ? dRho < k.Atmin * sRho : fdiv(dRho, sRho) < k.Atmin)
+                T rhoiVol = rhoi * hj.vol;
+                T dRho = fabs(rhoiVol - mj), sRho = rhoiVol + mj;
+                if (dRho < k.Atmin * sRho)
                 {
                     aMom = xmassi * xmassi;
                     bMom = xmassj * xmassj;
                 }
-                else if (sizeof(T) == 4 ? dRho > k.Atmax * sRho : fdiv(dRho, sRho) > k.Atmax)
+                else if (dRho > k.Atmax * sRho)
                 {
                     aMom = xmassi * xmassj;
                     bMom = aMom;
@@ -825,22 +666,16 @@ __global__ void __launch_bounds__(kChainMaxThreads, (sizeof(T) == 4 && !(kMode &
                     }
                     else
                     {
-                        aMom = pow(xmassi, T(2) - sigma) * pow(xmassj, sigma);
-                        bMom = pow(xmassj, T(2) - sigma) * pow(xmassi, sigma);
+                        // xm_i^(2-s) xm_j^s = xm_i^2 q and xm_j^(2-s) xm_i^s = xm_j^2 / q with q = (xm_j / xm_i)^s:
+                        // one logarithm and one exponential instead of four powers
+                        T q  = exp(sigma * log(xmassj / xmassi));
+                        aMom = xmassi * xmassi * q;
+                        bMom = xmassj * xmassj / q;
                     }
                 }
 
-                T aVisc, bVisc;
-                if constexpr (sizeof(T) == 4)
-                {
-                    aVisc = mj * invRhoi * visc;
-                    bVisc = hj.vol * visc;
-                }
-                else
-                {
-                    aVisc = fdiv(mj, rhoi) * visc;
-                    bVisc = fdiv(mj, rhoj) * visc;
-                }
+                T aVisc  = mj * invRhoi * visc;
+                T bVisc  = hj.vol * visc;
                 T aViscX = T(0.5) * (aVisc * tA1i + bVisc * tA1j);
                 T aViscY = T(0.5) * (aVisc * tA2i + bVisc * tA2j);
                 T aViscZ = T(0.5) * (aVisc * tA3i + bVisc * tA3j);
@@ -858,25 +693,12 @@ __global__ void __launch_bounds__(kChainMaxThreads, (sizeof(T) == 4 && !(kMode &
             uint32_t js[kNbChunk];
             loadChunk(a.nidx, t, t.ngPad, q0, js);
             unsigned qn = min(kNbChunk, t.count - q0);
-            if constexpr (sizeof(T) == 4)
-            {
-                // one pair per iteration: the unrolled 8-pair body overflowed the instruction cache (2.04 -> 1.71 ms
-                // at 128^3); unrolled by 2 or 4 it ran slower too (1.59 against 1.48 ms)
+            // one pair per iteration: the unrolled 8-pair body overflowed the instruction cache (FP32 2.04 -> 1.71 ms
+            // at 128^3; unrolled by 2 or 4 it ran slower too, 1.59 against 1.48 ms; FP64 2.23 -> 2.12 ms at 101^3)
 #pragma unroll 1
-                for (unsigned q = 0; q < qn; ++q)
-                {
-                    pairTerm(popChunk(js));
-                }
-            }
-            else
+            for (unsigned q = 0; q < qn; ++q)
             {
-                // bound by the FP64 pipe, the unrolled body is faster here (5.31 ms against 6.02 rolled)
-#pragma unroll
-                for (unsigned q = 0; q < kNbChunk; ++q)
-                {
-                    if (q >= qn) { break; }
-                    pairTerm(js[q]);
-                }
+                pairTerm(popChunk(js));
             }
             momX.flush();
             momY.flush();
@@ -1004,27 +826,7 @@ template<class T>
 int launchIadDivvCurlv(const ChainArrays<T>& a, const HydroConsts<T>& k, const DevBox& box, cudaStream_t s)
 {
     if (a.n == 0 || (a.groupList && a.numListed == 0)) { return kOk; }
-    if constexpr (sizeof(T) == 4)
-    {
-        switch (chainModeAv(a))
-        {
-        case 0: iadDivvCurlvFusedKernel<0><<<chainBlocks(a), a.threads, 0, s>>>(a, k, box); break;
-        case kModeTape: iadDivvCurlvFusedKernel<kModeTape><<<chainBlocks(a), a.threads, 0, s>>>(a, k, box); break;
-        case kModeBatch: iadDivvCurlvFusedKernel<kModeBatch><<<chainBlocks(a), a.threads, 0, s>>>(a, k, box); break;
-        case kModeList: iadDivvCurlvFusedKernel<kModeList><<<chainBlocks(a), a.threads, 0, s>>>(a, k, box); break;
-        case kModeAvClean:
-            iadDivvCurlvFusedKernel<kModeAvClean><<<chainBlocks(a), a.threads, 0, s>>>(a, k, box);
-            break;
-        case kModeAvClean | kModeBatch:
-            iadDivvCurlvFusedKernel<kModeAvClean | kModeBatch><<<chainBlocks(a), a.threads, 0, s>>>(a, k, box);
-            break;
-        case kModeAvClean | kModeList:
-            iadDivvCurlvFusedKernel<kModeAvClean | kModeList><<<chainBlocks(a), a.threads, 0, s>>>(a, k, box);
-            break;
-        default: return kErrArg;
-        }
-    }
-    else { SPHB_DISPATCH_AV(iadDivvCurlvKernel, a, k, box) }
+    SPHB_DISPATCH_AV(iadDivvCurlvFusedKernel, a, k, box)
     countLaunch();
     SPHB_CUDA_TRY(cudaGetLastError());
     return kOk;
