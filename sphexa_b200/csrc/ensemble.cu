@@ -722,7 +722,7 @@ int searchBatchedSkin(sphb_ensemble& e, const NeighborParams& np)
     SPHB_TRY(skinDecide(ctl, st));
     SPHB_TRY(findNeighbors(e.f[0].data(), e.f[1].data(), e.f[2].data(), e.pos.data(), e.f[3].data(), n, dummy, e.box,
                            np, e.nidx.data(), e.nc.data(), e.status.data(), st, e.views.data(), e.inst.data(), mode,
-                           (1u << kSkinModeTree) | (1u << kSkinModeBuild)));
+                           1u << kSkinModeTree));
     SkinLists sl{e.skinRows.data(), e.skinCount.data(), e.skinRadius.data(), e.skinCap, e.skinDist.data()};
     SPHB_TRY(buildSkinLists(e.f[0].data(), e.f[1].data(), e.f[2].data(), e.pos.data(), e.f[3].data(), n, dummy, e.box,
                             np, e.p.nb_skin, sl, e.status.data(), st, e.views.data(), e.inst.data(), mode,
@@ -763,7 +763,7 @@ int searchBatchedSkin(sphb_ensemble& e, const NeighborParams& np)
     a.inst         = e.inst.data();
     a.gate         = mode;
     SPHB_TRY(checkSkinGroups(a, st));
-    // the deferred counts stay zero unless the mode is the refilter, and then the listed searches see them
+    // the deferred counts stay zero in a step of tree searches, else the listed searches see them
     SPHB_TRY(findNeighborsListed(e.f[0].data(), e.f[1].data(), e.f[2].data(), e.pos.data(), e.f[3].data(), n, dummy,
                                  e.box, np, e.nidx.data(), e.nc.data(), e.status.data(), a.worklist, a.numWorklist, st,
                                  e.views.data(), e.inst.data()));

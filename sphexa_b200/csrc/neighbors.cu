@@ -239,7 +239,13 @@ __global__ void __launch_bounds__(kNbThreads, 8) findNeighborsKernel(const doubl
         // this lane's chunk buffer and its store to the chunked list layout (nidxAt)
         uint32_t* chunk     = &sh.nbuf[warp][0][lane];
         uint16_t* dchunk    = &sh.dbuf[warp][0][lane];
-        const double qScale = kSkinDistUnits / r; // skin rows: distance -> units of R / kSkinDistUnits
+        // skin rows: distance -> units of R / kSkinDistUnits. The FP32 distance of the pair serves where it is known
+        // to kSkinDistSlack units: both coordinates are rounded once relative to the group centre, 2^-24 reach each,
+        // and the FP32 arithmetic adds at most 4 * 2^-24 R, together 2^-24 (3.5 reach + 4 R) < 1.3e-6 R = 0.084 units
+        // for reach <= 5 R (a compact group reaches 2 to 3 R)
+        const double qScale  = kSkinDistUnits / r;
+        const float qScaleF  = float(qScale);
+        const bool exactDist = wrapTest || reach > 5.f * twoH;
         auto storeChunk = [&](unsigned c) {
             uint32_t* dst = outList + nidxAt(group, ngPad, c * kNbChunk, lane);
             if constexpr (kSkin)
@@ -308,10 +314,19 @@ __global__ void __launch_bounds__(kNbThreads, 8) findNeighborsKernel(const doubl
                 {
                     if constexpr (kSkin)
                     {
-                        // the build distance, from the reference's FP64 expression, for the refilter's bounds
-                        double4 pj = ldPos(pos + j);
-                        double q   = rint(sqrt(exactDistSq(pj.x, pj.y, pj.z, xi, yi, zi, box)) * qScale);
-                        dchunk[(count % kNbChunk) * kWarp] = uint16_t(fmin(q, kSkinDistUnits));
+                        // the build distance, for the refilter's bounds
+                        if (exactDist)
+                        {
+                            double4 pj = ldPos(pos + j);
+                            double q   = rint(sqrt(exactDistSq(pj.x, pj.y, pj.z, xi, yi, zi, box)) * qScale);
+                            dchunk[(count % kNbChunk) * kWarp] = uint16_t(fmin(q, kSkinDistUnits));
+                        }
+                        else
+                        {
+                            float dx = sh.cx[warp][k] - rix, dy = sh.cy[warp][k] - riy, dz = sh.cz[warp][k] - riz;
+                            float q  = rintf(sqrtf(fmaf(dz, dz, fmaf(dy, dy, dx * dx))) * qScaleF);
+                            dchunk[(count % kNbChunk) * kWarp] = uint16_t(fminf(q, float(kSkinDistUnits)));
+                        }
                     }
                     chunk[(count % kNbChunk) * kWarp] = uint32_t(j);
                     if (count % kNbChunk == kNbChunk - 1) { storeChunk(count / kNbChunk); }

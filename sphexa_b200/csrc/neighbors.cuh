@@ -83,7 +83,7 @@ __device__ inline double searchRadiusSq(double h) { return __dmul_rn(__dmul_rn(4
  *  R_i = 2 h_i (1 + skin) when the lists were built, in ascending index order, at most `cap` of them (chunked like
  *  the neighbour lists, with `cap` as the padded width). count[i] is the number found, which can exceed cap: the row
  *  is then incomplete and never used. dist holds, beside each entry, its distance at the build in units of
- *  R_i / kSkinDistUnits, rounded to nearest (16 bits, same chunked layout). */
+ *  R_i / kSkinDistUnits (16 bits, same chunked layout), within kSkinDistSlack units of the FP64 distance. */
 struct SkinLists
 {
     uint32_t* rows;
@@ -95,6 +95,10 @@ struct SkinLists
 
 //! units of the quantised build distance per R_i
 constexpr double kSkinDistUnits = 65535.0;
+
+/*! bound of |stored distance - FP64 distance| in those units: half a unit of rounding, 0.084 from the FP32 distance
+ *  of the build's pair test (see findNeighborsKernel), 0.01 from its scaling by R_i in FP32 */
+constexpr double kSkinDistSlack = 0.61;
 
 /*! Search all particles (x, y, z and the same coordinates packed as pos = (x, y, z, m)): updates h where the count
  *  left [ng0/4, ngmax+1], writes nc (count incl. self) and lists. With gate set, the launch does nothing unless bit
@@ -147,14 +151,14 @@ struct SkinFilterArgs
     DevBox box;
     NeighborParams prm;
     const uint8_t* inst;   // an ensemble: instance per slot (kGhost: padding, skipped), else null
-    const unsigned* gate;  // if set: the launch runs only when *gate == kSkinModeFilter
+    const unsigned* gate;  // if set: the launch runs only when *gate is kSkinModeBuild or kSkinModeFilter
 };
 
 //! neighbour-stage modes of a simulation stepped without host reads (ensemble), chosen on the device
 enum SkinMode : unsigned
 {
     kSkinModeTree   = 0, // tree search of every group, no rows
-    kSkinModeBuild  = 1, // tree search of every group and a build of the rows
+    kSkinModeBuild  = 1, // a build of the rows by tree search, then the refilter of them
     kSkinModeFilter = 2  // refilter of the rows, tree search of the deferred groups
 };
 

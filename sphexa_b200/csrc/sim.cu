@@ -438,8 +438,10 @@ int searchNeighbors(sphb_sim& s)
     }
     if (rebuild)
     {
+        // The rows are built by the tree search at R_i and then refiltered like those of any other step, with zero
+        // displacements: one traversal instead of two. A group whose row overflows or whose h iterates out of its
+        // row is searched as a deferred group.
         SPHB_TRY(allocateSkin(s));
-        SPHB_TRY(treeSearch());
         SkinLists sl{s.skinRows.data(), s.skinCount.data(), s.skinRadius.data(), s.skinCap, s.skinDist.data()};
         SPHB_TRY(buildSkinLists(s.f[fX].data(), s.f[fY].data(), s.f[fZ].data(), s.pos.data(), s.f[fH].data(), s.n, tv,
                                 s.box, np, s.p.nb_skin, sl, s.status.data(), st));
@@ -451,19 +453,24 @@ int searchNeighbors(sphb_sim& s)
         s.skinAnyMoved     = false;
         s.skinAge          = 0;
         s.skinDeferredLast = 0;
+        ++s.searchStats[0];
         ++s.searchStats[1];
-        return kOk;
     }
-
-    ++s.skinAge;
-    ++s.searchStats[2];
-    s.skinFiltered = true;
+    else
+    {
+        ++s.skinAge;
+        ++s.searchStats[2];
+        s.skinFiltered = true; // the deferred counts of a build step say nothing about the rows' age: not read
+    }
     SPHB_CUDA_TRY(cudaMemsetAsync(s.skinGrid.data(), 0, size_t(kSkinGrid) * kSkinGrid * kSkinGrid * sizeof(unsigned),
                                   st));
     SPHB_CUDA_TRY(cudaMemsetAsync(s.skinWork.data(), 0, 2 * sizeof(unsigned), st));
     const uint32_t* buildOf = s.skinAnyMoved ? s.skinBuild.data() : nullptr;
-    SPHB_TRY(skinDisplacement(s.pos.data(), s.skinXb.data(), s.skinYb.data(), s.skinZb.data(), buildOf, s.n, s.box,
-                              s.skinGrid.data(), st));
+    if (!rebuild)
+    {
+        SPHB_TRY(skinDisplacement(s.pos.data(), s.skinXb.data(), s.skinYb.data(), s.skinZb.data(), buildOf, s.n, s.box,
+                                  s.skinGrid.data(), st));
+    }
     SkinFilterArgs a{};
     a.pos  = s.pos.data();
     a.posq = s.mixed ? s.posq.data() : nullptr;

@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(kFilterThreads) skinCheckKernel(SkinFilterArgs
     const int lane         = threadIdx.x & (kWarp - 1);
     const size_t numGroups = (a.n + kWarp - 1) / kWarp;
     const size_t group     = size_t(blockIdx.x) * kFilterWarps + warp;
-    if (group >= numGroups || (a.gate && __ldg(a.gate) != kSkinModeFilter)) { return; }
+    if (group >= numGroups || (a.gate && __ldg(a.gate) == kSkinModeTree)) { return; }
     const size_t i    = group * kWarp + lane;
     const bool valid  = i < a.n && !(a.inst && a.inst[i] == kGhost);
     double4 pi        = valid ? loadPos(a.pos + i) : make_double4(0, 0, 0, 0);
@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(kFilterThreads) skinFilterKernel(SkinFilterArg
     const int lane         = threadIdx.x & (kWarp - 1);
     const size_t numGroups = (a.n + kWarp - 1) / kWarp;
     const size_t group     = size_t(blockIdx.x) * kFilterWarps + warp;
-    if (group >= numGroups || (a.gate && __ldg(a.gate) != kSkinModeFilter)) { return; }
+    if (group >= numGroups || (a.gate && __ldg(a.gate) == kSkinModeTree)) { return; }
     const unsigned gD = __ldg(a.groupD + group);
     if (gD == kDeferred) { return; }
     const double D   = double(__uint_as_float(gD));
@@ -322,12 +322,12 @@ __global__ void __launch_bounds__(kFilterThreads) skinFilterKernel(SkinFilterArg
             const float r2lo = r2f * (1.f - band);
             const float r2hi = r2f * (1.f + band);
             // Most entries are decided from their quantised build distance q (units of Ri / kSkinDistUnits, the true
-            // build distance within (q +- 0.5) units): now |x_i - x_j| lies within d_i + D of it, so entries with
+            // build distance within (q +- kSkinDistSlack) units): now |x_i - x_j| is within d_i + D of it, so entries with
             // q <= qIn are surely inside 2 h_i and entries with q >= qOut surely outside, by a relative margin of
             // 1e-9 that covers the FP64 rounding of the exact test. Only the rest are gathered and tested.
             const double unit = Ri / kSkinDistUnits;
-            const double tIn  = (2.0 * hi * (1.0 - 1e-9) - di - D) / unit - 0.501;
-            const double tOut = (2.0 * hi * (1.0 + 1e-9) + di + D) / unit + 0.501;
+            const double tIn  = (2.0 * hi * (1.0 - 1e-9) - di - D) / unit - kSkinDistSlack - 0.001;
+            const double tOut = (2.0 * hi * (1.0 + 1e-9) + di + D) / unit + kSkinDistSlack + 0.001;
             const int qIn     = tIn > 0.0 ? int(ceil(tIn)) - 1 : -1;               // largest q < tIn
             const int qOut    = tOut < kSkinDistUnits ? int(floor(tOut)) + 1 : 65536; // smallest q > tOut
             count           = 0;
@@ -426,7 +426,8 @@ __global__ void __launch_bounds__(kFilterThreads) skinFilterKernel(SkinFilterArg
  *  in the previous step; rows rebuilt within three steps of the last build give way to 32 steps of tree searches). */
 __global__ void skinDecideKernel(unsigned* ctl)
 {
-    unsigned deferred = ctl[kCtlDeferredA] + ctl[kCtlDeferredB];
+    // a build step defers only rows that overflow and groups whose h iterated: no sign of the rows' age
+    unsigned deferred = ctl[kCtlMode] == kSkinModeBuild ? 0u : ctl[kCtlDeferredA] + ctl[kCtlDeferredB];
     ctl[kCtlDeferredTotal] += deferred;
     ctl[kCtlDeferredA] = 0;
     ctl[kCtlDeferredB] = 0;
