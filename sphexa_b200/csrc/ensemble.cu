@@ -500,13 +500,13 @@ int rebuildTrees(sphb_ensemble& e)
             while (!converged)
             {
                 SPHB_TRY(focusUpdateTree(f, g, e.ts, st, &converged));
-                SPHB_TRY(focusUpdateCounts(f, keys, nk, e.ts, st));
+                SPHB_TRY(focusUpdateCounts(f, keys, nk, st));
                 if (++guard > 100) { return kErrNotConverged; }
             }
             f.firstCall = false;
         }
         SPHB_TRY(focusUpdateTree(f, g, e.ts, st, &converged));
-        SPHB_TRY(focusUpdateCounts(f, keys, nk, e.ts, st));
+        SPHB_TRY(focusUpdateCounts(f, keys, nk, st));
         SPHB_TRY(computeGeoCenters(f.tree, e.box, st));
         SPHB_TRY(e.layouts[k]->reserve(size_t(f.numLeaves) + 1));
         TreeView tv;

@@ -10,7 +10,6 @@
 
 #include "octree.cuh"
 #include "sfc.cuh"
-#include "sort.cuh"
 
 namespace sphb
 {
@@ -51,53 +50,132 @@ __host__ __device__ inline unsigned octalDigitAt(uint64_t key, unsigned level)
 // linked octree construction
 // ---------------------------------------------------------------------------------------------------------------
 
-__global__ void internalCountKernel(const uint64_t* leaves, int numLeaves, int* cnt)
-{
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > numLeaves) { return; }
-    if (i == numLeaves)
-    {
-        cnt[i] = 0;
-        return;
-    }
-    uint64_t key   = leaves[i];
-    unsigned level = treeLevelOf(leaves[i + 1] - key);
-    unsigned a     = alignmentLevel(key);
-    cnt[i]         = level > a ? int(level - a) : 0;
-}
+// The node order is level-major, and within a level the nodes are in key order, which is the order of the leaves that
+// start them: leaf i starts one node on every level from the coarsest aligned with its key to its own. The position
+// of a node is therefore its level's first index plus the number of leaves before i that start a node of the level: a
+// count per level and block of leaves, one scan, and the positions. This replaces a radix sort of the prefixes (eight
+// passes and two host reads); with one scan launch per array and no scan for the layout, the sync takes 235 instead
+// of 300 us at 4,096 particles, 510 instead of 630 at 27,000, 945 instead of 1,110 at 128^3.
 
-__global__ void emitNodesKernel(const uint64_t* leaves, int numLeaves, int numInternal, const int* offsets,
-                                uint64_t* prefixes, uint32_t* ids)
+constexpr int kLevels       = int(kMaxLevel) + 1;
+constexpr int kLevelThreads = 256;
+constexpr int kLevelWarps   = kLevelThreads / 32;
+
+/*! the levels [a, b] of the nodes that leaf i starts (b: the leaf itself); a > b past the end and for a malformed
+ *  leaf array */
+__device__ __forceinline__ void startedLevels(const uint64_t* leaves, int numLeaves, int i, uint64_t* key, int* a, int* b)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    *a = 1;
+    *b = 0;
     if (i >= numLeaves) { return; }
-    uint64_t key   = leaves[i];
-    unsigned level = treeLevelOf(leaves[i + 1] - key);
-    unsigned a     = alignmentLevel(key);
-    prefixes[numInternal + i] = encodePrefix(key, level);
-    ids[numInternal + i]      = uint32_t(numInternal + i);
-    int off                   = offsets[i];
-    for (unsigned l = a; l < level && off < numInternal; ++l, ++off)
+    *key = leaves[i];
+    *b   = min(int(treeLevelOf(leaves[i + 1] - *key)), int(kMaxLevel));
+    *a   = min(int(alignmentLevel(*key)), *b);
+}
+
+//! counts[l * gridDim.x + block] = nodes of level l started by the block's leaves
+__global__ void __launch_bounds__(kLevelThreads) levelCountKernel(const uint64_t* leaves, int numLeaves, int* counts)
+{
+    __shared__ int sh[kLevels];
+    if (threadIdx.x < kLevels) { sh[threadIdx.x] = 0; }
+    __syncthreads();
+    uint64_t key;
+    int a, b;
+    startedLevels(leaves, numLeaves, blockIdx.x * kLevelThreads + threadIdx.x, &key, &a, &b);
+    for (int l = 0; l < kLevels; ++l)
     {
-        prefixes[off] = encodePrefix(key, l);
-        ids[off]      = uint32_t(off);
+        unsigned m = __ballot_sync(0xffffffffu, l >= a && l <= b);
+        if ((threadIdx.x & 31) == 0 && m) { atomicAdd(&sh[l], __popc(m)); }
+    }
+    __syncthreads();
+    if (threadIdx.x < kLevels) { counts[threadIdx.x * gridDim.x + blockIdx.x] = sh[threadIdx.x]; }
+}
+
+//! counts -> first node index per level and block, and the level ranges (one block, one warp per level)
+__global__ void __launch_bounds__(kLevels * 32) levelScanKernel(int* counts, int numBlocks, int numNodes, int* levelRange)
+{
+    __shared__ int total[kLevels];
+    __shared__ int first[kLevels + 1];
+    int l = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int* row = counts + size_t(l) * numBlocks;
+    int sum  = 0;
+    for (int q = lane; q < numBlocks; q += 32)
+    {
+        sum += row[q];
+    }
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    if (lane == 0) { total[l] = sum; }
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        int run = 0;
+        for (int k = 0; k < kLevels; ++k)
+        {
+            first[k] = run;
+            run += total[k];
+        }
+        first[kLevels] = numNodes;
+    }
+    __syncthreads();
+    if (threadIdx.x <= kLevels) { levelRange[threadIdx.x] = first[threadIdx.x]; }
+    int carry = first[l];
+    for (int base = 0; base < numBlocks; base += 32)
+    {
+        int q = base + lane;
+        int v = q < numBlocks ? row[q] : 0;
+        int incl = v;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1)
+        {
+            int t = __shfl_up_sync(0xffffffffu, incl, off);
+            if (lane >= off) { incl += t; }
+        }
+        if (q < numBlocks) { row[q] = carry + incl - v; }
+        carry += __shfl_sync(0xffffffffu, incl, 31);
     }
 }
 
-__global__ void mapNodesKernel(const uint32_t* ids, int numNodes, int numInternal, int* nodeToLeaf, int* leafToNode)
+//! every node at its position (positions past the arrays, of a malformed leaf array, are dropped)
+__global__ void __launch_bounds__(kLevelThreads) emitNodesKernel(const uint64_t* leaves, int numLeaves, int numNodes,
+                                                                const int* firstOf, uint64_t* prefixes,
+                                                                int* nodeToLeaf, int* leafToNode)
 {
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= numNodes) { return; }
-    int leaf      = int(ids[p]) - numInternal;
-    nodeToLeaf[p] = leaf;
-    if (leaf >= 0) { leafToNode[leaf] = p; }
-}
-
-__global__ void levelRangeKernel(const uint64_t* prefixes, int numNodes, int* levelRange)
-{
-    int l = threadIdx.x;
-    if (l <= int(kMaxLevel)) { levelRange[l] = int(lowerBound(prefixes, numNodes, uint64_t(1) << (3 * l))); }
-    if (l == int(kMaxLevel) + 1) { levelRange[l] = numNodes; }
+    __shared__ int before[kLevelWarps][kLevels];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int i = blockIdx.x * kLevelThreads + threadIdx.x;
+    uint64_t key;
+    int a, b;
+    startedLevels(leaves, numLeaves, i, &key, &a, &b);
+    for (int l = 0; l < kLevels; ++l)
+    {
+        unsigned m = __ballot_sync(0xffffffffu, l >= a && l <= b);
+        if (lane == 0) { before[warp][l] = __popc(m); }
+    }
+    __syncthreads();
+    if (threadIdx.x < kLevels)
+    {
+        int run = firstOf[threadIdx.x * gridDim.x + blockIdx.x];
+        for (int w = 0; w < kLevelWarps; ++w)
+        {
+            int c                  = before[w][threadIdx.x];
+            before[w][threadIdx.x] = run;
+            run += c;
+        }
+    }
+    __syncthreads();
+    for (int l = 0; l < kLevels; ++l)
+    {
+        bool mine  = l >= a && l <= b;
+        unsigned m = __ballot_sync(0xffffffffu, mine);
+        if (!mine) { continue; }
+        int p = before[warp][l] + __popc(m & ((1u << lane) - 1u));
+        if (p < numNodes)
+        {
+            prefixes[p]   = encodePrefix(key, unsigned(l));
+            nodeToLeaf[p] = l == b ? i : -1;
+        }
+        if (l == b) { leafToNode[i] = min(p, numNodes - 1); }
+    }
 }
 
 struct LevelRange
@@ -120,6 +198,11 @@ __global__ void linkKernel(const uint64_t* prefixes, const int* nodeToLeaf, int 
     }
     uint64_t prefix = prefixes[p];
     unsigned level  = prefixLevel(prefix);
+    if (prefix == 0 || level >= kMaxLevel)
+    {
+        childOffsets[p] = 0; // malformed leaf array
+        return;
+    }
     uint64_t child  = encodePrefix(prefixStart(prefix), level + 1);
     int b           = lr.r[level + 1];
     int e           = lr.r[level + 2];
@@ -137,28 +220,56 @@ __global__ void linkKernel(const uint64_t* prefixes, const int* nodeToLeaf, int 
 // counts and geometry
 // ---------------------------------------------------------------------------------------------------------------
 
-__global__ void leafCountsKernel(const uint64_t* leaves, int numLeaves, const uint64_t* keys, size_t n,
-                                 unsigned* counts)
+constexpr int kCountThreads = 256;
+
+/*! counts[i] = keys in [leaves[i], leaves[i + 1]), the layout first[i] = keys below leaves[i] (i <= numLeaves; the
+ *  exclusive scan of the counts, since the leaves start at key 0), and the largest count into *maxCount; first and
+ *  maxCount may be null. One binary search per boundary: a leaf takes its end from the next thread. */
+__global__ void __launch_bounds__(kCountThreads) leafCountsKernel(const uint64_t* leaves, int numLeaves,
+                                                                 const uint64_t* keys, size_t n, unsigned* counts,
+                                                                 int* first, unsigned* maxCount)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= numLeaves) { return; }
-    size_t b  = lowerBound(keys, n, leaves[i]);
-    size_t e  = lowerBound(keys, n, leaves[i + 1]);
-    counts[i] = unsigned(e - b);
+    __shared__ size_t bound[kCountThreads];
+    int i = blockIdx.x * (kCountThreads - 1) + threadIdx.x;
+    size_t b = i <= numLeaves ? lowerBound(keys, n, leaves[i]) : n;
+    bound[threadIdx.x] = b;
+    __syncthreads();
+    unsigned c = 0;
+    if (threadIdx.x < kCountThreads - 1 && i <= numLeaves)
+    {
+        if (first) { first[i] = int(b); }
+        if (i < numLeaves)
+        {
+            c         = unsigned(bound[threadIdx.x + 1] - b);
+            counts[i] = c;
+        }
+    }
+    if (maxCount)
+    {
+        c = __reduce_max_sync(0xffffffffu, c);
+        if ((threadIdx.x & 31) == 0 && c) { atomicMax(maxCount, c); }
+    }
 }
 
-__global__ void nodeCountsKernel(const uint64_t* prefixes, int numNodes, const uint64_t* leaves, int numLeaves,
-                                 const int* leafScan, unsigned* nodeCounts)
+//! counts of every node: a leaf's own, or the layout at the ends of the leaves an internal node covers
+__global__ void nodeCountsKernel(const uint64_t* prefixes, const int* nodeToLeaf, int numNodes, const uint64_t* leaves,
+                                 int numLeaves, const unsigned* leafCounts, const int* layout, unsigned* nodeCounts)
 {
     int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= numNodes) { return; }
+    int leaf = nodeToLeaf[p];
+    if (leaf >= 0)
+    {
+        nodeCounts[p] = leafCounts[leaf];
+        return;
+    }
     uint64_t prefix = prefixes[p];
     unsigned level  = prefixLevel(prefix);
     uint64_t start  = prefixStart(prefix);
     uint64_t end    = start + nodeRangeAt(level);
     size_t b        = lowerBound(leaves, size_t(numLeaves) + 1, start);
     size_t e        = lowerBound(leaves, size_t(numLeaves) + 1, end);
-    nodeCounts[p]   = unsigned(leafScan[e] - leafScan[b]);
+    nodeCounts[p]   = unsigned(layout[e] - layout[b]);
 }
 
 __global__ void geoKernel(const uint64_t* prefixes, int numNodes, DevBox box, double* centers, double* sizes)
@@ -255,17 +366,6 @@ __global__ void rebalanceKernel(const uint64_t* leaves, int numLeaves, const int
             newLeaves[out + s] = key + uint64_t(s) * step;
         }
     }
-}
-
-__global__ void maxCountKernel(const unsigned* counts, int n, unsigned* flags)
-{
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    unsigned v = i < n ? counts[i] : 0u;
-    for (int off = 16; off > 0; off >>= 1)
-    {
-        v = max(v, __shfl_xor_sync(0xffffffffu, v, off));
-    }
-    if ((threadIdx.x & 31) == 0 && v) { atomicMax(flags + 1, v); }
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -442,29 +542,15 @@ int buildLinkedOctree(const uint64_t* leaves, int numLeaves, LinkedOctree& t, Tr
     SPHB_TRY(t.nodeCounts.reserve(nn));
     SPHB_TRY(t.centers.reserve(3 * size_t(nn)));
     SPHB_TRY(t.sizes.reserve(3 * size_t(nn)));
-    SPHB_TRY(s.ints.reserve(std::max(numLeaves + 1, int(kMaxLevel) + 2)));
-    SPHB_TRY(s.ints2.reserve(std::max(nn, numLeaves + 1) + 1));
-    SPHB_TRY(s.scanTmp.reserve(scanTempInts(numLeaves + 1) + 1));
-    SPHB_TRY(s.sortTmp.reserve(sortScratchBytes(nn)));
-
-    unsigned nb = ceilDiv(numLeaves + 1, 256);
-    internalCountKernel<<<nb, 256, 0, stream>>>(leaves, numLeaves, s.ints.data());
-    SPHB_TRY(exclusiveScan(s.ints.data(), s.ints.data(), numLeaves, s.scanTmp.data(), stream));
-    uint32_t* ids = reinterpret_cast<uint32_t*>(s.ints2.data());
-    emitNodesKernel<<<ceilDiv(numLeaves, 256), 256, 0, stream>>>(leaves, numLeaves, t.numInternal, s.ints.data(),
-                                                                 t.prefixes.data(), ids);
-    countLaunch(2);
-    SPHB_CUDA_TRY(cudaGetLastError());
-    if (nn > 1)
-    {
-        SPHB_TRY(sortByKey(t.prefixes.data(), ids, nn, false, s.sortTmp.data(), s.sortTmp.capacity(), stream));
-    }
-    mapNodesKernel<<<ceilDiv(nn, 256), 256, 0, stream>>>(ids, nn, t.numInternal, t.nodeToLeaf.data(),
-                                                         t.leafToNode.data());
+    unsigned nb = ceilDiv(numLeaves, kLevelThreads);
+    SPHB_TRY(s.ints.reserve(size_t(kLevels) * nb));
     // the level ranges stay on the device: the link kernel reads them there (no host round trip per tree build)
     SPHB_TRY(t.levelRangeD.reserve(kMaxLevel + 2));
-    levelRangeKernel<<<1, 32, 0, stream>>>(t.prefixes.data(), nn, t.levelRangeD.data());
-    countLaunch(2);
+    levelCountKernel<<<nb, kLevelThreads, 0, stream>>>(leaves, numLeaves, s.ints.data());
+    levelScanKernel<<<1, kLevels * 32, 0, stream>>>(s.ints.data(), int(nb), nn, t.levelRangeD.data());
+    emitNodesKernel<<<nb, kLevelThreads, 0, stream>>>(leaves, numLeaves, nn, s.ints.data(), t.prefixes.data(),
+                                                      t.nodeToLeaf.data(), t.leafToNode.data());
+    countLaunch(3);
     SPHB_CUDA_TRY(cudaGetLastError());
     SPHB_CUDA_TRY(cudaMemsetAsync(t.parents.data(), 0, sizeof(int) * std::max(1, (nn - 1) / 8), stream));
     linkKernel<<<ceilDiv(nn, 256), 256, 0, stream>>>(t.prefixes.data(), t.nodeToLeaf.data(), nn,
@@ -475,23 +561,21 @@ int buildLinkedOctree(const uint64_t* leaves, int numLeaves, LinkedOctree& t, Tr
 }
 
 int computeLeafCounts(const uint64_t* leaves, int numLeaves, const uint64_t* keys, size_t n, unsigned* counts,
-                      cudaStream_t stream)
+                      cudaStream_t stream, int* layout, unsigned* maxCount)
 {
-    leafCountsKernel<<<ceilDiv(numLeaves, 256), 256, 0, stream>>>(leaves, numLeaves, keys, n, counts);
+    unsigned nb = ceilDiv(numLeaves + 1, kCountThreads - 1);
+    leafCountsKernel<<<nb, kCountThreads, 0, stream>>>(leaves, numLeaves, keys, n, counts, layout, maxCount);
     countLaunch();
     SPHB_CUDA_TRY(cudaGetLastError());
     return kOk;
 }
 
-int computeNodeCounts(const uint64_t* leaves, const unsigned* leafCounts, LinkedOctree& t, TreeScratch& s,
+int computeNodeCounts(const uint64_t* leaves, const unsigned* leafCounts, const int* layout, LinkedOctree& t,
                       cudaStream_t stream)
 {
-    SPHB_TRY(s.ints.reserve(t.numLeaves + 1));
-    SPHB_TRY(s.scanTmp.reserve(scanTempInts(t.numLeaves + 1) + 1));
-    SPHB_TRY(exclusiveScan(reinterpret_cast<const int*>(leafCounts), s.ints.data(), t.numLeaves, s.scanTmp.data(),
-                           stream));
-    nodeCountsKernel<<<ceilDiv(t.numNodes, 256), 256, 0, stream>>>(t.prefixes.data(), t.numNodes, leaves,
-                                                                  t.numLeaves, s.ints.data(), t.nodeCounts.data());
+    nodeCountsKernel<<<ceilDiv(t.numNodes, 256), 256, 0, stream>>>(t.prefixes.data(), t.nodeToLeaf.data(), t.numNodes,
+                                                                  leaves, t.numLeaves, leafCounts, layout,
+                                                                  t.nodeCounts.data());
     countLaunch();
     SPHB_CUDA_TRY(cudaGetLastError());
     return kOk;
@@ -537,10 +621,7 @@ int globalTreeStep(GlobalTree& g, const uint64_t* keys, size_t n, TreeScratch& s
     SPHB_TRY(exclusiveScan(s.ints.data(), s.ints.data(), L + 1, s.scanTmp.data(), stream));
     // the counts of the current leaves, before knowing whether they change: in the steady state nothing splits or
     // merges and one read back serves both decisions
-    SPHB_TRY(computeLeafCounts(g.leaves.data(), L, keys, n, g.counts.data(), stream));
-    maxCountKernel<<<ceilDiv(L, 256), 256, 0, stream>>>(g.counts.data(), L, s.flags.data());
-    countLaunch();
-    SPHB_CUDA_TRY(cudaGetLastError());
+    SPHB_TRY(computeLeafCounts(g.leaves.data(), L, keys, n, g.counts.data(), stream, nullptr, s.flags.data() + 1));
     unsigned msg[3]; // new leaf count, any op, largest count
     SPHB_TRY(readBack(stream, {{msg, s.ints.data() + L, sizeof(int)}, {msg + 1, s.flags.data(), 2 * sizeof(unsigned)}}));
     int newL       = int(msg[0]);
@@ -557,11 +638,9 @@ int globalTreeStep(GlobalTree& g, const uint64_t* keys, size_t n, TreeScratch& s
         g.numLeaves = newL;
         g.hostStale = true;
         SPHB_TRY(g.counts.reserve(newL));
-        SPHB_TRY(computeLeafCounts(g.leaves.data(), newL, keys, n, g.counts.data(), stream));
         SPHB_CUDA_TRY(cudaMemsetAsync(s.flags.data() + 1, 0, sizeof(unsigned), stream));
-        maxCountKernel<<<ceilDiv(newL, 256), 256, 0, stream>>>(g.counts.data(), newL, s.flags.data());
-        countLaunch();
-        SPHB_CUDA_TRY(cudaGetLastError());
+        SPHB_TRY(computeLeafCounts(g.leaves.data(), newL, keys, n, g.counts.data(), stream, nullptr,
+                                   s.flags.data() + 1));
         SPHB_TRY(readBack(stream, {{msg + 2, s.flags.data() + 1, sizeof(unsigned)}}));
     }
     *maxCount = anyOp ? msg[2] : 0u;
@@ -698,16 +777,13 @@ int focusUpdateTree(FocusTree& f, const GlobalTree& g, TreeScratch& s, cudaStrea
     return kOk;
 }
 
-int focusUpdateCounts(FocusTree& f, const uint64_t* keys, size_t n, TreeScratch& s, cudaStream_t stream)
+int focusUpdateCounts(FocusTree& f, const uint64_t* keys, size_t n, cudaStream_t stream)
 {
     int L = f.numLeaves;
     SPHB_TRY(f.leafCounts.reserve(L));
     SPHB_TRY(f.layout.reserve(L + 1));
-    SPHB_TRY(s.scanTmp.reserve(scanTempInts(L + 1) + 1));
-    SPHB_TRY(computeLeafCounts(f.leaves.data(), L, keys, n, f.leafCounts.data(), stream));
-    SPHB_TRY(computeNodeCounts(f.leaves.data(), f.leafCounts.data(), f.tree, s, stream));
-    SPHB_TRY(exclusiveScan(reinterpret_cast<const int*>(f.leafCounts.data()), f.layout.data(), L, s.scanTmp.data(),
-                           stream));
+    SPHB_TRY(computeLeafCounts(f.leaves.data(), L, keys, n, f.leafCounts.data(), stream, f.layout.data()));
+    SPHB_TRY(computeNodeCounts(f.leaves.data(), f.leafCounts.data(), f.layout.data(), f.tree, stream));
     return kOk;
 }
 

@@ -35,19 +35,19 @@ struct TreeScratch
     DeviceBuffer<int> ints2;
     DeviceBuffer<int> scanTmp;
     DeviceBuffer<uint64_t> keys;
-    DeviceBuffer<char> sortTmp;
     DeviceBuffer<unsigned> flags; // small device status words
 };
 
 /*! Build (or rebuild) the linked octree of `leaves` (numLeaves + 1 keys, device) into `tree`. */
 int buildLinkedOctree(const uint64_t* leaves, int numLeaves, LinkedOctree& tree, TreeScratch& s, cudaStream_t stream);
 
-/*! counts[i] = number of sorted keys in [leaves[i], leaves[i+1]) (cstone/tree/csarray.hpp:76-86,181-235) */
+/*! counts[i] = number of sorted keys in [leaves[i], leaves[i+1]) (cstone/tree/csarray.hpp:76-86,181-235); with layout,
+ *  the first key of every leaf too (numLeaves + 1 entries); with maxCount (zero on entry), the largest count */
 int computeLeafCounts(const uint64_t* leaves, int numLeaves, const uint64_t* keys, size_t n, unsigned* counts,
-                      cudaStream_t stream);
+                      cudaStream_t stream, int* layout = nullptr, unsigned* maxCount = nullptr);
 
-/*! node counts of every octree node from the leaf counts (sum over each node's leaf range) */
-int computeNodeCounts(const uint64_t* leaves, const unsigned* leafCounts, LinkedOctree& tree, TreeScratch& s,
+/*! node counts of every octree node from the leaf counts and layout (sum over each node's leaf range) */
+int computeNodeCounts(const uint64_t* leaves, const unsigned* leafCounts, const int* layout, LinkedOctree& tree,
                       cudaStream_t stream);
 
 /*! geometric centres and half sizes of every node inside `box` (cstone/focus/source_center.hpp:147-158) */
@@ -97,6 +97,6 @@ int initFocusTree(FocusTree& f, unsigned bucket, TreeScratch& s, cudaStream_t st
 int focusUpdateTree(FocusTree& f, const GlobalTree& g, TreeScratch& s, cudaStream_t stream, bool* converged);
 
 /*! FocusedOctree::updateCounts at one rank (octree_focus_mpi.hpp:192-251) + layout (cstone/domain/layout.hpp) */
-int focusUpdateCounts(FocusTree& f, const uint64_t* keys, size_t n, TreeScratch& s, cudaStream_t stream);
+int focusUpdateCounts(FocusTree& f, const uint64_t* keys, size_t n, cudaStream_t stream);
 
 } // namespace sphb

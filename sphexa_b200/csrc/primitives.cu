@@ -187,6 +187,38 @@ __global__ void __launch_bounds__(kScanThreads) scanTilesKernel(const int* in, i
     if (blockIdx.x == numTiles - 1 && threadIdx.x == 0) { out[n] = tileOffsets[numTiles]; }
 }
 
+//! tiles that one block scans in turn, carrying the sum, instead of three launches over all tiles
+constexpr size_t kScanOneBlock = 8;
+
+/*! exclusiveScan by one block, tile after tile: the tree arrays of up to 32,768 leaves, for which three launches of
+ *  3 us each are all latency. in and out may be the same. */
+__global__ void __launch_bounds__(kScanThreads) scanOneBlockKernel(const int* in, int* out, size_t n)
+{
+    int carry = 0;
+    for (size_t tile = 0; tile < n; tile += kScanTile)
+    {
+        size_t base = tile + size_t(threadIdx.x) * kScanItems;
+        int v[kScanItems];
+        int s = 0;
+#pragma unroll
+        for (int k = 0; k < kScanItems; ++k)
+        {
+            v[k] = base + k < n ? in[base + k] : 0;
+            s += v[k];
+        }
+        int total;
+        int ex = blockExclusiveScan(s, &total) + carry;
+#pragma unroll
+        for (int k = 0; k < kScanItems; ++k)
+        {
+            if (base + k < n) { out[base + k] = ex; }
+            ex += v[k];
+        }
+        carry += total;
+    }
+    if (threadIdx.x == 0) { out[n] = carry; }
+}
+
 struct Gather8Args
 {
     const uint64_t* src[16];
@@ -217,6 +249,13 @@ int exclusiveScan(const int* in, int* out, size_t n, int* tmp, cudaStream_t stre
     }
     size_t numTiles = (n + kScanTile - 1) / kScanTile;
     if (numTiles > size_t(kScanTile)) { return kErrCapacity; }
+    if (numTiles <= kScanOneBlock)
+    {
+        scanOneBlockKernel<<<1, kScanThreads, 0, stream>>>(in, out, n);
+        countLaunch();
+        SPHB_CUDA_TRY(cudaGetLastError());
+        return kOk;
+    }
     tileSumKernel<<<unsigned(numTiles), kScanThreads, 0, stream>>>(in, n, tmp);
     scanTileSumsKernel<<<1, kScanThreads, 0, stream>>>(tmp, int(numTiles));
     scanTilesKernel<<<unsigned(numTiles), kScanThreads, 0, stream>>>(in, out, n, tmp, int(numTiles));
