@@ -136,10 +136,23 @@ int syncDomain(sphb_sim& s)
     SPHB_TRY(updateBox(s));
     s.boxFirstCall = false;
     SPHB_TRY(launchSfcKeys(s.f[fX].data(), s.f[fY].data(), s.f[fZ].data(), s.keys.data(), s.n, s.box, st));
-    // particles move a fraction of h per step, so the previous order is nearly sorted (often exactly)
+    // particles move a fraction of h per step, so the previous step's leaves still hold few particles each; without
+    // a tree (the first sync), or with leaves too large for a warp, the previous order may still be nearly sorted
     bool identity = false;
-    SPHB_TRY(sortNearlySorted(s.keys.data(), s.order.data(), s.n, s.sortScratch.data(), s.sortScratch.capacity(),
-                              &identity, st));
+    if (!s.ftree.firstCall && s.p.bucket_focus <= 64)
+    {
+        LeafSort how;
+        SPHB_TRY(s.keysAlt.reserve(s.n));
+        SPHB_TRY(sortByLeaves(s.keys.data(), s.keysAlt.data(), s.order.data(), s.n, s.ftree.leaves.data(),
+                              s.ftree.numLeaves, s.leafSort, s.sortScratch.data(), s.sortScratch.capacity(), &how, st));
+        if (how == LeafSort::keysOut) { s.keys.swap(s.keysAlt); }
+        identity = how == LeafSort::identity;
+    }
+    else
+    {
+        SPHB_TRY(sortNearlySorted(s.keys.data(), s.order.data(), s.n, s.sortScratch.data(), s.sortScratch.capacity(),
+                                  &identity, st));
+    }
     s.lastSyncIdentity = identity;
     if (s.skinValid && !identity)
     {

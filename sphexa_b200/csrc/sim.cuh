@@ -57,6 +57,8 @@ struct sphb_sim
     DeviceBuffer<double> f[kNumConserved];
     DeviceBuffer<double> fAlt[kNumConserved];
     DeviceBuffer<uint64_t> id, idAlt, keys;
+    DeviceBuffer<uint64_t> keysAlt; // sorted keys of the sort by leaves, swapped with keys
+    LeafSortScratch leafSort;
     DeviceBuffer<uint32_t> order;
     DeviceBuffer<char> sortScratch;
     DeviceBuffer<double4> pos;

@@ -13,6 +13,7 @@
 #include <cudaTypedefs.h>
 
 #include "common.cuh"
+#include "primitives.cuh"
 #include "sort.cuh"
 
 namespace sphb
@@ -631,6 +632,258 @@ int repairSegmentedAsync(uint64_t* keys, uint32_t* values, const uint64_t* seg, 
         keys, values, seg, n, kRepairTile / 2);
     inversionsSegKernel<<<blocks, 256, 0, stream>>>(keys, seg, n, flags + 1);
     SPHB_CUDA_TRY(cudaGetLastError());
+    return kOk;
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// Sort of a step's particles by the leaves of the previous step's tree
+//
+// Bound by memory: 2 reads and 2 writes of the pairs plus the leaf searches, whatever moved. The repair of nearly sorted
+// keys pays only while particles stay within a tile of 2,048; one that crosses an octant boundary of the curve far up
+// moves by up to n, and then both repair passes (45 us each at 4,096 particles, 91 us at 128^3) were followed by the
+// radix sort (eight passes of 18 to 38 us and an 8 KB host read). Sync of a step with such a motion: 16^3 235 -> 154 us,
+// 30^3 510 -> 168 us, 81^3 (Noh) 663 -> 263 us, 128^3 0.95 -> 0.43 ms. A warp sorts a leaf in registers; 128 keys
+// (four per lane) is where its bitonic network still fits 32 registers.
+// ---------------------------------------------------------------------------------------------------------------
+
+namespace
+{
+
+//! the largest leaf a warp sorts (four elements per lane)
+constexpr int kLeafSortCap = 128;
+
+//! largest l with leaves[l] <= key (leaves[0] = 0; l = numLeaves for keys past the last leaf)
+__device__ __forceinline__ int leafOf(const uint64_t* __restrict__ leaves, int numLeaves, uint64_t key)
+{
+    int lo = 0, hi = numLeaves + 1;
+    while (hi - lo > 1)
+    {
+        int mid = (lo + hi) >> 1;
+        if (__ldg(leaves + mid) <= key) { lo = mid; }
+        else { hi = mid; }
+    }
+    return lo;
+}
+
+/*! values = 0..n-1; slot[i] = {leaf of key i, its place among the leaf's keys in arrival order}, counts[l] = keys per
+ *  leaf (zero on entry); flags[0] = 1 if any adjacent pair is out of order, flags[1] = 1 if a leaf exceeds
+ *  kLeafSortCap. The lanes of a leaf (most of a warp: the keys are nearly in order) share one atomic. */
+__global__ void __launch_bounds__(256) leafSlotKernel(const uint64_t* __restrict__ keys, size_t n,
+                                                      const uint64_t* __restrict__ leaves, int numLeaves,
+                                                      uint32_t* __restrict__ values, uint2* __restrict__ slot,
+                                                      int* counts, unsigned* flags)
+{
+    size_t i   = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
+    bool valid = i < n;
+    int leaf   = -1;
+    bool inv   = false;
+    if (valid)
+    {
+        uint64_t k = keys[i];
+        inv        = i + 1 < n && k > keys[i + 1];
+        leaf       = leafOf(leaves, numLeaves, k);
+        values[i]  = uint32_t(i);
+    }
+    unsigned lane  = threadIdx.x & (kWarp - 1);
+    unsigned peers = __match_any_sync(0xffffffffu, leaf);
+    int leader     = __ffs(peers) - 1;
+    int base       = 0;
+    if (int(lane) == leader && valid) { base = atomicAdd(counts + leaf, __popc(peers)); }
+    base      = __shfl_sync(0xffffffffu, base, leader);
+    int place = base + __popc(peers & ((1u << lane) - 1u));
+    if (valid) { slot[i] = make_uint2(unsigned(leaf), unsigned(place)); }
+    unsigned anyInv  = __ballot_sync(0xffffffffu, inv);
+    unsigned anyFull = __ballot_sync(0xffffffffu, valid && place >= kLeafSortCap);
+    if (lane == 0 && anyInv) { flags[0] = 1u; }
+    if (lane == 0 && anyFull) { flags[1] = 1u; }
+}
+
+/*! composite[first[leaf] + place] = (the upper 32 bits of the key within its leaf, index): what a warp sorts. A leaf
+ *  of level L leaves 63 - 3 L bits of the key open. */
+__global__ void __launch_bounds__(256) leafScatterKernel(const uint64_t* __restrict__ keys, size_t n,
+                                                         const uint64_t* __restrict__ leaves, int numLeaves,
+                                                         const uint2* __restrict__ slot, const int* __restrict__ first,
+                                                         uint64_t* __restrict__ composite)
+{
+    size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
+    if (i >= n) { return; }
+    uint2 s        = slot[i];
+    uint64_t start = __ldg(leaves + s.x);
+    int shift      = 0;
+    if (int(s.x) < numLeaves) { shift = max(0, 31 - int(__clzll(__ldg(leaves + s.x + 1) - start))); }
+    size_t dst     = size_t(__ldg(first + s.x)) + s.y;
+    if (dst < n) { composite[dst] = (((keys[i] - start) >> shift) << 32) | uint64_t(i); }
+}
+
+//! bitonic sort of 32 kPer values of a warp, value e in register e / 32 of lane e % 32
+template<int kPer>
+__device__ __forceinline__ void warpSort(uint64_t (&v)[kPer], int lane)
+{
+#pragma unroll
+    for (int size = 2; size <= 32 * kPer; size <<= 1)
+    {
+#pragma unroll
+        for (int stride = size >> 1; stride > 0; stride >>= 1)
+        {
+            if (stride >= 32)
+            {
+#pragma unroll
+                for (int r = 0; r < kPer; ++r)
+                {
+                    int q = r ^ (stride / 32);
+                    if (q > r)
+                    {
+                        bool up = ((r * 32) & size) == 0;
+                        if ((v[r] > v[q]) == up)
+                        {
+                            uint64_t t = v[r];
+                            v[r]       = v[q];
+                            v[q]       = t;
+                        }
+                    }
+                }
+            }
+            else
+            {
+#pragma unroll
+                for (int r = 0; r < kPer; ++r)
+                {
+                    uint64_t o = __shfl_xor_sync(0xffffffffu, v[r], stride);
+                    bool up    = ((r * 32 + lane) & size) == 0;
+                    bool low   = (lane & stride) == 0;
+                    v[r]       = ((v[r] < o) == (up == low)) ? v[r] : o;
+                }
+            }
+        }
+    }
+}
+
+/*! One leaf: its composites sorted, then the keys and values in that order. Composites that agree in their upper half
+ *  may belong to different keys (the open bits beyond 32): such a leaf is ranked by its full keys instead. */
+template<int kPer>
+__device__ __forceinline__ void sortLeaf(const uint64_t* composite, const uint64_t* __restrict__ keysIn, int first, int m,
+                                         int lane, uint64_t* keysOut, uint32_t* values)
+{
+    uint64_t v[kPer];
+#pragma unroll
+    for (int r = 0; r < kPer; ++r)
+    {
+        int e = r * 32 + lane;
+        v[r]  = e < m ? composite[first + e] : ~uint64_t(0);
+    }
+    warpSort<kPer>(v, lane);
+    uint64_t key[kPer];
+    bool tie = false;
+#pragma unroll
+    for (int r = 0; r < kPer; ++r)
+    {
+        int e         = r * 32 + lane;
+        key[r]        = e < m ? __ldg(keysIn + uint32_t(v[r])) : ~uint64_t(0);
+        uint64_t next = __shfl_down_sync(0xffffffffu, v[r], 1);
+        if (r + 1 < kPer)
+        {
+            uint64_t wrap = __shfl_sync(0xffffffffu, v[r + 1 < kPer ? r + 1 : r], 0);
+            if (lane == 31) { next = wrap; }
+        }
+        tie = tie || (e + 1 < m && (lane < 31 || r + 1 < kPer) && (v[r] >> 32) == (next >> 32));
+    }
+    int place[kPer];
+#pragma unroll
+    for (int r = 0; r < kPer; ++r)
+    {
+        place[r] = r * 32 + lane;
+    }
+    if (__any_sync(0xffffffffu, tie))
+    {
+#pragma unroll
+        for (int r = 0; r < kPer; ++r)
+        {
+            place[r] = 0;
+        }
+#pragma unroll
+        for (int q = 0; q < kPer; ++q)
+        {
+            for (int src = 0; src < 32; ++src)
+            {
+                if (q * 32 + src >= m) { break; }
+                uint64_t ko = __shfl_sync(0xffffffffu, key[q], src);
+                uint32_t io = __shfl_sync(0xffffffffu, uint32_t(v[q]), src);
+#pragma unroll
+                for (int r = 0; r < kPer; ++r)
+                {
+                    place[r] += (ko < key[r] || (ko == key[r] && io < uint32_t(v[r]))) ? 1 : 0;
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < kPer; ++r)
+    {
+        if (r * 32 + lane < m)
+        {
+            keysOut[first + place[r]] = key[r];
+            values[first + place[r]]  = uint32_t(v[r]);
+        }
+    }
+}
+
+//! one warp per leaf (and one for the keys past the last leaf)
+__global__ void __launch_bounds__(256) leafSortKernel(const uint64_t* __restrict__ composite,
+                                                      const uint64_t* __restrict__ keysIn, int numLeaves,
+                                                      const int* __restrict__ first, uint64_t* __restrict__ keysOut,
+                                                      uint32_t* __restrict__ values)
+{
+    int leaf = int((blockIdx.x * size_t(blockDim.x) + threadIdx.x) / kWarp);
+    int lane = threadIdx.x & (kWarp - 1);
+    if (leaf > numLeaves) { return; }
+    int b = first[leaf], m = first[leaf + 1] - b;
+    if (m <= 0) { return; }
+    if (m <= 32) { sortLeaf<1>(composite, keysIn, b, m, lane, keysOut, values); }
+    else if (m <= 64) { sortLeaf<2>(composite, keysIn, b, m, lane, keysOut, values); }
+    else { sortLeaf<4>(composite, keysIn, b, min(m, kLeafSortCap), lane, keysOut, values); }
+}
+
+} // namespace
+
+int sortByLeaves(uint64_t* keys, uint64_t* keysOut, uint32_t* values, size_t n, const uint64_t* leaves, int numLeaves,
+                 LeafSortScratch& ls, void* scratch, size_t scratchBytes, LeafSort* result, cudaStream_t stream)
+{
+    *result = LeafSort::inPlace;
+    if (n == 0)
+    {
+        *result = LeafSort::identity;
+        return kOk;
+    }
+    if (n >= (size_t(1) << 30) || numLeaves < 1) { return kErrArg; }
+    if (!scratch || scratchBytes < sortScratchBytes(n)) { return kErrCapacity; }
+    size_t buckets = size_t(numLeaves) + 1;
+    SPHB_TRY(ls.slot.reserve(n));
+    SPHB_TRY(ls.first.reserve(buckets + 1 + 2));
+    SPHB_TRY(ls.scanTmp.reserve(scanTempInts(buckets) + 1));
+    int* counts     = ls.first.data() + 2;
+    unsigned* flags = reinterpret_cast<unsigned*>(ls.first.data());
+    SPHB_CUDA_TRY(cudaMemsetAsync(ls.first.data(), 0, (buckets + 2) * sizeof(int), stream));
+    leafSlotKernel<<<ceilDiv(n, 256), 256, 0, stream>>>(keys, n, leaves, numLeaves, values, ls.slot.data(), counts,
+                                                        flags);
+    countLaunch();
+    SPHB_CUDA_TRY(cudaGetLastError());
+    unsigned msg[2];
+    SPHB_TRY(readBack(stream, {{msg, flags, sizeof(msg)}}));
+    if (!msg[0])
+    {
+        *result = LeafSort::identity;
+        return kOk;
+    }
+    if (msg[1]) { return sortByKey(keys, values, n, false, scratch, scratchBytes, stream); }
+    uint64_t* composite = carve(scratch, n).keysAlt;
+    SPHB_TRY(exclusiveScan(counts, counts, buckets, ls.scanTmp.data(), stream));
+    leafScatterKernel<<<ceilDiv(n, 256), 256, 0, stream>>>(keys, n, leaves, numLeaves, ls.slot.data(), counts,
+                                                           composite);
+    leafSortKernel<<<ceilDiv(buckets * kWarp, 256), 256, 0, stream>>>(composite, keys, numLeaves, counts, keysOut,
+                                                                      values);
+    countLaunch(2);
+    SPHB_CUDA_TRY(cudaGetLastError());
+    *result = LeafSort::keysOut;
     return kOk;
 }
 

@@ -19,6 +19,30 @@ int sortByKey(uint64_t* keys, uint32_t* values, size_t n, bool initValues, void*
 int sortNearlySorted(uint64_t* keys, uint32_t* values, size_t n, void* scratch, size_t scratchBytes, bool* identity,
                      cudaStream_t stream);
 
+//! where sortByLeaves left the sorted keys
+enum class LeafSort
+{
+    identity, // the keys were in order already
+    inPlace,  // in keys
+    keysOut   // in keysOut
+};
+
+//! device buffers of sortByLeaves
+struct LeafSortScratch
+{
+    DeviceBuffer<uint2> slot;
+    DeviceBuffer<int> first;
+    DeviceBuffer<int> scanTmp;
+};
+
+/*! The same stable sort (values = 0..n-1 first) with the help of a cornerstone leaf array that held few keys per leaf
+ *  for keys close to these, the tree of the previous step: every key finds its leaf, a scan of the leaf counts places
+ *  the leaves, and one warp sorts each leaf. One host read, of whether anything is out of order and whether a leaf
+ *  grew past 128 keys (then the radix sort runs, in place). It reads and writes the keys twice whatever the particles'
+ *  motion is, where the radix sort takes eight passes. */
+int sortByLeaves(uint64_t* keys, uint64_t* keysOut, uint32_t* values, size_t n, const uint64_t* leaves, int numLeaves,
+                 LeafSortScratch& ls, void* scratch, size_t scratchBytes, LeafSort* result, cudaStream_t stream);
+
 /*! The same sort without any host synchronisation (stream-capturable): runs exactly the passes of passMask (bit p
  *  = byte p of the key, from the least significant) and ORs a look-back timeout into *errorOut (device) if set. */
 int sortByKeyAsync(uint64_t* keys, uint32_t* values, size_t n, bool initValues, void* scratch, size_t scratchBytes,
