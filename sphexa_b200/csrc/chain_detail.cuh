@@ -18,23 +18,24 @@ constexpr int kModeBatch   = 2;
 constexpr int kModeAvClean = 4;
 constexpr int kModeList    = 8; // block time steps: only the groups of a device-side list
 
-/*! Neighbour-sum accumulator. FP64: every term is added as it comes, in list order (the reference's order).
- *  FP32: terms are summed plainly within one list chunk of 8 neighbours and each chunk sum is added to a
- *  Kahan-compensated accumulator; explicit round-to-nearest intrinsics keep the compiler from fusing or reordering
- *  the compensation. */
+/*! Neighbour-sum accumulator. Terms are summed plainly within one list chunk of 8 neighbours, in list order, and the
+ *  chunk sums are added in chunk order: FP64 plainly, FP32 with Kahan compensation (explicit round-to-nearest
+ *  intrinsics keep the compiler from fusing or reordering it). A chunk may be summed by another lane (foldChunks), so
+ *  the result does not depend on how many lanes share a target. */
 template<class T>
 struct BlockSum;
 
 template<>
 struct BlockSum<double>
 {
-    double s;
+    double s, part;
     __device__ explicit BlockSum(double v = 0.0)
         : s(v)
+        , part(0.0)
     {
     }
-    __device__ void add(double v) { s += v; }
-    __device__ void flush() {}
+    __device__ void add(double v) { part += v; }
+    __device__ void addChunk(double v) { s += v; }
     __device__ double get() const { return s; }
 };
 
@@ -49,20 +50,79 @@ struct BlockSum<float>
     {
     }
     __device__ void add(float v) { part += v; }
-    __device__ void flush()
+    __device__ void addChunk(float v)
     {
-        float y = __fsub_rn(part, comp);
+        float y = __fsub_rn(v, comp);
         float t = __fadd_rn(s, y);
         comp    = __fsub_rn(__fsub_rn(t, s), y);
         s       = t;
-        part    = 0.f;
     }
     __device__ float get() const { return s; }
 };
 
+/*! Add the chunk sums of one round to the accumulators and clear them: this lane's own (kSplit = 1), or those of the
+ *  kSplit lanes that share a target, in chunk order (chunks first .. first + kSplit - 1 of numChunks); every lane of
+ *  the warp calls it, and the lanes of a target end with equal sums. */
+template<int kSplit, class... S>
+__device__ __forceinline__ void foldChunks(unsigned first, unsigned numChunks, S&... acc)
+{
+    if constexpr (kSplit == 1) { (acc.addChunk(acc.part), ...); }
+    else
+    {
+#pragma unroll
+        for (int s = 0; s < kSplit; ++s)
+        {
+            auto one = [&](auto& a) {
+                auto v = __shfl_sync(0xffffffffu, a.part, s, kSplit);
+                if (first + s < numChunks) { a.addChunk(v); }
+            };
+            (one(acc), ...);
+        }
+    }
+    ((acc.part = 0), ...);
+}
+
+//! the largest value over the lanes that share a target
+template<int kSplit, class T>
+__device__ __forceinline__ T maxOverSplit(T v)
+{
+#pragma unroll
+    for (int off = 1; off < kSplit; off <<= 1)
+    {
+        T o = __shfl_xor_sync(0xffffffffu, v, off);
+        v   = o > v ? o : v;
+    }
+    return v;
+}
+
 //! a / b: IEEE division in FP64 (the reference's rounding), the fast 2-ulp reciprocal-multiply in FP32
 __device__ __forceinline__ double fdiv(double a, double b) { return a / b; }
 __device__ __forceinline__ float fdiv(float a, float b) { return __fdividef(a, b); }
+
+// Sums of products with the rounding written out. Left to the compiler, which product of a sum becomes the FMA's can
+// differ between the instances of a kernel (one lane or several per target, a single simulation or an ensemble), and
+// with it the last bit of their results.
+
+//! a . b
+template<class T>
+__device__ __forceinline__ T dot3(T ax, T ay, T az, T bx, T by, T bz)
+{
+    return fma(az, bz, fma(ay, by, ax * bx));
+}
+
+//! a b + c d
+template<class T>
+__device__ __forceinline__ T prodSum(T a, T b, T c, T d)
+{
+    return fma(a, b, c * d);
+}
+
+//! a b - c d
+template<class T>
+__device__ __forceinline__ T prodDiff(T a, T b, T c, T d)
+{
+    return fma(a, b, -(c * d));
+}
 
 //! linear interpolation in a 20000-entry table on [0, 2] (sph/include/sph/table_lookup.hpp:14-26)
 template<class T>
@@ -300,43 +360,72 @@ struct Target
     unsigned lane;
     unsigned count;
     unsigned ngPad;
+    unsigned sub{0};       // which of the lanes that share the target
+    unsigned numChunks{0}; // list chunks of the target
+    unsigned rounds{0};    // turns of the chunk loop: the target's own, or the warp's most where lanes share targets
 };
 
+//! the rest of a target's description once its particle is known; without a particle (valid false) an empty list
+template<int kSplit>
+__device__ __forceinline__ void fillTarget(Target& t, bool valid, const unsigned* nc, unsigned ngmax)
+{
+    if (!valid) { t.i = 0; }
+    t.group     = t.i >> 5;
+    t.lane      = unsigned(t.i & 31);
+    t.count     = valid ? min(nc[t.i] - 1u, ngmax) : 0u;
+    t.ngPad     = paddedNgmax(ngmax);
+    t.numChunks = (t.count + kNbChunk - 1) / kNbChunk;
+    t.rounds    = t.numChunks;
+    if constexpr (kSplit > 1)
+    {
+        t.rounds = __reduce_max_sync(0xffffffffu, (t.numChunks + kSplit - 1) / kSplit);
+    }
+}
+
+template<int kSplit = 1>
 __device__ __forceinline__ bool targetOf(size_t n, const unsigned* nc, unsigned ngmax, Target& t,
                                          const uint8_t* inst = nullptr)
 {
-    t.i = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
-    if (t.i >= n) { return false; }
-    if (inst && inst[t.i] == kGhost) { return false; }
-    t.group = t.i >> 5;
-    t.lane  = unsigned(t.i & 31);
-    t.count = min(nc[t.i] - 1u, ngmax);
-    t.ngPad = paddedNgmax(ngmax);
-    return true;
+    size_t thread = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
+    t.i           = thread / kSplit;
+    t.sub         = unsigned(thread % kSplit);
+    bool valid    = t.i < n && !(inst && inst[t.i] == kGhost);
+    if (kSplit == 1 && !valid) { return false; }
+    fillTarget<kSplit>(t, valid, nc, ngmax);
+    return valid;
 }
 
 /*! The target of this thread: thread i of the launch, or in list mode lane i % 32 of group groupList[i / 32], whose
- *  particles are [groupBounds[g], groupBounds[g + 1]) (GroupView slices of sph/include/sph/groups.hpp:96-103; a warp
- *  is one group of at most 32). *w receives the list slot. */
-template<int kMode, class T>
-__device__ __forceinline__ bool chainTarget(const ChainArrays<T>& a, unsigned ngmax, Target& t, unsigned* w = nullptr)
+ *  particles are [groupBounds[g], groupBounds[g + 1]) (GroupView slices of sph/include/sph/groups.hpp:96-103; a group
+ *  is at most 32 particles). kSplit threads share a target; with kSplit > 1 every thread gets a usable target, with an
+ *  empty list where there is no particle (false is returned). */
+template<int kMode, int kSplit = 1, class T>
+__device__ __forceinline__ bool chainTarget(const ChainArrays<T>& a, unsigned ngmax, Target& t)
 {
     if constexpr (kMode & kModeList)
     {
-        size_t slot = (blockIdx.x * size_t(blockDim.x) + threadIdx.x) >> 5;
-        if (w) { *w = unsigned(slot); }
-        if (slot >= a.numListed) { return false; }
-        uint32_t g = __ldg(a.groupList + slot);
-        t.i        = size_t(__ldg(a.groupBounds + g)) + (threadIdx.x & 31);
-        if (t.i >= __ldg(a.groupBounds + g + 1)) { return false; }
-        t.group = t.i >> 5;
-        t.lane  = unsigned(t.i & 31);
-        t.count = min(a.nc[t.i] - 1u, ngmax);
-        t.ngPad = paddedNgmax(ngmax);
-        return true;
+        size_t thread = (blockIdx.x * size_t(blockDim.x) + threadIdx.x) / kSplit;
+        size_t slot   = thread >> 5;
+        t.sub         = threadIdx.x % kSplit;
+        bool valid    = slot < a.numListed;
+        if (kSplit == 1 && !valid) { return false; }
+        if (valid)
+        {
+            uint32_t g = __ldg(a.groupList + slot);
+            t.i        = size_t(__ldg(a.groupBounds + g)) + (thread & 31);
+            valid      = t.i < __ldg(a.groupBounds + g + 1);
+        }
+        if (kSplit == 1 && !valid) { return false; }
+        fillTarget<kSplit>(t, valid, a.nc, ngmax);
+        return valid;
     }
-    else { return targetOf(a.n, a.nc, ngmax, t, (kMode & kModeBatch) ? a.batch.inst : nullptr); }
+    else { return targetOf<kSplit>(a.n, a.nc, ngmax, t, (kMode & kModeBatch) ? a.batch.inst : nullptr); }
 }
+
+/*! Run term(j) over this lane's chunk of a round (chunk round * kSplit + sub): every neighbour of a full chunk in an
+ *  unrolled body, or one neighbour per iteration (kRolled). */
+template<int kSplit, bool kRolled, class F>
+__device__ __forceinline__ void overChunk(const uint32_t* nidx, const Target& t, unsigned round, F&& term);
 
 template<class T>
 __device__ __forceinline__ AVRec<T> loadAV(const AVRec<T>* p)
@@ -380,8 +469,8 @@ __device__ __forceinline__ void loadDV(const DVRec<T>* p, T (&g)[6])
 template<class T>
 __device__ __forceinline__ T avRvCorrection(T rx, T ry, T rz, T etaAb, T etaCrit, const T (&gi)[6], const T (&gj)[6])
 {
-    T dmy1 = rx * (gi[0] * rx + gi[1] * ry + gi[2] * rz) + ry * (gi[3] * ry + gi[4] * rz) + rz * (gi[5] * rz);
-    T dmy2 = rx * (gj[0] * rx + gj[1] * ry + gj[2] * rz) + ry * (gj[3] * ry + gj[4] * rz) + rz * (gj[5] * rz);
+    T dmy1 = dot3(rx, ry, rz, dot3(gi[0], gi[1], gi[2], rx, ry, rz), prodSum(gi[3], ry, gi[4], rz), gi[5] * rz);
+    T dmy2 = dot3(rx, ry, rz, dot3(gj[0], gj[1], gj[2], rx, ry, rz), prodSum(gj[3], ry, gj[4], rz), gj[5] * rz);
     T dmy3 = T(1);
     if (etaAb < etaCrit)
     {
@@ -421,6 +510,33 @@ __device__ __forceinline__ uint32_t popChunk(uint32_t (&js)[kNbChunk])
         js[r] = js[r + 1];
     }
     return j;
+}
+
+template<int kSplit, bool kRolled, class F>
+__device__ __forceinline__ void overChunk(const uint32_t* nidx, const Target& t, unsigned round, F&& term)
+{
+    unsigned q0 = (round * kSplit + t.sub) * kNbChunk;
+    if (kSplit > 1 && q0 >= t.count) { return; }
+    uint32_t js[kNbChunk];
+    loadChunk(nidx, t, t.ngPad, q0, js);
+    unsigned qn = min(kNbChunk, t.count - q0);
+    if constexpr (kRolled)
+    {
+#pragma unroll 1
+        for (unsigned q = 0; q < qn; ++q)
+        {
+            term(popChunk(js));
+        }
+    }
+    else
+    {
+#pragma unroll
+        for (unsigned q = 0; q < kNbChunk; ++q)
+        {
+            if (q >= qn) { break; }
+            term(js[q]);
+        }
+    }
 }
 
 /*! Maximum (kMax) or minimum of one double per thread, published as ordered bits with one atomic per block on

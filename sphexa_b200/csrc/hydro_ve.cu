@@ -24,16 +24,23 @@ namespace
 
 using namespace chain;
 
+constexpr int kSplitThreads = 128; // block size of the launches whose lanes share targets
+// launches of at most so many targets take eight or four lanes per target (chainSplit)
+constexpr size_t kEightLaneTargets = 16384;
+constexpr size_t kFourLaneTargets  = 65536;
+
+
 // ---------------------------------------------------------------------------------------------------------------
 // XMass: rho0_i = (m_i + sum_j W_ij m_j) K / h_i^3, xm_i = m_i / rho0_i (sph/include/sph/hydro_ve/xmass_kern.hpp:50-79)
 // ---------------------------------------------------------------------------------------------------------------
 // FP32: at most 32 registers, eight 256-thread blocks per SM: more gathers in flight (0.348 -> 0.325 ms at 128^3)
-template<class T, int kMode>
-__global__ void __launch_bounds__(kChainMaxThreads, sizeof(T) == 4 ? 8 : 0)
+template<class T, int kMode, int kSplit>
+__global__ void __launch_bounds__(kChainMaxThreads, sizeof(T) == 4 && kSplit == 1 ? 8 : 0)
     xmassKernel(ChainArrays<T> a, HydroConsts<T> k, DevBox box)
 {
     Target t;
-    if (!chainTarget<kMode>(a, k.ngmax, t)) { return; }
+    const bool valid = chainTarget<kMode, kSplit>(a, k.ngmax, t);
+    if (kSplit == 1 && !valid) { return; }
     Pos<T> pi  = posOf(a, t.i);
     double hiD = a.h[t.i];
     T hi       = T(hiD);
@@ -43,23 +50,17 @@ __global__ void __launch_bounds__(kChainMaxThreads, sizeof(T) == 4 ? 8 : 0)
     T hh       = T(0.5) * hInv * hInv;
 
     BlockSum<T> rho0(mi);
-    for (unsigned q0 = 0; q0 < t.count; q0 += kNbChunk)
+    for (unsigned round = 0; round < t.rounds; ++round)
     {
-        uint32_t js[kNbChunk];
-        loadChunk(a.nidx, t, t.ngPad, q0, js);
-        unsigned qn = min(kNbChunk, t.count - q0);
-#pragma unroll
-        for (unsigned q = 0; q < kNbChunk; ++q)
-        {
-            if (q >= qn) { break; }
-            uint32_t j = js[q];
-            Pos<T> pj  = posOf(a, j);
-            Sep<T> r   = separation(pi, pj, 2.0 * hiD, box, k);
-            T r2       = r.rx * r.rx + r.ry * r.ry + r.rz * r.rz;
-            rho0.add(kernelWr2(a.wh, k, r2, hInv, hh) * T(pj.m));
-        }
-        rho0.flush();
+        overChunk<kSplit, false>(a.nidx, t, round, [&](uint32_t j) {
+        Pos<T> pj  = posOf(a, j);
+        Sep<T> r   = separation(pi, pj, 2.0 * hiD, box, k);
+        T r2       = dot3(r.rx, r.ry, r.rz, r.rx, r.ry, r.rz);
+        rho0.add(kernelWr2(a.wh, k, r2, hInv, hh) * T(pj.m));
+        });
+        foldChunks<kSplit>(round * kSplit, t.numChunks, rho0);
     }
+    if (kSplit > 1 && (!valid || t.sub != 0)) { return; }
     a.xm[t.i] = mi / (rho0.get() * k.K * h3Inv);
 }
 
@@ -69,12 +70,13 @@ __global__ void __launch_bounds__(kChainMaxThreads, sizeof(T) == 4 ? 8 : 0)
 // ---------------------------------------------------------------------------------------------------------------
 // FP32: at most 40 registers, six 256-thread blocks per SM, for the gathers' latency (0.625 -> 0.566 ms at 128^3,
 // though it spills a little; 48 registers gave 0.588, 32 gave 0.582)
-template<class T, int kMode>
-__global__ void __launch_bounds__(kChainMaxThreads, sizeof(T) == 4 ? 6 : 0)
+template<class T, int kMode, int kSplit>
+__global__ void __launch_bounds__(kChainMaxThreads, sizeof(T) == 4 && kSplit == 1 ? 6 : 0)
     veDefGradhEosKernel(ChainArrays<T> a, HydroConsts<T> k, DevBox box)
 {
     Target t;
-    if (!chainTarget<kMode>(a, k.ngmax, t)) { return; }
+    const bool valid = chainTarget<kMode, kSplit>(a, k.ngmax, t);
+    if (kSplit == 1 && !valid) { return; }
     Pos<T> pi  = posOf(a, t.i);
     double hiD = a.h[t.i];
     T hi       = T(hiD);
@@ -85,60 +87,52 @@ __global__ void __launch_bounds__(kChainMaxThreads, sizeof(T) == 4 ? 6 : 0)
     [[maybe_unused]] float hhV = 0.5f * float(hInv) * float(hInv);
 
     BlockSum<T> kxS(xmassi), whomegaS(-T(3) * xmassi), wrho0S(-T(3) * mi);
-    for (unsigned q0 = 0; q0 < t.count; q0 += kNbChunk)
+    for (unsigned round = 0; round < t.rounds; ++round)
     {
-        uint32_t js[kNbChunk];
-        loadChunk(a.nidx, t, t.ngPad, q0, js);
-        unsigned qn = min(kNbChunk, t.count - q0);
-#pragma unroll
-        for (unsigned q = 0; q < kNbChunk; ++q)
+        overChunk<kSplit, false>(a.nidx, t, round, [&](uint32_t j) {
+        Pos<T> pj  = posOf(a, j);
+        Sep<T> r   = separation(pi, pj, 2.0 * hiD, box, k);
+        T r2       = dot3(r.rx, r.ry, r.rz, r.rx, r.ry, r.rz);
+        T w, dterh;
+        if constexpr (sizeof(T) == 4)
         {
-            if (q >= qn) { break; }
-            uint32_t j = js[q];
-            Pos<T> pj  = posOf(a, j);
-            Sep<T> r   = separation(pi, pj, 2.0 * hiD, box, k);
-            T r2       = r.rx * r.rx + r.ry * r.ry + r.rz * r.rz;
-            T w, dterh;
-            if constexpr (sizeof(T) == 4)
+            if (k.usePoly)
             {
-                if (k.usePoly)
-                {
-                    // t = v^2/2 - 1 from r2 (no square root); W and dW's polynomial side by side in packed FP32
-                    // (sm_100 FFMA2); v dW = v^2 P'(t) = 2 (t + 1) P'(t) (0.638 -> 0.624 ms at 128^3)
-                    float tt   = fmaf(r2, hhV, -1.0f);
-                    float2 acc = make_float2(k.wpoly[kPolyTerms - 1], k.dwpoly[kPolyTerms - 1]);
+                // t = v^2/2 - 1 from r2 (no square root); W and dW's polynomial side by side in packed FP32
+                // (sm_100 FFMA2); v dW = v^2 P'(t) = 2 (t + 1) P'(t) (0.638 -> 0.624 ms at 128^3)
+                float tt   = fmaf(r2, hhV, -1.0f);
+                float2 acc = make_float2(k.wpoly[kPolyTerms - 1], k.dwpoly[kPolyTerms - 1]);
 #pragma unroll
-                    for (int p = kPolyTerms - 2; p >= 0; --p)
-                    {
-                        acc = __ffma2_rn(acc, make_float2(tt, tt), make_float2(k.wpoly[p], k.dwpoly[p]));
-                    }
-                    bool in = tt < 1.0f;
-                    w       = in ? acc.x : 0.0f;
-                    dterh   = in ? -(3.0f * acc.x + 2.0f * (tt + 1.0f) * acc.y) : 0.0f;
-                }
-                else
+                for (int p = kPolyTerms - 2; p >= 0; --p)
                 {
-                    T vloc = T(r2 * rsqrtf(float(r2))) * hInv;
-                    w      = kernelW(a.wh, k, vloc);
-                    dterh  = -(T(3) * w + vloc * kernelDW(a.whd, k, vloc));
+                    acc = __ffma2_rn(acc, make_float2(tt, tt), make_float2(k.wpoly[p], k.dwpoly[p]));
                 }
+                bool in = tt < 1.0f;
+                w       = in ? acc.x : 0.0f;
+                dterh   = in ? -prodSum(3.0f, acc.x, 2.0f * (tt + 1.0f), acc.y) : 0.0f;
             }
             else
             {
-                T vloc = T(sqrt(r2)) * hInv;
+                T vloc = T(r2 * rsqrtf(float(r2))) * hInv;
                 w      = kernelW(a.wh, k, vloc);
-                T dw   = kernelDW(a.whd, k, vloc);
-                dterh  = -(T(3) * w + vloc * dw);
+                dterh  = -prodSum(T(3), w, vloc, kernelDW(a.whd, k, vloc));
             }
-            T xmassj   = __ldg(a.xm + j);
-            kxS.add(w * xmassj);
-            whomegaS.add(dterh * xmassj);
-            wrho0S.add(dterh * T(pj.m));
         }
-        kxS.flush();
-        whomegaS.flush();
-        wrho0S.flush();
+        else
+        {
+            T vloc = T(sqrt(r2)) * hInv;
+            w      = kernelW(a.wh, k, vloc);
+            T dw   = kernelDW(a.whd, k, vloc);
+            dterh  = -prodSum(T(3), w, vloc, dw);
+        }
+        T xmassj   = __ldg(a.xm + j);
+        kxS.add(w * xmassj);
+        whomegaS.add(dterh * xmassj);
+        wrho0S.add(dterh * T(pj.m));
+        });
+        foldChunks<kSplit>(round * kSplit, t.numChunks, kxS, whomegaS, wrho0S);
     }
+    if (kSplit > 1 && (!valid || t.sub != 0)) { return; }
     T kxi      = kxS.get() * (k.K * h3Inv);
     T whomegai = whomegaS.get() * (k.K * h3Inv * hInv);
     T wrho0i   = wrho0S.get() * (k.K * h3Inv * hInv);
@@ -147,10 +141,10 @@ __global__ void __launch_bounds__(kChainMaxThreads, sizeof(T) == 4 ? 6 : 0)
         a.tape.whomega[t.i] = whomegai;
         a.tape.wrho0[t.i]   = wrho0i;
     }
-    whomegai   = whomegai * mi / xmassi + (kxi - k.K * xmassi * h3Inv) * wrho0i;
+    whomegai   = fma(fma(-(k.K * xmassi), h3Inv, kxi), wrho0i, whomegai * mi / xmassi);
     T rhoi     = kxi * mi / xmassi;
     T dhdrho   = -hi / (rhoi * T(3));
-    T gradhi   = T(1) - dhdrho * whomegai;
+    T gradhi   = fma(-dhdrho, whomegai, T(1));
 
     // EOS in FP64 (per particle): rho = kx m / xm, p = rho u (gamma - 1), c = sqrt(gamma u (gamma - 1))
     double gamma = k.gamma, cv = k.cv;
@@ -208,14 +202,16 @@ __device__ __forceinline__ int expOf(T v)
 // FP32: at most 80 registers (three 256-thread blocks per SM), as MomentumEnergy: measured 1.04 -> 0.95 ms at 128^3
 // against 87 registers. FP64 ran the two list passes of the reference before, bound by its FP64 pipe and the second
 // gather: 2.10 -> 1.16 ms at 101^3.
-template<class T, int kMode>
-__global__ void __launch_bounds__(kChainMaxThreads, sizeof(T) == 4 ? 3 : 0)
+template<class T, int kMode, int kSplit>
+__global__ void __launch_bounds__(kChainMaxThreads, sizeof(T) == 4 && kSplit == 1 ? 3 : 0)
     iadDivvCurlvFusedKernel(ChainArrays<T> a, HydroConsts<T> k, DevBox box)
 {
     Target t;
-    bool valid     = chainTarget<kMode>(a, k.ngmax, t);
-    double divvOut = -INFINITY;
-    if (valid)
+    const bool valid = chainTarget<kMode, kSplit>(a, k.ngmax, t);
+    double divvOut   = -INFINITY;
+    BlockSum<T> s11, s12, s13, s22, s23, s33;
+    BlockSum<T> mxx, mxy, mxz, myx, myy, myz, mzx, mzy, mzz;
+    if (kSplit > 1 || valid)
     {
         Pos<T> pi      = posOf(a, t.i);
         double hiD     = a.h[t.i];
@@ -223,61 +219,44 @@ __global__ void __launch_bounds__(kChainMaxThreads, sizeof(T) == 4 ? 3 : 0)
         T hiInv        = T(1) / hi;
         T hh           = T(0.5) * hiInv * hiInv;
         HydroRec<T> hr = a.hrec[t.i];
-
-        BlockSum<T> s11, s12, s13, s22, s23, s33;
-        BlockSum<T> mxx, mxy, mxz, myx, myy, myz, mzx, mzy, mzz;
-        for (unsigned q0 = 0; q0 < t.count; q0 += kNbChunk)
+        for (unsigned round = 0; round < t.rounds; ++round)
         {
-            uint32_t js[kNbChunk];
-            loadChunk(a.nidx, t, t.ngPad, q0, js);
-            unsigned qn = min(kNbChunk, t.count - q0);
-#pragma unroll
-            for (unsigned q = 0; q < kNbChunk; ++q)
-            {
-                if (q >= qn) { break; }
-                uint32_t j     = js[q];
-                Pos<T> pj      = posOf(a, j);
-                HydroRec<T> hj = loadHydro(a.hrec + j);
-                Sep<T> r       = separation(pi, pj, 2.0 * hiD, box, k);
-                T r2           = r.rx * r.rx + r.ry * r.ry + r.rz * r.rz;
-                T w            = kernelWr2(a.wh, k, r2, hiInv, hh);
-                T voljW        = hj.vol * w;
-                s11.add(r.rx * r.rx * voljW);
-                s12.add(r.rx * r.ry * voljW);
-                s13.add(r.rx * r.rz * voljW);
-                s22.add(r.ry * r.ry * voljW);
-                s23.add(r.ry * r.rz * voljW);
-                s33.add(r.rz * r.rz * voljW);
-                T xw = hj.xm * w;
-                T fx = (hj.vx - hr.vx) * xw;
-                T fy = (hj.vy - hr.vy) * xw;
-                T fz = (hj.vz - hr.vz) * xw;
-                mxx.add(fx * r.rx);
-                mxy.add(fx * r.ry);
-                mxz.add(fx * r.rz);
-                myx.add(fy * r.rx);
-                myy.add(fy * r.ry);
-                myz.add(fy * r.rz);
-                mzx.add(fz * r.rx);
-                mzy.add(fz * r.ry);
-                mzz.add(fz * r.rz);
-            }
-            s11.flush();
-            s12.flush();
-            s13.flush();
-            s22.flush();
-            s23.flush();
-            s33.flush();
-            mxx.flush();
-            mxy.flush();
-            mxz.flush();
-            myx.flush();
-            myy.flush();
-            myz.flush();
-            mzx.flush();
-            mzy.flush();
-            mzz.flush();
+            overChunk<kSplit, false>(a.nidx, t, round, [&](uint32_t j) {
+            Pos<T> pj      = posOf(a, j);
+            HydroRec<T> hj = loadHydro(a.hrec + j);
+            Sep<T> r       = separation(pi, pj, 2.0 * hiD, box, k);
+            T r2           = dot3(r.rx, r.ry, r.rz, r.rx, r.ry, r.rz);
+            T w            = kernelWr2(a.wh, k, r2, hiInv, hh);
+            T voljW        = hj.vol * w;
+            s11.add(r.rx * r.rx * voljW);
+            s12.add(r.rx * r.ry * voljW);
+            s13.add(r.rx * r.rz * voljW);
+            s22.add(r.ry * r.ry * voljW);
+            s23.add(r.ry * r.rz * voljW);
+            s33.add(r.rz * r.rz * voljW);
+            T xw = hj.xm * w;
+            T fx = (hj.vx - hr.vx) * xw;
+            T fy = (hj.vy - hr.vy) * xw;
+            T fz = (hj.vz - hr.vz) * xw;
+            mxx.add(fx * r.rx);
+            mxy.add(fx * r.ry);
+            mxz.add(fx * r.rz);
+            myx.add(fy * r.rx);
+            myy.add(fy * r.ry);
+            myz.add(fy * r.rz);
+            mzx.add(fz * r.rx);
+            mzy.add(fz * r.ry);
+            mzz.add(fz * r.rz);
+            });
+            foldChunks<kSplit>(round * kSplit, t.numChunks, s11, s12, s13, s22, s23, s33, mxx, mxy, mxz, myx, myy, myz,
+                               mzx, mzy, mzz);
         }
+    }
+    if (valid && t.sub == 0)
+    {
+        T hi           = T(a.h[t.i]);
+        T hiInv        = T(1) / hi;
+        HydroRec<T> hr = a.hrec[t.i];
         T tau11 = s11.get(), tau12 = s12.get(), tau13 = s13.get();
         T tau22 = s22.get(), tau23 = s23.get(), tau33 = s33.get();
         int expSum = expOf(tau11) + expOf(tau12) + expOf(tau13) + expOf(tau22) + expOf(tau23) + expOf(tau33);
@@ -288,16 +267,18 @@ __global__ void __launch_bounds__(kChainMaxThreads, sizeof(T) == 4 ? 3 : 0)
         tau22 *= norm;
         tau23 *= norm;
         tau33 *= norm;
-        T det = tau11 * tau22 * tau33 + T(2) * tau12 * tau23 * tau13 - tau11 * tau23 * tau23 - tau22 * tau13 * tau13 -
-                tau33 * tau12 * tau12;
+        T det = prodSum(tau11 * tau22, tau33, T(2) * tau12 * tau23, tau13);
+        det   = fma(-(tau11 * tau23), tau23, det);
+        det   = fma(-(tau22 * tau13), tau13, det);
+        det   = fma(-(tau33 * tau12), tau12, det);
         T factor = norm * (hi * hi * hi) / (det * k.K);
         if (isnan(factor) && t.count == 0) { factor = T(0); }
-        T c11i = (tau22 * tau33 - tau23 * tau23) * factor;
-        T c12i = (tau13 * tau23 - tau33 * tau12) * factor;
-        T c13i = (tau12 * tau23 - tau22 * tau13) * factor;
-        T c22i = (tau11 * tau33 - tau13 * tau13) * factor;
-        T c23i = (tau13 * tau12 - tau11 * tau23) * factor;
-        T c33i = (tau11 * tau22 - tau12 * tau12) * factor;
+        T c11i = prodDiff(tau22, tau33, tau23, tau23) * factor;
+        T c12i = prodDiff(tau13, tau23, tau33, tau12) * factor;
+        T c13i = prodDiff(tau12, tau23, tau22, tau13) * factor;
+        T c22i = prodDiff(tau11, tau33, tau13, tau13) * factor;
+        T c23i = prodDiff(tau13, tau12, tau11, tau23) * factor;
+        T c33i = prodDiff(tau11, tau22, tau12, tau12) * factor;
 
         // dV_ab = -sum_c C_bc M_ac
         T M[3][3] = {{mxx.get(), mxy.get(), mxz.get()}, {myx.get(), myy.get(), myz.get()},
@@ -310,7 +291,7 @@ __global__ void __launch_bounds__(kChainMaxThreads, sizeof(T) == 4 ? 3 : 0)
 #pragma unroll
             for (int q = 0; q < 3; ++q)
             {
-                dV[p][q] = -(C[q][0] * M[p][0] + C[q][1] * M[p][1] + C[q][2] * M[p][2]);
+                dV[p][q] = -dot3(C[q][0], C[q][1], C[q][2], M[p][0], M[p][1], M[p][2]);
             }
         }
         T hiInv3 = hiInv * hiInv * hiInv;
@@ -319,7 +300,7 @@ __global__ void __launch_bounds__(kChainMaxThreads, sizeof(T) == 4 ? 3 : 0)
         T cx     = dV[2][1] - dV[1][2];
         T cy     = dV[0][2] - dV[2][0];
         T cz     = dV[1][0] - dV[0][1];
-        T curlv  = normKx * sqrt(cx * cx + cy * cy + cz * cz);
+        T curlv  = normKx * sqrt(dot3(cx, cy, cz, cx, cy, cz));
         if constexpr (kMode & kModeAvClean)
         {
             DVRec<T> g{{normKx * dV[0][0], normKx * (dV[0][1] + dV[1][0]), normKx * (dV[0][2] + dV[2][0]),
@@ -356,12 +337,13 @@ __global__ void __launch_bounds__(kChainMaxThreads, sizeof(T) == 4 ? 3 : 0)
 // 0.817 -> 0.795 ms at 128^3 against 256; at most 56 registers for three such blocks per SM. FP64 keeps the common
 // bound with no block minimum (0): an explicit minimum of 1 raised it from 96 to 108 registers and slowed it from
 // 2.45 to 2.64 ms at 128 threads.
-template<class T, int kMode>
-__global__ void __launch_bounds__(sizeof(T) == 4 ? kAvMaxThreads : kChainMaxThreads, sizeof(T) == 4 ? 3 : 0)
+template<class T, int kMode, int kSplit>
+__global__ void __launch_bounds__(sizeof(T) == 4 ? kAvMaxThreads : kChainMaxThreads, sizeof(T) == 4 && kSplit == 1 ? 3 : 0)
     avSwitchesKernel(ChainArrays<T> a, HydroConsts<T> k, DevBox box, double dt)
 {
     Target t;
-    if (!chainTarget<kMode>(a, k.ngmax, t)) { return; }
+    const bool valid = chainTarget<kMode, kSplit>(a, k.ngmax, t);
+    if (kSplit == 1 && !valid) { return; }
     Pos<T> pi      = posOf(a, t.i);
     double hiD     = a.h[t.i];
     HydroRec<T> hr = a.hrec[t.i];
@@ -377,57 +359,50 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? kAvMaxThreads : kChainMaxThre
 
     BlockSum<T> gx, gy, gz;
     int vsigJ = -1;
-    for (unsigned q0 = 0; q0 < t.count; q0 += kNbChunk)
+    for (unsigned round = 0; round < t.rounds; ++round)
     {
-        uint32_t js[kNbChunk];
-        loadChunk(a.nidx, t, t.ngPad, q0, js);
-        unsigned qn = min(kNbChunk, t.count - q0);
-#pragma unroll
-        for (unsigned q = 0; q < kNbChunk; ++q)
+        overChunk<kSplit, false>(a.nidx, t, round, [&](uint32_t j) {
+        Pos<T> pj      = posOf(a, j);
+        AVRec<T> hj    = loadAV(a.avrec + j);
+        T divvJ        = hj.divv;
+        Sep<T> r       = separation(pi, pj, 2.0 * hiD, box, k);
+        T r2           = dot3(r.rx, r.ry, r.rz, r.rx, r.ry, r.rz);
+        T rv           = dot3(r.rx, r.ry, r.rz, hr.vx - hj.vx, hr.vy - hj.vy, hr.vz - hj.vz);
+        // 1/r from one rsqrt: 3 r.v / r without a division, and in FP64 r itself for the kernel's table
+        T vsig = T(0);
+        [[maybe_unused]] T rinv = T(0);
+        if constexpr (sizeof(T) == 8) { rinv = rsqrt(r2); }
+        if (rv < T(0))
         {
-            if (q >= qn) { break; }
-            uint32_t j = js[q];
-            Pos<T> pj      = posOf(a, j);
-            AVRec<T> hj    = loadAV(a.avrec + j);
-            T divvJ        = hj.divv;
-            Sep<T> r       = separation(pi, pj, 2.0 * hiD, box, k);
-            T r2           = r.rx * r.rx + r.ry * r.ry + r.rz * r.rz;
-            T rv           = r.rx * (hr.vx - hj.vx) + r.ry * (hr.vy - hj.vy) + r.rz * (hr.vz - hj.vz);
-            // 1/r from one rsqrt: 3 r.v / r without a division, and in FP64 r itself for the kernel's table
-            T vsig = T(0);
-            [[maybe_unused]] T rinv = T(0);
-            if constexpr (sizeof(T) == 8) { rinv = rsqrt(r2); }
-            if (rv < T(0))
-            {
-                if constexpr (sizeof(T) == 4) { rinv = rsqrtf(r2); }
-                vsig = ci + hj.c - T(3) * rv * rinv;
-            }
-            if constexpr (kMode & kModeTape)
-            {
-                if (!(vijsignalI > vsig)) { vsigJ = int(j); }
-            }
-            vijsignalI = vijsignalI > vsig ? vijsignalI : vsig;
-            T W;
-            if constexpr (sizeof(T) == 4) { W = kernelWr2(a.wh, k, r2, hiInv, hh); }
-            else { W = kernelW(a.wh, k, r2 * rinv * hiInv); }
-            // sum fac W r and apply -C_i once after the loop (the same vector, 9 FMAs less per pair)
-            T sw = hj.vol * (divvI - divvJ) * (KhiInv3 * W);
-            gx.add(sw * r.rx);
-            gy.add(sw * r.ry);
-            gz.add(sw * r.rz);
+            if constexpr (sizeof(T) == 4) { rinv = rsqrtf(r2); }
+            vsig = fma(T(-3) * rv, rinv, ci + hj.c);
         }
-        gx.flush();
-        gy.flush();
-        gz.flush();
+        if constexpr (kMode & kModeTape)
+        {
+            if (!(vijsignalI > vsig)) { vsigJ = int(j); }
+        }
+        vijsignalI = vijsignalI > vsig ? vijsignalI : vsig;
+        T W;
+        if constexpr (sizeof(T) == 4) { W = kernelWr2(a.wh, k, r2, hiInv, hh); }
+        else { W = kernelW(a.wh, k, r2 * rinv * hiInv); }
+        // sum fac W r and apply -C_i once after the loop (the same vector, 9 FMAs less per pair)
+        T sw = hj.vol * (divvI - divvJ) * (KhiInv3 * W);
+        gx.add(sw * r.rx);
+        gy.add(sw * r.ry);
+        gz.add(sw * r.rz);
+        });
+        foldChunks<kSplit>(round * kSplit, t.numChunks, gx, gy, gz);
     }
+    vijsignalI = maxOverSplit<kSplit>(vijsignalI);
+    if (kSplit > 1 && (!valid || t.sub != 0)) { return; }
     T gdx = gx.get(), gdy = gy.get(), gdz = gz.get();
     {
         T sx = gdx, sy = gdy, sz = gdz;
-        gdx  = -(gr.c11 * sx + gr.c12 * sy + gr.c13 * sz);
-        gdy  = -(gr.c12 * sx + gr.c22 * sy + gr.c23 * sz);
-        gdz  = -(gr.c13 * sx + gr.c23 * sy + gr.c33 * sz);
+        gdx  = -dot3(gr.c11, gr.c12, gr.c13, sx, sy, sz);
+        gdy  = -dot3(gr.c12, gr.c22, gr.c23, sx, sy, sz);
+        gdz  = -dot3(gr.c13, gr.c23, gr.c33, sx, sy, sz);
     }
-    T graddivv = sqrt(gdx * gdx + gdy * gdy + gdz * gdz);
+    T graddivv = sqrt(dot3(gdx, gdy, gdz, gdx, gdy, gdz));
     if constexpr (kMode & kModeTape)
     {
         a.tape.gx[t.i]    = gdx;
@@ -441,7 +416,7 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? kAvMaxThreads : kChainMaxThre
     if (divvI < T(0))
     {
         T aConst = hi * hi * graddivv;
-        alphaloc = k.alphamax * aConst / (aConst + hi * fabs(divvI) + T(0.05) * ci);
+        alphaloc = k.alphamax * aConst / fma(T(0.05), ci, fma(hi, fabs(divvI), aConst));
     }
     if (alphaloc >= alphaI) { alphaI = alphaloc; }
     else
@@ -450,7 +425,7 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? kAvMaxThreads : kChainMaxThre
         T alphadot = alphaloc >= k.alphamin ? (alphaloc - alphaI) / decay : (k.alphamin - alphaI) / decay;
         double dtq = dt;
         if constexpr (kMode & kModeBatch) { dtq = a.batch.dt[a.batch.inst[t.i]]; }
-        alphaI += alphadot * T(dtq);
+        alphaI = fma(alphadot, T(dtq), alphaI);
     }
     a.alpha[t.i]      = double(alphaI);
     a.grec[t.i].alpha = alphaI; // the alpha slot of the record is not read by this kernel
@@ -466,14 +441,14 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? kAvMaxThreads : kChainMaxThre
 // 3.98 ms at 101^3, the result unchanged to 4e-15.
 // FP32 without AV cleaning: at most 80 registers (three 256-thread blocks per SM) keeps more warps resident for the
 // gathers; measured 2.11 -> 2.05 ms at 128^3 against 96 registers (the AV-cleaning form would spill)
-template<class T, int kMode>
-__global__ void __launch_bounds__(kChainMaxThreads, (sizeof(T) == 4 && !(kMode & kModeAvClean)) ? 3 : 1)
+template<class T, int kMode, int kSplit>
+__global__ void __launch_bounds__(kChainMaxThreads, (sizeof(T) == 4 && kSplit == 1 && !(kMode & kModeAvClean)) ? 3 : 1)
     momentumEnergyKernel(ChainArrays<T> a, HydroConsts<T> k, DevBox box)
 {
     Target t;
-    bool valid   = chainTarget<kMode>(a, k.ngmax, t);
-    double dtMin = INFINITY;
-    if (valid)
+    const bool valid = chainTarget<kMode, kSplit>(a, k.ngmax, t);
+    double dtMin     = INFINITY;
+    if (kSplit > 1 || valid)
     {
         Pos<T> pi      = posOf(a, t.i);
         double hiD     = a.h[t.i];
@@ -516,7 +491,7 @@ __global__ void __launch_bounds__(kChainMaxThreads, (sizeof(T) == 4 && !(kMode &
                 HydroRec<T> hj = loadHydro(a.hrec + j);
                 GradRec<T> gj  = loadGrad(a.grec + j);
                 Sep<T> r       = separation(pi, pj, 2.0 * hiD, box, k);
-                float r2       = r.rx * r.rx + r.ry * r.ry + r.rz * r.rz;
+                float r2       = dot3(r.rx, r.ry, r.rz, r.rx, r.ry, r.rz);
                 float rinv     = rsqrtf(r2);
                 float dist     = r2 * rinv;
                 float vxij     = hr.vx - hj.vx;
@@ -546,12 +521,12 @@ __global__ void __launch_bounds__(kChainMaxThreads, (sizeof(T) == 4 && !(kMode &
                 float cj     = hj.c;
                 float xmassj = hj.xm;
                 float rhoj   = fdiv(mj, hj.vol);
-                float rv     = r.rx * vxij + r.ry * vyij + r.rz * vzij;
+                float rv     = dot3(r.rx, r.ry, r.rz, vxij, vyij, vzij);
                 float wij    = rv * rinv;
                 float visc   = 0.0f;
                 if (wij < 0.0f)
                 {
-                    float vijSignal = (alphaI + gj.alpha) * 0.25f * (ci + cj) - 2.0f * wij;
+                    float vijSignal = fmaf((alphaI + gj.alpha) * 0.25f, ci + cj, -2.0f * wij);
                     visc            = -vijSignal * wij;
                 }
                 float vijsignal = 0.5f * (ci + cj) - 2.0f * wij;
@@ -573,8 +548,8 @@ __global__ void __launch_bounds__(kChainMaxThreads, (sizeof(T) == 4 && !(kMode &
                 {
                     float sigma = k.ramp * (fdiv(dRho, sRho) - k.Atmin);
                     float lxj   = log2f(xmassj);
-                    aMom        = exp2f((2.0f - sigma) * lxi + sigma * lxj);
-                    bMom        = exp2f((2.0f - sigma) * lxj + sigma * lxi);
+                    aMom        = exp2f(prodSum(2.0f - sigma, lxi, sigma, lxj));
+                    bMom        = exp2f(prodSum(2.0f - sigma, lxj, sigma, lxi));
                 }
                 float aVisc = mj * invRhoi * visc;
                 float bVisc = hj.vol * visc;
@@ -582,13 +557,13 @@ __global__ void __launch_bounds__(kChainMaxThreads, (sizeof(T) == 4 && !(kMode &
                 float2 dv = __ffma2_rn(tA3, make_float2(vzij, vzij),
                                        __ffma2_rn(tA2, make_float2(vyij, vyij),
                                                   __fmul2_rn(tA1, make_float2(vxij, vxij))));
-                aViscE.add(0.5f * (aVisc * dv.x + bVisc * dv.y));
+                aViscE.add(0.5f * prodSum(aVisc, dv.x, bVisc, dv.y));
                 energyS.add(mj * aMom * dv.x);
-                float cI = mj * prhoi * aMom + 0.5f * aVisc;
-                float cJ = mj * hj.prho * bMom + 0.5f * bVisc;
-                momX.add(cI * tA1.x + cJ * tA1.y);
-                momY.add(cI * tA2.x + cJ * tA2.y);
-                momZ.add(cI * tA3.x + cJ * tA3.y);
+                float cI = prodSum(mj * prhoi, aMom, 0.5f, aVisc);
+                float cJ = prodSum(mj * hj.prho, bMom, 0.5f, bVisc);
+                momX.add(prodSum(cI, tA1.x, cJ, tA1.y));
+                momY.add(prodSum(cI, tA2.x, cJ, tA2.y));
+                momZ.add(prodSum(cI, tA3.x, cJ, tA3.y));
             }
             else
             {
@@ -596,7 +571,7 @@ __global__ void __launch_bounds__(kChainMaxThreads, (sizeof(T) == 4 && !(kMode &
                 HydroRec<T> hj = loadHydro(a.hrec + j);
                 GradRec<T> gj  = loadGrad(a.grec + j);
                 Sep<T> r       = separation(pi, pj, 2.0 * hiD, box, k);
-                T r2           = r.rx * r.rx + r.ry * r.ry + r.rz * r.rz;
+                T r2           = dot3(r.rx, r.ry, r.rz, r.rx, r.ry, r.rz);
                 // 1/r from one rsqrt (r and w_ij = r.v / r without a square root or a division), m_j / rho_j as
                 // vol_j, and the Atwood thresholds compared without a division (FP32: 1.68 -> 1.58 ms at 128^3; the
                 // errors against FP64 unchanged)
@@ -613,18 +588,18 @@ __global__ void __launch_bounds__(kChainMaxThreads, (sizeof(T) == 4 && !(kMode &
                 T Wi           = hiInv3 * kernelW(a.wh, k, v1);
                 T Wj           = hjInv3 * kernelW(a.wh, k, v2);
 
-                T tA1i = -(gr.c11 * r.rx + gr.c12 * r.ry + gr.c13 * r.rz) * Wi;
-                T tA2i = -(gr.c12 * r.rx + gr.c22 * r.ry + gr.c23 * r.rz) * Wi;
-                T tA3i = -(gr.c13 * r.rx + gr.c23 * r.ry + gr.c33 * r.rz) * Wi;
-                T tA1j = -(gj.c11 * r.rx + gj.c12 * r.ry + gj.c13 * r.rz) * Wj;
-                T tA2j = -(gj.c12 * r.rx + gj.c22 * r.ry + gj.c23 * r.rz) * Wj;
-                T tA3j = -(gj.c13 * r.rx + gj.c23 * r.ry + gj.c33 * r.rz) * Wj;
+                T tA1i = -dot3(gr.c11, gr.c12, gr.c13, r.rx, r.ry, r.rz) * Wi;
+                T tA2i = -dot3(gr.c12, gr.c22, gr.c23, r.rx, r.ry, r.rz) * Wi;
+                T tA3i = -dot3(gr.c13, gr.c23, gr.c33, r.rx, r.ry, r.rz) * Wi;
+                T tA1j = -dot3(gj.c11, gj.c12, gj.c13, r.rx, r.ry, r.rz) * Wj;
+                T tA2j = -dot3(gj.c12, gj.c22, gj.c23, r.rx, r.ry, r.rz) * Wj;
+                T tA3j = -dot3(gj.c13, gj.c23, gj.c33, r.rx, r.ry, r.rz) * Wj;
 
                 T mj     = T(pj.m);
                 T cj     = hj.c;
                 T xmassj = hj.xm;
 
-                T rv   = r.rx * vxij + r.ry * vyij + r.rz * vzij;
+                T rv   = dot3(r.rx, r.ry, r.rz, vxij, vyij, vzij);
                 if constexpr (kMode & kModeAvClean)
                 {
                     T gradVj[6];
@@ -635,7 +610,7 @@ __global__ void __launch_bounds__(kChainMaxThreads, (sizeof(T) == 4 && !(kMode &
                 T visc = T(0);
                 if (wij < T(0))
                 {
-                    T vijSignal = (alphaI + gj.alpha) * T(0.25) * (ci + cj) - T(2) * wij;
+                    T vijSignal = fma((alphaI + gj.alpha) * T(0.25), ci + cj, T(-2) * wij);
                     visc        = -vijSignal * wij;
                 }
                 T vijsignal = T(0.5) * (ci + cj) - T(2) * wij;
@@ -661,8 +636,8 @@ __global__ void __launch_bounds__(kChainMaxThreads, (sizeof(T) == 4 && !(kMode &
                     if constexpr (sizeof(T) == 4)
                     {
                         T lxj = log2f(xmassj);
-                        aMom  = exp2f((T(2) - sigma) * lxi + sigma * lxj);
-                        bMom  = exp2f((T(2) - sigma) * lxj + sigma * lxi);
+                        aMom  = exp2f(prodSum(T(2) - sigma, lxi, sigma, lxj));
+                        bMom  = exp2f(prodSum(T(2) - sigma, lxj, sigma, lxi));
                     }
                     else
                     {
@@ -676,73 +651,95 @@ __global__ void __launch_bounds__(kChainMaxThreads, (sizeof(T) == 4 && !(kMode &
 
                 T aVisc  = mj * invRhoi * visc;
                 T bVisc  = hj.vol * visc;
-                T aViscX = T(0.5) * (aVisc * tA1i + bVisc * tA1j);
-                T aViscY = T(0.5) * (aVisc * tA2i + bVisc * tA2j);
-                T aViscZ = T(0.5) * (aVisc * tA3i + bVisc * tA3j);
-                aViscE.add(aViscX * vxij + aViscY * vyij + aViscZ * vzij);
-                energyS.add(mj * aMom * (vxij * tA1i + vyij * tA2i + vzij * tA3i));
+                T aViscX = T(0.5) * prodSum(aVisc, tA1i, bVisc, tA1j);
+                T aViscY = T(0.5) * prodSum(aVisc, tA2i, bVisc, tA2j);
+                T aViscZ = T(0.5) * prodSum(aVisc, tA3i, bVisc, tA3j);
+                aViscE.add(dot3(aViscX, aViscY, aViscZ, vxij, vyij, vzij));
+                energyS.add(mj * aMom * dot3(vxij, vyij, vzij, tA1i, tA2i, tA3i));
                 T momI = mj * prhoi * aMom;
                 T momJ = mj * hj.prho * bMom;
-                momX.add(momI * tA1i + momJ * tA1j + aViscX);
-                momY.add(momI * tA2i + momJ * tA2j + aViscY);
-                momZ.add(momI * tA3i + momJ * tA3j + aViscZ);
+                momX.add(fma(momI, tA1i, fma(momJ, tA1j, aViscX)));
+                momY.add(fma(momI, tA2i, fma(momJ, tA2j, aViscY)));
+                momZ.add(fma(momI, tA3i, fma(momJ, tA3j, aViscZ)));
             }
         };
-        for (unsigned q0 = 0; q0 < t.count; q0 += kNbChunk)
+        // one pair per iteration: the unrolled 8-pair body overflowed the instruction cache (FP32 2.04 -> 1.71 ms at
+        // 128^3; unrolled by 2 or 4 it ran slower too, 1.59 against 1.48 ms; FP64 2.23 -> 2.12 ms at 101^3)
+        for (unsigned round = 0; round < t.rounds; ++round)
         {
-            uint32_t js[kNbChunk];
-            loadChunk(a.nidx, t, t.ngPad, q0, js);
-            unsigned qn = min(kNbChunk, t.count - q0);
-            // one pair per iteration: the unrolled 8-pair body overflowed the instruction cache (FP32 2.04 -> 1.71 ms
-            // at 128^3; unrolled by 2 or 4 it ran slower too, 1.59 against 1.48 ms; FP64 2.23 -> 2.12 ms at 101^3)
-#pragma unroll 1
-            for (unsigned q = 0; q < qn; ++q)
+            overChunk<kSplit, true>(a.nidx, t, round, pairTerm);
+            foldChunks<kSplit>(round * kSplit, t.numChunks, momX, momY, momZ, energyS, aViscE);
+        }
+        maxvsignalI = maxOverSplit<kSplit>(maxvsignalI);
+        if (valid && t.sub == 0)
+        {
+            if constexpr (kMode & kModeTape)
             {
-                pairTerm(popChunk(js));
+                a.tape.energy[t.i] = energyS.get();
+                a.tape.avisc[t.i]  = aViscE.get();
             }
-            momX.flush();
-            momY.flush();
-            momZ.flush();
-            energyS.flush();
-            aViscE.flush();
-        }
-        if constexpr (kMode & kModeTape)
-        {
-            a.tape.energy[t.i] = energyS.get();
-            a.tape.avisc[t.i]  = aViscE.get();
-        }
-        T aViscEnergy = aViscE.get() > T(0) ? aViscE.get() : T(0);
-        a.du[t.i] = double(k.K * (prhoi * energyS.get() + T(0.5) * aViscEnergy));
-        a.ax[t.i] = -k.K * momX.get();
-        a.ay[t.i] = -k.K * momY.get();
-        a.az[t.i] = -k.K * momZ.get();
+            T aViscEnergy = aViscE.get() > T(0) ? aViscE.get() : T(0);
+            a.du[t.i] = double(k.K * prodSum(prhoi, energyS.get(), T(0.5), aViscEnergy));
+            a.ax[t.i] = -k.K * momX.get();
+            a.ay[t.i] = -k.K * momY.get();
+            a.az[t.i] = -k.K * momZ.get();
 
-        double v = maxvsignalI > T(0) ? double(maxvsignalI) : double(ci);
-        // FP32: h read again here rather than kept in two registers across the pair loop (1.478 -> 1.465 ms)
-        double hEnd = sizeof(T) == 4 ? a.h[t.i] : hiD;
-        dtMin       = hEnd > 0.0 ? k.Kcour * hEnd / v : INFINITY;
+            double v = maxvsignalI > T(0) ? double(maxvsignalI) : double(ci);
+            // FP32: h read again here rather than kept in two registers across the pair loop (1.478 -> 1.465 ms)
+            double hEnd = sizeof(T) == 4 ? a.h[t.i] : hiD;
+            dtMin       = hEnd > 0.0 ? k.Kcour * hEnd / v : INFINITY;
+        }
     }
     if constexpr (kMode & kModeList)
     {
         // the group's Courant step lowers its block time step (momentum_energy_gpu.cu:96-103); rounding to float is
         // monotonic, so min(float, double) stored as float equals the min of the float values
-        unsigned w  = unsigned((blockIdx.x * size_t(blockDim.x) + threadIdx.x) >> 5);
+        unsigned w  = unsigned((blockIdx.x * size_t(blockDim.x) + threadIdx.x) / (32 * kSplit));
         double gmin = dtMin;
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1)
         {
             gmin = fmin(gmin, __shfl_xor_sync(0xffffffffu, gmin, off));
         }
-        if ((threadIdx.x & 31) == 0 && w < a.numListed) { a.groupDt[w] = fminf(a.groupDt[w], float(gmin)); }
+        if ((threadIdx.x & 31) == 0 && w < a.numListed)
+        {
+            // a group's targets span kSplit warps; time steps are positive, so their bits order as integers
+            if constexpr (kSplit == 1) { a.groupDt[w] = fminf(a.groupDt[w], float(gmin)); }
+            else { atomicMin(reinterpret_cast<int*>(a.groupDt + w), __float_as_int(float(gmin))); }
+        }
     }
     reduceOrdered<false, (kMode & kModeBatch) != 0>(dtMin, a.n, a.reduce + 1, a.batch, 1);
 }
 
 template<class T>
+size_t chainTargets(const ChainArrays<T>& a)
+{
+    return a.groupList ? size_t(a.numListed) * 32 : a.n;
+}
+
+/*! Lanes that share a target. A launch of few targets leaves most of the GPU idle while each thread walks its ~100
+ *  neighbours alone; several lanes take a chunk of eight neighbours each. The sums are the same bit for bit.
+ *  Measured (us for the five loops, one lane / four / eight): 4,096 targets FP32 215 / 89 / 73, 9,261 targets FP64
+ *  409 / 164 / 147, 24,000 targets FP32 (AV cleaning) 245 / 147 / 165, 27,000 targets FP64 420 / 266 / 297, 125,000
+ *  targets FP32 475 / 491 / 610. */
+template<class T>
+int chainSplit(const ChainArrays<T>& a)
+{
+    size_t targets = chainTargets(a);
+    return targets <= kEightLaneTargets ? 8 : targets <= kFourLaneTargets ? 4 : 1;
+}
+
+template<class T>
 unsigned chainBlocks(const ChainArrays<T>& a)
 {
-    if (a.groupList) { return ceilDiv(size_t(a.numListed) * 32, unsigned(a.threads)); }
-    return ceilDiv(a.n, size_t(a.threads));
+    return ceilDiv(chainTargets(a), size_t(a.threads));
+}
+
+//! blocks of kSplitThreads threads for `lanes` lanes per target
+template<class T>
+unsigned splitBlocks(const ChainArrays<T>& a, int lanes)
+{
+    return ceilDiv(chainTargets(a) * lanes, size_t(kSplitThreads));
 }
 
 } // namespace
@@ -765,30 +762,37 @@ int chainModeAv(const ChainArrays<T>& a)
     return (mode & kModeTape) ? -1 : (mode | kModeAvClean); // the adjoint has no AV-cleaning variant
 }
 
+#define SPHB_LAUNCH(KERNEL, MODE, ...) KERNEL<T, (MODE), 1><<<chainBlocks(a), a.threads, 0, s>>>(__VA_ARGS__)
+#define SPHB_LAUNCH_SPLIT(KERNEL, MODE, ...)                                                                           \
+    switch (chainSplit(a))                                                                                              \
+    {                                                                                                                   \
+    case 8: KERNEL<T, (MODE), 8><<<splitBlocks(a, 8), kSplitThreads, 0, s>>>(__VA_ARGS__); break;                      \
+    case 4: KERNEL<T, (MODE), 4><<<splitBlocks(a, 4), kSplitThreads, 0, s>>>(__VA_ARGS__); break;                      \
+    default: SPHB_LAUNCH(KERNEL, MODE, __VA_ARGS__); break;                                                             \
+    }
+
+// the taped form keeps one lane per target (it records which neighbour sets the signal velocity), the ensemble's batch
+// form as well (its launches cover every member)
 #define SPHB_DISPATCH_AV(KERNEL, ...)                                                                                   \
     switch (chainModeAv(a))                                                                                             \
     {                                                                                                                   \
-    case 0: KERNEL<T, 0><<<chainBlocks(a), a.threads, 0, s>>>(__VA_ARGS__); break;                                    \
-    case kModeTape: KERNEL<T, kModeTape><<<chainBlocks(a), a.threads, 0, s>>>(__VA_ARGS__); break;                    \
-    case kModeBatch: KERNEL<T, kModeBatch><<<chainBlocks(a), a.threads, 0, s>>>(__VA_ARGS__); break;                  \
-    case kModeAvClean: KERNEL<T, kModeAvClean><<<chainBlocks(a), a.threads, 0, s>>>(__VA_ARGS__); break;              \
-    case kModeList: KERNEL<T, kModeList><<<chainBlocks(a), a.threads, 0, s>>>(__VA_ARGS__); break;                    \
-    case kModeAvClean | kModeList:                                                                                      \
-        KERNEL<T, kModeAvClean | kModeList><<<chainBlocks(a), a.threads, 0, s>>>(__VA_ARGS__);                          \
-        break;                                                                                                          \
-    case kModeAvClean | kModeBatch:                                                                                     \
-        KERNEL<T, kModeAvClean | kModeBatch><<<chainBlocks(a), a.threads, 0, s>>>(__VA_ARGS__);                         \
-        break;                                                                                                          \
+    case 0: SPHB_LAUNCH_SPLIT(KERNEL, 0, __VA_ARGS__) break;                                                            \
+    case kModeTape: SPHB_LAUNCH(KERNEL, kModeTape, __VA_ARGS__); break;                                                 \
+    case kModeBatch: SPHB_LAUNCH(KERNEL, kModeBatch, __VA_ARGS__); break;                                               \
+    case kModeAvClean: SPHB_LAUNCH_SPLIT(KERNEL, kModeAvClean, __VA_ARGS__) break;                                      \
+    case kModeList: SPHB_LAUNCH_SPLIT(KERNEL, kModeList, __VA_ARGS__) break;                                            \
+    case kModeAvClean | kModeList: SPHB_LAUNCH_SPLIT(KERNEL, kModeAvClean | kModeList, __VA_ARGS__) break;              \
+    case kModeAvClean | kModeBatch: SPHB_LAUNCH(KERNEL, kModeAvClean | kModeBatch, __VA_ARGS__); break;                 \
     default: return kErrArg;                                                                                            \
     }
 
 #define SPHB_DISPATCH(KERNEL, ...)                                                                                      \
     switch (chainMode(a))                                                                                               \
     {                                                                                                                   \
-    case 0: KERNEL<T, 0><<<chainBlocks(a), a.threads, 0, s>>>(__VA_ARGS__); break;                                    \
-    case kModeTape: KERNEL<T, kModeTape><<<chainBlocks(a), a.threads, 0, s>>>(__VA_ARGS__); break;                    \
-    case kModeBatch: KERNEL<T, kModeBatch><<<chainBlocks(a), a.threads, 0, s>>>(__VA_ARGS__); break;                  \
-    case kModeList: KERNEL<T, kModeList><<<chainBlocks(a), a.threads, 0, s>>>(__VA_ARGS__); break;                    \
+    case 0: SPHB_LAUNCH_SPLIT(KERNEL, 0, __VA_ARGS__) break;                                                            \
+    case kModeTape: SPHB_LAUNCH(KERNEL, kModeTape, __VA_ARGS__); break;                                                 \
+    case kModeBatch: SPHB_LAUNCH(KERNEL, kModeBatch, __VA_ARGS__); break;                                               \
+    case kModeList: SPHB_LAUNCH_SPLIT(KERNEL, kModeList, __VA_ARGS__) break;                                            \
     default: return kErrArg;                                                                                            \
     }
 

@@ -50,3 +50,19 @@ def test_fp64_forces_against_the_restatement(cuda_device, side, keep, coincident
         a, b = g.get(f), o.get(f)
         assert np.all(np.isfinite(a)), f
         assert np.max(np.abs(a - b)) <= 1e-12 * np.max(np.abs(b)), f
+
+
+@pytest.mark.parametrize("precision,av_clean", [("mixed", False), ("fp64", False), ("mixed", True)])
+@pytest.mark.parametrize("n", [1, 31, 33, 16384, 16385, 65536, 65537])
+def test_lanes_per_target_leave_the_sums_alone(cuda_device, n, precision, av_clean):
+    """Eight, four or one lane share a target by the number of targets; an ensemble's launches always use one. The same
+    particles give the same bits on both sides of either limit."""
+    from sphexa_b200.ensemble import Ensemble
+    from sphexa_b200.simulation import Simulation
+    ic = contrast(max(8, int(np.ceil(n ** (1.0 / 3.0)))), n)
+    ic["params"]["avClean"] = av_clean
+    sim, ens = Simulation(ic, precision), Ensemble([ic], precision)
+    sim.step()
+    ens.step(1, graph=False)
+    for f in FIELDS + ("x", "vx", "temp", "nc"):
+        assert np.array_equal(sim.get(f), ens.get(0, f), equal_nan=True), f
