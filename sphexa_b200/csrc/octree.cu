@@ -789,36 +789,302 @@ int focusUpdateCounts(FocusTree& f, const uint64_t* keys, size_t n, cudaStream_t
 
 } // namespace sphb
 
+// ------------------------------------------------------------------------------------------------------------------
+// The converged tree of sorted keys, directly
+//
+// The fixed point of the rebalance steps (split leaves with more than `bucket` keys above the deepest level, merge 8
+// sibling leaves with at most `bucket` together) is unique: the internal nodes are the nodes above the deepest level
+// with more than `bucket` keys. Let c_p be the deepest level of a node that holds the keys p - 1 and p, and E_p that of
+// a node that holds the keys p .. p + bucket (at most one above the deepest). The deepest internal node that holds key
+// p is then on level D_p = max(E_p, min(D_{p-1}, c_p)), and functions x -> max(e, min(x, c)) compose, so D is a scan. The
+// leaf of key p is on level D_p + 1, it starts at p if c_p <= D_p, and the empty leaves between two keys' leaves are the
+// children that the paths between them pass by. A second scan, of the leaves that each key opens, places them.
+// Two reads of the keys and one host read, instead of a rebalance, a scan, a recount and a host read for every few
+// levels, with buffers that grew in between: 150,000 leaves of 4,000,037 clustered keys 2.6 -> 0.2 ms.
+// ------------------------------------------------------------------------------------------------------------------
+namespace sphb
+{
+namespace
+{
+
+constexpr int kConvThreads = 256;
+constexpr int kConvItems   = 8;
+constexpr int kConvTile    = kConvThreads * kConvItems;
+
+//! x -> max(e, min(x, c)) on levels -1 .. 21
+struct LevelClamp
+{
+    int e, c;
+};
+
+__device__ __forceinline__ LevelClamp clampIdentity() { return {-1, int(kMaxLevel)}; }
+
+//! first f, then g
+__device__ __forceinline__ LevelClamp clampThen(LevelClamp f, LevelClamp g)
+{
+    return {max(g.e, min(f.e, g.c)), min(f.c, g.c)};
+}
+
+//! deepest level of a node that holds both keys
+__device__ __forceinline__ int commonLevel(uint64_t a, uint64_t b)
+{
+    return a == b ? int(kMaxLevel) : (int(__clzll((long long)(a ^ b))) - 1) / 3;
+}
+
+//! the keys below the removal key (the last leaf ends there)
+__device__ inline size_t keptKeys(const uint64_t* keys, size_t n) { return lowerBound(keys, n, kRootRange); }
+
+__device__ __forceinline__ LevelClamp clampOf(const uint64_t* __restrict__ keys, size_t n, unsigned bucket, size_t p)
+{
+    if (p >= n) { return clampIdentity(); }
+    uint64_t k = __ldg(keys + p);
+    int c      = p ? commonLevel(__ldg(keys + p - 1), k) : -1;
+    int e      = -1;
+    if (p + bucket < n) { e = min(commonLevel(k, __ldg(keys + p + bucket)), int(kMaxLevel) - 1); }
+    return {e, c};
+}
+
+//! exclusive scan of one clamp per thread over the block; *total receives the composition of all
+__device__ LevelClamp blockScanClamp(LevelClamp v, LevelClamp* total)
+{
+    __shared__ LevelClamp warpTotal[kConvThreads / 32 + 1];
+    int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    LevelClamp incl = v;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1)
+    {
+        LevelClamp o{__shfl_up_sync(0xffffffffu, incl.e, off), __shfl_up_sync(0xffffffffu, incl.c, off)};
+        if (lane >= off) { incl = clampThen(o, incl); }
+    }
+    if (lane == 31) { warpTotal[warp] = incl; }
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        LevelClamp run = clampIdentity();
+        for (int w = 0; w < kConvThreads / 32; ++w)
+        {
+            LevelClamp t = warpTotal[w];
+            warpTotal[w] = run;
+            run          = clampThen(run, t);
+        }
+        warpTotal[kConvThreads / 32] = run;
+    }
+    __syncthreads();
+    LevelClamp ex{__shfl_up_sync(0xffffffffu, incl.e, 1), __shfl_up_sync(0xffffffffu, incl.c, 1)};
+    if (lane == 0) { ex = clampIdentity(); }
+    ex     = clampThen(warpTotal[warp], ex);
+    *total = warpTotal[kConvThreads / 32];
+    __syncthreads();
+    return ex;
+}
+
+__global__ void __launch_bounds__(kConvThreads) convTileKernel(const uint64_t* keys, size_t n, unsigned bucket, int2* tiles)
+{
+    __shared__ size_t kept;
+    if (threadIdx.x == 0) { kept = keptKeys(keys, n); }
+    __syncthreads();
+    size_t base  = size_t(blockIdx.x) * kConvTile + size_t(threadIdx.x) * kConvItems;
+    LevelClamp v = clampIdentity();
+#pragma unroll
+    for (int q = 0; q < kConvItems; ++q)
+    {
+        v = clampThen(v, clampOf(keys, kept, bucket, base + q));
+    }
+    LevelClamp total;
+    blockScanClamp(v, &total);
+    if (threadIdx.x == 0) { tiles[blockIdx.x] = make_int2(total.e, total.c); }
+}
+
+//! tiles[t].x = D of the key before tile t
+__global__ void __launch_bounds__(kConvThreads) convScanKernel(int2* tiles, int numTiles)
+{
+    LevelClamp carry = clampIdentity();
+    for (int base = 0; base < numTiles; base += kConvThreads)
+    {
+        int t        = base + threadIdx.x;
+        LevelClamp v = t < numTiles ? LevelClamp{tiles[t].x, tiles[t].y} : clampIdentity();
+        LevelClamp total;
+        LevelClamp ex = clampThen(carry, blockScanClamp(v, &total));
+        if (t < numTiles) { tiles[t].x = max(ex.e, min(-1, ex.c)); }
+        carry = clampThen(carry, total);
+    }
+}
+
+//! sum of the octal digits from level lo to level hi of the key, or of 7 minus the digit
+__device__ __forceinline__ int digitSum(uint64_t key, int lo, int hi, bool complement)
+{
+    int sum = 0;
+    for (int l = lo; l <= hi; ++l)
+    {
+        sum += int(octalDigitAt(key, unsigned(l)));
+    }
+    return complement ? 7 * max(0, hi - lo + 1) - sum : sum;
+}
+
+/*! leaves that key p opens: its own, if p is the first key in it, and the empty ones before it; for p == n the empty
+ *  ones after the last key. dPrev = D_{p-1}, d = D_p. */
+__device__ __forceinline__ int opened(const uint64_t* __restrict__ keys, size_t n, size_t p, int dPrev, int d)
+{
+    if (n == 0) { return p == 0 ? 1 : 0; } // the root
+    if (p == n) { return digitSum(__ldg(keys + n - 1), 1, dPrev + 1, true); }
+    uint64_t k = __ldg(keys + p);
+    if (p == 0) { return digitSum(k, 1, d + 1, false) + 1; }
+    uint64_t o = __ldg(keys + p - 1);
+    int c      = commonLevel(o, k);
+    if (c > d) { return 0; }
+    return digitSum(o, c + 2, dPrev + 1, true) + int(octalDigitAt(k, unsigned(c + 1))) -
+           int(octalDigitAt(o, unsigned(c + 1))) + digitSum(k, c + 2, d + 1, false);
+}
+
+/*! kEmit false: sums[tile] = leaves opened by the tile's keys. kEmit true: the leaves, from the scanned sums, if all
+ *  numLeaves + 1 keys fit into capacity. */
+template<bool kEmit>
+__global__ void __launch_bounds__(kConvThreads) convLeavesKernel(const uint64_t* __restrict__ keys, size_t nAll,
+                                                                unsigned bucket, const int2* __restrict__ tiles,
+                                                                int* sums, uint64_t* leaves, size_t capacity,
+                                                                const int* numLeaves)
+{
+    __shared__ size_t kept;
+    __shared__ int warpSum[kConvThreads / 32];
+    if (threadIdx.x == 0) { kept = keptKeys(keys, nAll); }
+    __syncthreads();
+    const size_t n    = kept;
+    const size_t base = size_t(blockIdx.x) * kConvTile + size_t(threadIdx.x) * kConvItems;
+    LevelClamp f[kConvItems];
+    LevelClamp v = clampIdentity();
+#pragma unroll
+    for (int q = 0; q < kConvItems; ++q)
+    {
+        f[q] = clampOf(keys, n, bucket, base + q);
+        v    = clampThen(v, f[q]);
+    }
+    LevelClamp total;
+    LevelClamp ex = blockScanClamp(v, &total);
+    int d         = max(ex.e, min(tiles[blockIdx.x].x, ex.c));
+    int dPrev[kConvItems + 1];
+    int w[kConvItems];
+    int sum  = 0;
+    dPrev[0] = d;
+#pragma unroll
+    for (int q = 0; q < kConvItems; ++q)
+    {
+        d            = max(f[q].e, min(d, f[q].c));
+        dPrev[q + 1] = d;
+        w[q]         = base + q <= n ? opened(keys, n, base + q, dPrev[q], d) : 0;
+        sum += w[q];
+    }
+    int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int incl = sum;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1)
+    {
+        int t = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= off) { incl += t; }
+    }
+    if (lane == 31) { warpSum[warp] = incl; }
+    __syncthreads();
+    int before = 0, all = 0;
+    for (int q = 0; q < kConvThreads / 32; ++q)
+    {
+        before += q < warp ? warpSum[q] : 0;
+        all += warpSum[q];
+    }
+    if constexpr (!kEmit)
+    {
+        if (threadIdx.x == 0) { sums[blockIdx.x] = all; }
+        return;
+    }
+    const int num = *numLeaves;
+    if (num < 1 || size_t(num) + 1 > capacity) { return; }
+    auto put = [&](int pos, uint64_t key) {
+        if (pos >= 0 && pos < num) { leaves[pos] = key; } // (keys out of order place leaves anywhere)
+    };
+    int pos = sums[blockIdx.x] + before + incl - sum;
+    for (int q = 0; q < kConvItems; ++q)
+    {
+        size_t p = base + q;
+        if (p > n || w[q] == 0) { continue; }
+        int at = pos;
+        pos += w[q];
+        if (n == 0)
+        {
+            put(0, 0);
+            continue;
+        }
+        // children right of the previous key's path, from its leaf upwards
+        uint64_t o = p ? __ldg(keys + p - 1) : 0;
+        uint64_t k = p < n ? __ldg(keys + p) : 0;
+        int c      = p == 0 ? -1 : p == n ? -1 : commonLevel(o, k);
+        if (p > 0)
+        {
+            for (int l = dPrev[q] + 1; l >= c + 2 - (p == n ? 1 : 0); --l)
+            {
+                if (l < 1) { break; }
+                uint64_t range  = nodeRangeAt(unsigned(l));
+                uint64_t parent = o & ~(8 * range - 1);
+                for (unsigned dig = octalDigitAt(o, unsigned(l)) + 1; dig < 8; ++dig)
+                {
+                    put(at++, parent + dig * range);
+                }
+            }
+        }
+        if (p == n) { continue; }
+        // children left of this key's path, from the first level on which the paths differ downwards
+        for (int l = max(c + 1, 1); l <= dPrev[q + 1] + 1; ++l)
+        {
+            uint64_t range  = nodeRangeAt(unsigned(l));
+            uint64_t parent = k & ~(8 * range - 1);
+            unsigned first  = l == c + 1 && p > 0 ? octalDigitAt(o, unsigned(l)) + 1 : 0;
+            for (unsigned dig = first; dig < octalDigitAt(k, unsigned(l)); ++dig)
+            {
+                put(at++, parent + dig * range);
+            }
+        }
+        uint64_t leafRange = nodeRangeAt(unsigned(dPrev[q + 1] + 1));
+        put(at, k & ~(leafRange - 1));
+    }
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) { leaves[num] = kRootRange; }
+}
+
+} // namespace
+} // namespace sphb
+
 extern "C" int sphb_compute_octree(const uint64_t* sorted_keys, size_t n, unsigned bucket, uint64_t* leaves,
                                    uint32_t* counts, size_t capacity, size_t* num_leaves, void* stream)
 {
     using namespace sphb;
     if (!num_leaves || bucket == 0 || (n && !sorted_keys)) { return SPHB_ERR_ARG; }
+    if (n >= (size_t(1) << 30)) { return SPHB_ERR_ARG; }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    // computeOctree (csarray.hpp:432-440): start from the root with count n and step until no change
-    GlobalTree g;
-    TreeScratch s;
-    SPHB_TRY(initGlobalTree(g, bucket, st));
-    unsigned c = unsigned(n);
-    SPHB_CUDA_TRY(cudaMemcpyAsync(g.counts.data(), &c, sizeof(unsigned), cudaMemcpyHostToDevice, st));
-    unsigned maxCount = 1;
-    int guard         = 0;
-    while (maxCount != 0)
+    size_t numTiles = (n + 1 + kConvTile - 1) / kConvTile;
+    // per tile: the level clamp (two ints), the leaves opened, and the scan's scratch
+    DeviceBuffer<int> tmp;
+    SPHB_TRY(tmp.reserve(3 * numTiles + 2 + scanTempInts(numTiles) + 1));
+    int2* tiles  = reinterpret_cast<int2*>(tmp.data());
+    int* sums    = tmp.data() + 2 * numTiles;
+    int* scanTmp = sums + numTiles + 1;
+    size_t cap   = leaves && counts ? capacity : 0;
+    convTileKernel<<<unsigned(numTiles), kConvThreads, 0, st>>>(sorted_keys, n, bucket, tiles);
+    convScanKernel<<<1, kConvThreads, 0, st>>>(tiles, int(numTiles));
+    convLeavesKernel<false><<<unsigned(numTiles), kConvThreads, 0, st>>>(sorted_keys, n, bucket, tiles, sums, nullptr, 0,
+                                                                          nullptr);
+    countLaunch(3);
+    SPHB_CUDA_TRY(cudaGetLastError());
+    SPHB_TRY(exclusiveScan(sums, sums, numTiles, scanTmp, st));
+    convLeavesKernel<true><<<unsigned(numTiles), kConvThreads, 0, st>>>(sorted_keys, n, bucket, tiles, sums, leaves, cap,
+                                                                         sums + numTiles);
+    countLaunch();
+    SPHB_CUDA_TRY(cudaGetLastError());
+    int num = 0;
+    SPHB_TRY(readBack(st, {{&num, sums + numTiles, sizeof(int)}}));
+    if (num < 1) { return SPHB_ERR_ARG; } // keys out of order
+    *num_leaves = size_t(num);
+    if (size_t(num) + 1 <= cap)
     {
-        SPHB_TRY(globalTreeStep(g, sorted_keys, n, s, st, &maxCount));
-        if (++guard > 1000) { return SPHB_ERR_NOT_CONVERGED; }
-        if (maxCount == 0) { break; }
+        SPHB_TRY(computeLeafCounts(leaves, num, sorted_keys, n, counts, st));
+        SPHB_CUDA_TRY(cudaStreamSynchronize(st));
     }
-    *num_leaves = size_t(g.numLeaves);
-    if (size_t(g.numLeaves) + 1 <= capacity && leaves && counts)
-    {
-        SPHB_CUDA_TRY(cudaMemcpyAsync(leaves, g.leaves.data(), (g.numLeaves + 1) * sizeof(uint64_t),
-                                      cudaMemcpyDeviceToDevice, st));
-        SPHB_CUDA_TRY(cudaMemcpyAsync(counts, g.counts.data(), g.numLeaves * sizeof(unsigned),
-                                      cudaMemcpyDeviceToDevice, st));
-    }
-    SPHB_CUDA_TRY(cudaStreamSynchronize(st));
-    return size_t(g.numLeaves) + 1 <= capacity ? SPHB_OK : SPHB_ERR_CAPACITY;
+    return size_t(num) + 1 <= capacity ? SPHB_OK : SPHB_ERR_CAPACITY;
 }
 
 // ------------------------------------------------------------------------------------------------------------------
