@@ -103,7 +103,6 @@ struct sphb_ensemble
     DeviceBuffer<double> gamma, cv, dt, dtm1, ttot, cons;
     DeviceBuffer<unsigned long long> reduce;
     DeviceBuffer<unsigned> status; // [0] search overflow, [1] h flag, [2] sort look-back timeout
-    DeviceBuffer<uint32_t> sortFlags; // [0] pairs out of order before the tile repair, [1] after it
 
     // trees
     std::vector<std::unique_ptr<GlobalTree>> gtrees;
@@ -112,6 +111,9 @@ struct sphb_ensemble
     TreeScratch ts;
     DeviceBuffer<TreeView> views;
     DeviceBuffer<LeafDesc> leafDescs;
+    DeviceBuffer<LeafSet> leafSets; // the members' leaves as sort buckets
+    size_t numBuckets{0};
+    LeafSortScratch leafSort;
     int maxLeaves{0};
     DeviceBuffer<double> alphaBackup, hBackup;
     uint64_t launchesPerStep{0};
@@ -326,7 +328,6 @@ int allocate(sphb_ensemble& e)
     SPHB_TRY(e.cons.reserve(size_t(kNumCons) * m));
     SPHB_TRY(e.reduce.reserve(2 * size_t(m)));
     SPHB_TRY(e.status.reserve(4));
-    SPHB_TRY(e.sortFlags.reserve(2));
     SPHB_TRY(e.views.reserve(m));
     SPHB_TRY(e.leafDescs.reserve(m));
     for (auto& ev : e.ev)
@@ -425,21 +426,25 @@ void swapState(sphb_ensemble& e)
 }
 
 /*! keys, segmented sort, gather of 16 fields into the other buffer set, which then becomes the current one (a
- *  captured step records the buffers of its set; the two captured steps alternate). The sort is decided on the
- *  device, as the single simulation's nearly-sorted sort is on the host: the particles of the previous step are
- *  nearly in order within every instance, so the tiles holding out-of-order pairs are repaired in shared memory,
- *  and the full segmented radix sort (by key over all slots, then stably by instance) runs only if pairs remain out
- *  of order (every one of its kernels reads that count and returns at once when it is zero). The result is the same
- *  stable sort either way. */
+ *  captured step records the buffers of its set; the two captured steps alternate). The particles are sorted by the
+ *  leaves of their member's tree, as in a single simulation; the trees stay those of the last rebuild, so a leaf can
+ *  outgrow a warp: then the full segmented radix sort (by key over all slots, then stably by instance) takes its
+ *  place, decided on the device (every one of its kernels reads that flag and returns at once when it is zero). Before
+ *  the first trees the radix sort runs. The result is the same stable sort either way. */
 int syncBatched(sphb_ensemble& e, bool withLayout)
 {
     cudaStream_t st = e.stream;
     size_t n        = e.slots;
     SPHB_TRY(launchSfcKeys(e.f[0].data(), e.f[1].data(), e.f[2].data(), e.keys.data(), n, e.box, st));
     SPHB_CUDA_TRY(cudaMemcpyAsync(e.keysTmp.data(), e.keys.data(), n * sizeof(uint64_t), cudaMemcpyDeviceToDevice, st));
-    SPHB_TRY(repairSegmentedAsync(e.keysTmp.data(), e.order.data(), e.segOfSlot.data(), n, e.sortFlags.data(), st));
-    const uint32_t* remaining = e.sortFlags.data() + 1;
-    SPHB_TRY(sortByKeyAsync(e.keysTmp.data(), e.order.data(), n, false, e.sortScratch.data(),
+    const uint32_t* remaining = nullptr;
+    if (withLayout)
+    {
+        SPHB_TRY(sortSegmentsByLeavesAsync(e.keys.data(), e.keysTmp.data(), e.order.data(), n, e.segOfSlot.data(),
+                                           e.leafSets.data(), e.numBuckets, e.leafSort, e.sortScratch.data(),
+                                           e.sortScratch.capacity(), &remaining, st));
+    }
+    SPHB_TRY(sortByKeyAsync(e.keysTmp.data(), e.order.data(), n, !withLayout, e.sortScratch.data(),
                             e.sortScratch.capacity(), 0xffu, e.status.data() + 2, st, remaining));
     const void* segSrc[1] = {e.segOfSlot.data()};
     void* segDst[1]       = {e.segKey.data()};
@@ -485,6 +490,8 @@ int rebuildTrees(sphb_ensemble& e)
     cudaStream_t st = e.stream;
     std::vector<TreeView> views(e.num);
     std::vector<LeafDesc> descs(e.num);
+    std::vector<LeafSet> sets(e.num);
+    e.numBuckets = 0;
     e.maxLeaves = 0;
     for (int k = 0; k < e.num; ++k)
     {
@@ -519,6 +526,8 @@ int rebuildTrees(sphb_ensemble& e)
         tv.blockHi      = e.blockHi.data();
         tv.numNodes     = f.tree.numNodes;
         views[k]        = tv;
+        sets[k] = LeafSet{f.leaves.data(), f.numLeaves, uint32_t(e.numBuckets)};
+        e.numBuckets += size_t(f.numLeaves) + 1;
         descs[k]        = LeafDesc{f.leaves.data(), e.layouts[k]->data(), f.numLeaves, uint32_t(e.off[k]),
                             uint32_t(e.n[k])};
         e.maxLeaves     = std::max(e.maxLeaves, f.numLeaves);
@@ -526,6 +535,11 @@ int rebuildTrees(sphb_ensemble& e)
     SPHB_CUDA_TRY(cudaMemcpyAsync(e.views.data(), views.data(), e.num * sizeof(TreeView), cudaMemcpyHostToDevice, st));
     SPHB_CUDA_TRY(
         cudaMemcpyAsync(e.leafDescs.data(), descs.data(), e.num * sizeof(LeafDesc), cudaMemcpyHostToDevice, st));
+    SPHB_TRY(e.leafSets.reserve(e.num));
+    SPHB_CUDA_TRY(cudaMemcpyAsync(e.leafSets.data(), sets.data(), e.num * sizeof(LeafSet), cudaMemcpyHostToDevice, st));
+    SPHB_TRY(e.leafSort.slot.reserve(e.slots));
+    SPHB_TRY(e.leafSort.first.reserve(e.numBuckets + 3));
+    SPHB_TRY(e.leafSort.scanTmp.reserve(scanTempInts(e.numBuckets) + 1));
     dim3 grid(unsigned(ceilDiv(size_t(e.maxLeaves) + 1, 256)), unsigned(e.num));
     forestLayoutKernel<<<grid, 256, 0, st>>>(e.leafDescs.data(), e.keys.data());
     countLaunch();

@@ -205,99 +205,6 @@ __global__ void __launch_bounds__(kRepairThreads) repairTilesKernel(uint64_t* ke
     }
 }
 
-//! *count += adjacent pairs of one segment out of key order: seg[i] == seg[i + 1] and keys[i] > keys[i + 1]
-__global__ void __launch_bounds__(256) inversionsSegKernel(const uint64_t* __restrict__ keys,
-                                                           const uint64_t* __restrict__ seg, size_t n,
-                                                           uint32_t* count)
-{
-    uint32_t c = 0;
-    for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i + 1 < n; i += size_t(gridDim.x) * blockDim.x)
-    {
-        c += (keys[i] > keys[i + 1] && seg[i] == seg[i + 1]) ? 1u : 0u;
-    }
-    c = __reduce_add_sync(0xffffffffu, c);
-    __shared__ uint32_t warpSum[8];
-    if ((threadIdx.x & 31) == 0) { warpSum[threadIdx.x >> 5] = c; }
-    __syncthreads();
-    if (threadIdx.x == 0)
-    {
-        uint32_t s = 0;
-        for (int w = 0; w < 8; ++w)
-        {
-            s += warpSum[w];
-        }
-        if (s) { atomicAdd(count, s); }
-    }
-}
-
-/*! repairTilesKernel for an array of contiguous segments (slot ranges that keep their segment): the tile is sorted
- *  stably by (segment, key), so a tile that straddles two segments keeps each segment's slots within it. */
-__global__ void __launch_bounds__(kRepairThreads) repairTilesSegKernel(uint64_t* keys, uint32_t* vals,
-                                                                      const uint64_t* seg, size_t n, size_t offset)
-{
-    __shared__ uint64_t sk[kRepairTile];
-    __shared__ uint32_t sv[kRepairTile];
-    __shared__ uint16_t sp[kRepairTile];
-    __shared__ uint8_t sg[kRepairTile];
-    size_t t0 = offset + size_t(blockIdx.x) * kRepairTile;
-    if (t0 >= n) { return; }
-    size_t len = min(size_t(kRepairTile), n - t0);
-    bool d     = false;
-    for (size_t q = threadIdx.x; q + 1 < len; q += kRepairThreads)
-    {
-        d = d || (keys[t0 + q] > keys[t0 + q + 1] && seg[t0 + q] == seg[t0 + q + 1]);
-    }
-    if (__syncthreads_or(d) == 0) { return; }
-    // segments are ranked by their order within the tile (they are contiguous and ascending)
-    uint64_t seg0 = seg[t0];
-    for (int q = threadIdx.x; q < kRepairTile; q += kRepairThreads)
-    {
-        bool in = size_t(q) < len;
-        sk[q]   = in ? keys[t0 + q] : ~uint64_t(0);
-        sv[q]   = in ? vals[t0 + q] : 0u;
-        sp[q]   = uint16_t(q);
-        sg[q]   = in ? uint8_t(min(seg[t0 + q] - seg0, uint64_t(254))) : uint8_t(255);
-    }
-    __syncthreads();
-    for (int size = 2; size <= kRepairTile; size <<= 1)
-    {
-        for (int stride = size >> 1; stride > 0; stride >>= 1)
-        {
-            for (int q = threadIdx.x; q < kRepairTile; q += kRepairThreads)
-            {
-                int p = q ^ stride;
-                if (p > q)
-                {
-                    bool up      = (q & size) == 0;
-                    bool greater = sg[q] > sg[p] ||
-                                   (sg[q] == sg[p] && (sk[q] > sk[p] || (sk[q] == sk[p] && sp[q] > sp[p])));
-                    if (greater == up)
-                    {
-                        uint64_t k = sk[q];
-                        sk[q]      = sk[p];
-                        sk[p]      = k;
-                        uint32_t v = sv[q];
-                        sv[q]      = sv[p];
-                        sv[p]      = v;
-                        uint16_t o = sp[q];
-                        sp[q]      = sp[p];
-                        sp[p]      = o;
-                        uint8_t g  = sg[q];
-                        sg[q]      = sg[p];
-                        sg[p]      = g;
-                    }
-                }
-            }
-            __syncthreads();
-        }
-    }
-    for (size_t q = threadIdx.x; q < len; q += kRepairThreads)
-    {
-        keys[t0 + q] = sk[q];
-        vals[t0 + q] = sv[q];
-    }
-}
-
 /*! One onesweep pass over bits [shift, shift+8).
  *
  * Shared memory: per-warp digit counters (8 x 256), the tile's exclusive digit prefix (256) and the tile index.
@@ -618,23 +525,6 @@ int runPasses(uint64_t* keys, uint32_t* values, size_t n, const SortScratch& s, 
 
 } // namespace
 
-int repairSegmentedAsync(uint64_t* keys, uint32_t* values, const uint64_t* seg, size_t n, uint32_t* flags,
-                         cudaStream_t stream)
-{
-    SPHB_CUDA_TRY(cudaMemsetAsync(flags, 0, 2 * sizeof(uint32_t), stream));
-    if (n == 0) { return kOk; }
-    unsigned blocks = unsigned(std::min<size_t>(ceilDiv(n, 256 * 8), size_t(smCount()) * 8));
-    iotaKernel<<<ceilDiv(n, 256), 256, 0, stream>>>(values, n);
-    inversionsSegKernel<<<blocks, 256, 0, stream>>>(keys, seg, n, flags);
-    repairTilesSegKernel<<<unsigned(ceilDiv(n, size_t(kRepairTile))), kRepairThreads, 0, stream>>>(keys, values, seg,
-                                                                                                   n, 0);
-    repairTilesSegKernel<<<unsigned(ceilDiv(n, size_t(kRepairTile))), kRepairThreads, 0, stream>>>(
-        keys, values, seg, n, kRepairTile / 2);
-    inversionsSegKernel<<<blocks, 256, 0, stream>>>(keys, seg, n, flags + 1);
-    SPHB_CUDA_TRY(cudaGetLastError());
-    return kOk;
-}
-
 // ---------------------------------------------------------------------------------------------------------------
 // Sort of a step's particles by the leaves of the previous step's tree
 //
@@ -642,8 +532,9 @@ int repairSegmentedAsync(uint64_t* keys, uint32_t* values, const uint64_t* seg, 
 // keys pays only while particles stay within a tile of 2,048; one that crosses an octant boundary of the curve far up
 // moves by up to n, and then both repair passes (45 us each at 4,096 particles, 91 us at 128^3) were followed by the
 // radix sort (eight passes of 18 to 38 us and an 8 KB host read). Sync of a step with such a motion: 16^3 235 -> 154 us,
-// 30^3 510 -> 168 us, 81^3 (Noh) 663 -> 263 us, 128^3 0.95 -> 0.43 ms. A warp sorts a leaf in registers; 128 keys
-// (four per lane) is where its bitonic network still fits 32 registers.
+// 30^3 510 -> 168 us, 81^3 (Noh) 663 -> 263 us, 128^3 0.95 -> 0.43 ms. A warp sorts a leaf in registers, at most
+// 128 keys (four per lane): the tree splits leaves of more than 64, so only a sudden compression exceeds it. An ensemble
+// of 663,000 particles in 16 members (its trees stay those of the last rebuild) 0.69 -> 0.21 ms.
 // ---------------------------------------------------------------------------------------------------------------
 
 namespace
@@ -665,53 +556,69 @@ __device__ __forceinline__ int leafOf(const uint64_t* __restrict__ leaves, int n
     return lo;
 }
 
-/*! values = 0..n-1; slot[i] = {leaf of key i, its place among the leaf's keys in arrival order}, counts[l] = keys per
- *  leaf (zero on entry); flags[0] = 1 if any adjacent pair is out of order, flags[1] = 1 if a leaf exceeds
- *  kLeafSortCap. The lanes of a leaf (most of a warp: the keys are nearly in order) share one atomic. */
-__global__ void __launch_bounds__(256) leafSlotKernel(const uint64_t* __restrict__ keys, size_t n,
-                                                      const uint64_t* __restrict__ leaves, int numLeaves,
-                                                      uint32_t* __restrict__ values, uint2* __restrict__ slot,
-                                                      int* counts, unsigned* flags)
+//! the leaves that hold key i: one tree, or the tree of the key's segment
+template<bool kSeg>
+__device__ __forceinline__ LeafSet leafSetOf(const LeafSet& one, const LeafSet* __restrict__ many,
+                                             const uint64_t* __restrict__ seg, size_t i)
+{
+    if constexpr (kSeg) { return many[seg[i]]; }
+    else { return one; }
+}
+
+/*! values = 0..n-1; slot[i] = {bucket (leaf) of key i, its place among the bucket's keys in arrival order}, counts[l] =
+ *  keys per bucket (zero on entry); flags[0] = 1 if any adjacent pair is out of order (one tree only), flags[1] = 1 if
+ *  a bucket exceeds kLeafSortCap. The lanes of a bucket (most of a warp: the keys are nearly in order) share one
+ *  atomic. */
+template<bool kSeg>
+__global__ void __launch_bounds__(256) leafSlotKernel(const uint64_t* __restrict__ keys, size_t n, LeafSet one,
+                                                      const LeafSet* __restrict__ many,
+                                                      const uint64_t* __restrict__ seg, uint32_t* __restrict__ values,
+                                                      uint2* __restrict__ slot, int* counts, unsigned* flags)
 {
     size_t i   = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
     bool valid = i < n;
-    int leaf   = -1;
+    int bucket = -1;
     bool inv   = false;
     if (valid)
     {
         uint64_t k = keys[i];
-        inv        = i + 1 < n && k > keys[i + 1];
-        leaf       = leafOf(leaves, numLeaves, k);
-        values[i]  = uint32_t(i);
+        if constexpr (!kSeg) { inv = i + 1 < n && k > keys[i + 1]; }
+        LeafSet t = leafSetOf<kSeg>(one, many, seg, i);
+        bucket    = int(t.bucket0) + leafOf(t.leaves, t.numLeaves, k);
+        values[i] = uint32_t(i);
     }
     unsigned lane  = threadIdx.x & (kWarp - 1);
-    unsigned peers = __match_any_sync(0xffffffffu, leaf);
+    unsigned peers = __match_any_sync(0xffffffffu, bucket);
     int leader     = __ffs(peers) - 1;
     int base       = 0;
-    if (int(lane) == leader && valid) { base = atomicAdd(counts + leaf, __popc(peers)); }
+    if (int(lane) == leader && valid) { base = atomicAdd(counts + bucket, __popc(peers)); }
     base      = __shfl_sync(0xffffffffu, base, leader);
     int place = base + __popc(peers & ((1u << lane) - 1u));
-    if (valid) { slot[i] = make_uint2(unsigned(leaf), unsigned(place)); }
+    if (valid) { slot[i] = make_uint2(unsigned(bucket), unsigned(place)); }
     unsigned anyInv  = __ballot_sync(0xffffffffu, inv);
     unsigned anyFull = __ballot_sync(0xffffffffu, valid && place >= kLeafSortCap);
     if (lane == 0 && anyInv) { flags[0] = 1u; }
     if (lane == 0 && anyFull) { flags[1] = 1u; }
 }
 
-/*! composite[first[leaf] + place] = (the upper 32 bits of the key within its leaf, index): what a warp sorts. A leaf
+/*! composite[first[bucket] + place] = (the upper 32 bits of the key within its leaf, index): what a warp sorts. A leaf
  *  of level L leaves 63 - 3 L bits of the key open. */
-__global__ void __launch_bounds__(256) leafScatterKernel(const uint64_t* __restrict__ keys, size_t n,
-                                                         const uint64_t* __restrict__ leaves, int numLeaves,
+template<bool kSeg>
+__global__ void __launch_bounds__(256) leafScatterKernel(const uint64_t* __restrict__ keys, size_t n, LeafSet one,
+                                                         const LeafSet* __restrict__ many,
+                                                         const uint64_t* __restrict__ seg,
                                                          const uint2* __restrict__ slot, const int* __restrict__ first,
-                                                         uint64_t* __restrict__ composite)
+                                                         uint64_t* __restrict__ composite, const unsigned* flags)
 {
     size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
-    if (i >= n) { return; }
+    if (i >= n || (kSeg && flags[1] != 0)) { return; }
     uint2 s        = slot[i];
-    uint64_t start = __ldg(leaves + s.x);
+    LeafSet t      = leafSetOf<kSeg>(one, many, seg, i);
+    int leaf       = int(s.x - t.bucket0);
+    uint64_t start = __ldg(t.leaves + leaf);
     int shift      = 0;
-    if (int(s.x) < numLeaves) { shift = max(0, 31 - int(__clzll(__ldg(leaves + s.x + 1) - start))); }
-    size_t dst     = size_t(__ldg(first + s.x)) + s.y;
+    if (leaf < t.numLeaves) { shift = max(0, 31 - int(__clzll(__ldg(t.leaves + leaf + 1) - start))); }
+    size_t dst = size_t(__ldg(first + s.x)) + s.y;
     if (dst < n) { composite[dst] = (((keys[i] - start) >> shift) << 32) | uint64_t(i); }
 }
 
@@ -827,16 +734,16 @@ __device__ __forceinline__ void sortLeaf(const uint64_t* composite, const uint64
     }
 }
 
-//! one warp per leaf (and one for the keys past the last leaf)
+//! one warp per bucket; with gate set, nothing runs if *gate is not 0
 __global__ void __launch_bounds__(256) leafSortKernel(const uint64_t* __restrict__ composite,
-                                                      const uint64_t* __restrict__ keysIn, int numLeaves,
+                                                      const uint64_t* __restrict__ keysIn, int numBuckets,
                                                       const int* __restrict__ first, uint64_t* __restrict__ keysOut,
-                                                      uint32_t* __restrict__ values)
+                                                      uint32_t* __restrict__ values, const unsigned* gate)
 {
-    int leaf = int((blockIdx.x * size_t(blockDim.x) + threadIdx.x) / kWarp);
-    int lane = threadIdx.x & (kWarp - 1);
-    if (leaf > numLeaves) { return; }
-    int b = first[leaf], m = first[leaf + 1] - b;
+    int bucket = int((blockIdx.x * size_t(blockDim.x) + threadIdx.x) / kWarp);
+    int lane   = threadIdx.x & (kWarp - 1);
+    if (bucket >= numBuckets || (gate && *gate != 0)) { return; }
+    int b = first[bucket], m = first[bucket + 1] - b;
     if (m <= 0) { return; }
     if (m <= 32) { sortLeaf<1>(composite, keysIn, b, m, lane, keysOut, values); }
     else if (m <= 64) { sortLeaf<2>(composite, keysIn, b, m, lane, keysOut, values); }
@@ -863,8 +770,9 @@ int sortByLeaves(uint64_t* keys, uint64_t* keysOut, uint32_t* values, size_t n, 
     int* counts     = ls.first.data() + 2;
     unsigned* flags = reinterpret_cast<unsigned*>(ls.first.data());
     SPHB_CUDA_TRY(cudaMemsetAsync(ls.first.data(), 0, (buckets + 2) * sizeof(int), stream));
-    leafSlotKernel<<<ceilDiv(n, 256), 256, 0, stream>>>(keys, n, leaves, numLeaves, values, ls.slot.data(), counts,
-                                                        flags);
+    LeafSet one{leaves, numLeaves, 0};
+    leafSlotKernel<false><<<ceilDiv(n, 256), 256, 0, stream>>>(keys, n, one, nullptr, nullptr, values, ls.slot.data(),
+                                                               counts, flags);
     countLaunch();
     SPHB_CUDA_TRY(cudaGetLastError());
     unsigned msg[2];
@@ -877,13 +785,42 @@ int sortByLeaves(uint64_t* keys, uint64_t* keysOut, uint32_t* values, size_t n, 
     if (msg[1]) { return sortByKey(keys, values, n, false, scratch, scratchBytes, stream); }
     uint64_t* composite = carve(scratch, n).keysAlt;
     SPHB_TRY(exclusiveScan(counts, counts, buckets, ls.scanTmp.data(), stream));
-    leafScatterKernel<<<ceilDiv(n, 256), 256, 0, stream>>>(keys, n, leaves, numLeaves, ls.slot.data(), counts,
-                                                           composite);
-    leafSortKernel<<<ceilDiv(buckets * kWarp, 256), 256, 0, stream>>>(composite, keys, numLeaves, counts, keysOut,
-                                                                      values);
+    leafScatterKernel<false><<<ceilDiv(n, 256), 256, 0, stream>>>(keys, n, one, nullptr, nullptr, ls.slot.data(), counts,
+                                                                  composite, nullptr);
+    leafSortKernel<<<ceilDiv(buckets * kWarp, 256), 256, 0, stream>>>(composite, keys, int(buckets), counts, keysOut,
+                                                                      values, nullptr);
     countLaunch(2);
     SPHB_CUDA_TRY(cudaGetLastError());
     *result = LeafSort::keysOut;
+    return kOk;
+}
+
+int sortSegmentsByLeavesAsync(const uint64_t* keys, uint64_t* keysOut, uint32_t* values, size_t n, const uint64_t* seg,
+                              const LeafSet* sets, size_t numBuckets, LeafSortScratch& ls, void* scratch,
+                              size_t scratchBytes, const unsigned** overflow, cudaStream_t stream)
+{
+    if (!scratch || scratchBytes < sortScratchBytes(n) || ls.slot.capacity() < n ||
+        ls.first.capacity() < numBuckets + 3 || ls.scanTmp.capacity() < scanTempInts(numBuckets) + 1)
+    {
+        return kErrCapacity;
+    }
+    int* counts     = ls.first.data() + 2;
+    unsigned* flags = reinterpret_cast<unsigned*>(ls.first.data());
+    *overflow       = flags + 1;
+    SPHB_CUDA_TRY(cudaMemsetAsync(ls.first.data(), 0, (numBuckets + 2) * sizeof(int), stream));
+    if (n == 0) { return kOk; }
+    uint64_t* composite = carve(scratch, n).keysAlt;
+    LeafSet none{nullptr, 0, 0};
+    leafSlotKernel<true><<<ceilDiv(n, 256), 256, 0, stream>>>(keys, n, none, sets, seg, values, ls.slot.data(), counts,
+                                                              flags);
+    countLaunch();
+    SPHB_TRY(exclusiveScan(counts, counts, numBuckets, ls.scanTmp.data(), stream));
+    leafScatterKernel<true><<<ceilDiv(n, 256), 256, 0, stream>>>(keys, n, none, sets, seg, ls.slot.data(), counts,
+                                                                 composite, flags);
+    leafSortKernel<<<ceilDiv(numBuckets * kWarp, 256), 256, 0, stream>>>(composite, keys, int(numBuckets), counts,
+                                                                         keysOut, values, flags + 1);
+    countLaunch(2);
+    SPHB_CUDA_TRY(cudaGetLastError());
     return kOk;
 }
 

@@ -48,12 +48,22 @@ int sortByLeaves(uint64_t* keys, uint64_t* keysOut, uint32_t* values, size_t n, 
 int sortByKeyAsync(uint64_t* keys, uint32_t* values, size_t n, bool initValues, void* scratch, size_t scratchBytes,
                    unsigned passMask, uint32_t* errorOut, cudaStream_t stream, const uint32_t* gate = nullptr);
 
-/*! The local repair of sortNearlySorted for an array of contiguous segments (seg[i] ascending; a slot never leaves
- *  its segment), without any host synchronisation: values = 0..n-1, flags[0] = number of adjacent pairs of one
- *  segment out of key order, then the tiles holding such pairs are sorted stably by (segment, key) in shared memory
- *  (two overlapping tilings), flags[1] = pairs still out of order. If flags[1] is 0, keys/values are the stable
- *  sort by (segment, key); otherwise a full sort of the repaired sequence (gated on flags + 1) completes it. */
-int repairSegmentedAsync(uint64_t* keys, uint32_t* values, const uint64_t* seg, size_t n, uint32_t* flags,
-                         cudaStream_t stream);
+//! one cornerstone leaf array among several: its leaves are the buckets bucket0 .. bucket0 + numLeaves - 1, and the
+//! bucket after them takes the keys past the last leaf
+struct LeafSet
+{
+    const uint64_t* leaves;
+    int numLeaves;
+    uint32_t bucket0;
+};
+
+/*! sortByLeaves for an array of contiguous segments (seg[i] ascending; sets[k] the leaves of segment k, numBuckets
+ *  buckets over all segments), without any host synchronisation. values = 0..n-1, then the stable order by (segment,
+ *  key) and the keys in it in keysOut; if a bucket grew past 128 keys, **overflow (device) is not 0 and only values =
+ *  0..n-1 was written. The buffers of ls must be large enough beforehand (slot n, first numBuckets + 3, scanTmp
+ *  scanTempInts(numBuckets) + 1). */
+int sortSegmentsByLeavesAsync(const uint64_t* keys, uint64_t* keysOut, uint32_t* values, size_t n, const uint64_t* seg,
+                              const LeafSet* sets, size_t numBuckets, LeafSortScratch& ls, void* scratch,
+                              size_t scratchBytes, const unsigned** overflow, cudaStream_t stream);
 
 } // namespace sphb
