@@ -378,6 +378,17 @@ extern "C" int sphb_sim_load_fields(sphb_sim* s, const sphb_field* fields, int n
     return simimpl::finishLoad(*s);
 }
 
+namespace sphb
+{
+namespace simimpl
+{
+int convertArray(const void* src, int srcType, void* dst, int dstType, size_t n, cudaStream_t stream)
+{
+    return convert(src, srcType, dst, dstType, n, stream);
+}
+} // namespace simimpl
+} // namespace sphb
+
 extern "C" int sphb_sim_store_fields(sphb_sim* s, const sphb_field* fields, int num_fields, int on_device)
 {
     if (s) { SPHB_TRY(simimpl::waitLateFields(*s, true)); }

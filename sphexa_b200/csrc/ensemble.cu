@@ -1195,17 +1195,21 @@ extern "C" int sphb_ensemble_get_field(sphb_ensemble* e, int k, const char* name
     if (!fieldPtr(e, name, &ptr, &kind)) { return SPHB_ERR_ARG; }
     size_t nk   = e->n[k];
     size_t elem = kind == 0 || kind == 3 ? 8 : kind == 2 ? 4 : e->elemBytes();
-    std::vector<char> host(nk * elem);
     const char* src = static_cast<const char*>(ptr) + e->off[k] * elem;
+    if (elem == 8)
+    {
+        // doubles, and the bits of keys and ids, as they are
+        SPHB_CUDA_TRY(cudaMemcpyAsync(out, src, nk * elem, cudaMemcpyDeviceToHost, e->stream));
+        SPHB_CUDA_TRY(cudaStreamSynchronize(e->stream));
+        return SPHB_OK;
+    }
+    std::vector<char> host(nk * elem);
     SPHB_CUDA_TRY(cudaMemcpyAsync(host.data(), src, nk * elem, cudaMemcpyDeviceToHost, e->stream));
     SPHB_CUDA_TRY(cudaStreamSynchronize(e->stream));
     for (size_t i = 0; i < nk; ++i)
     {
-        double v;
-        if (kind == 0 || kind == 3 || (kind == 1 && elem == 8)) { std::memcpy(&v, host.data() + 8 * i, 8); }
-        else if (kind == 1) { v = double(reinterpret_cast<const float*>(host.data())[i]); }
-        else { v = double(reinterpret_cast<const uint32_t*>(host.data())[i]); }
-        out[i] = v;
+        out[i] = kind == 1 ? double(reinterpret_cast<const float*>(host.data())[i])
+                           : double(reinterpret_cast<const uint32_t*>(host.data())[i]);
     }
     return SPHB_OK;
 }

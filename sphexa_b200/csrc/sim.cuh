@@ -218,6 +218,8 @@ namespace simimpl
 int runStage(sphb_sim& s, int stage);
 //! device pointer and element kind (0 double, 1 J-loop type, 2 uint32, 3 uint64) of a field by reference name
 bool findField(sphb_sim& s, const char* name, void** ptr, int* kind);
+//! dst[i] = src[i] converted between element types (SPHB_F32 ...) on the device; SPHB_U64 only to itself
+int convertArray(const void* src, int srcType, void* dst, int dstType, size_t n, cudaStream_t stream);
 //! the ideal-gas heat capacity of the simulation's parameters
 double cv(const sphb_sim& s);
 //! after the conserved fields and ids were written: reset the step state as sphb_sim_upload does
