@@ -50,7 +50,7 @@ __global__ void eosRefreshKernel(ChainArrays<T> a, HydroConsts<T> k)
     a.c[i]      = T(c);
     T vx = T(a.vx[i]), vy = T(a.vy[i]), vz = T(a.vz[i]);
     a.hrec[i] = HydroRec<T>{vx, vy, vz, T(1) / hi, xmassi, xmassi / kxi, T(c), T(prho)};
-    if (a.avrec) { a.avrec[i] = AVRec<T>{vx, vy, vz, T(c), xmassi / kxi, a.divv[i], T(0), T(0)}; }
+    if (a.avrec) { a.avrec[i] = AVRec<T>{xmassi / kxi, a.divv[i]}; }
 }
 
 // One warp per group, one lane per particle: a thread per group walked its particles alone, 32 dependent loads of

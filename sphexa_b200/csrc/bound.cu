@@ -266,7 +266,7 @@ template<class T>
 __global__ void packRecordsKernel(size_t n, const double* h, const double* vx, const double* vy, const double* vz,
                                   const double* alpha, const T* xm, const T* kx, const T* c, const T* prho,
                                   const T* c11, const T* c12, const T* c13, const T* c22, const T* c23, const T* c33,
-                                  const T* divv, HydroRec<T>* hrec, GradRec<T>* grec, AVRec<T>* avrec)
+                                  const T* divv, HydroRec<T>* hrec, GradRec<T>* grec, AVFullRec<T>* avfull)
 {
     size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
     if (i >= n) { return; }
@@ -274,27 +274,28 @@ __global__ void packRecordsKernel(size_t n, const double* h, const double* vx, c
     HydroRec<T> hr  = {T(vx[i]), T(vy[i]), T(vz[i]), T(1) / hi, xm[i], xm[i] / kx[i], c[i], prho[i]};
     hrec[i]         = hr;
     if (grec) { grec[i] = GradRec<T>{c11[i], c12[i], c13[i], c22[i], c23[i], c33[i], divv[i], T(alpha[i])}; }
-    if (avrec) { avrec[i] = AVRec<T>{hr.vx, hr.vy, hr.vz, hr.c, hr.vol, divv[i], T(0), T(0)}; }
+    if (avfull) { avfull[i] = AVFullRec<T>{hr.vx, hr.vy, hr.vz, hr.c, hr.vol, divv[i], T(0), T(0)}; }
 }
 
 template<class T>
-int packRecordsT(sphb_sim& s, bool withGrad)
+int packRecordsT(sphb_sim& s, bool withGrad, bool withAv)
 {
+    if (withAv) { SPHB_TRY(s.avfull.reserve(s.n * sizeof(AVFullRec<T>))); }
     auto* hrec  = reinterpret_cast<HydroRec<T>*>(s.hrec.data());
     auto* grec  = withGrad ? reinterpret_cast<GradRec<T>*>(s.grec.data()) : nullptr;
-    auto* avrec = withGrad ? reinterpret_cast<AVRec<T>*>(s.avrec.data()) : nullptr;
+    auto* avfull = withAv ? reinterpret_cast<AVFullRec<T>*>(s.avfull.data()) : nullptr;
     packRecordsKernel<T><<<ceilDiv(s.n, 256), 256, 0, s.stream>>>(
         s.n, s.f[fH].data(), s.f[fVx].data(), s.f[fVy].data(), s.f[fVz].data(), s.f[fAlpha].data(), s.dptr<T>(dXm),
         s.dptr<T>(dKx), s.dptr<T>(dC), s.dptr<T>(dPrho), s.dptr<T>(dC11), s.dptr<T>(dC12), s.dptr<T>(dC13),
-        s.dptr<T>(dC22), s.dptr<T>(dC23), s.dptr<T>(dC33), s.dptr<T>(dDivv), hrec, grec, avrec);
+        s.dptr<T>(dC22), s.dptr<T>(dC23), s.dptr<T>(dC33), s.dptr<T>(dDivv), hrec, grec, avfull);
     countLaunch();
     SPHB_CUDA_TRY(cudaGetLastError());
     return kOk;
 }
 
-int packRecords(sphb_sim& s, bool withGrad)
+int packRecords(sphb_sim& s, bool withGrad, bool withAv = false)
 {
-    return s.mixed ? packRecordsT<float>(s, withGrad) : packRecordsT<double>(s, withGrad);
+    return s.mixed ? packRecordsT<float>(s, withGrad, withAv) : packRecordsT<double>(s, withGrad, withAv);
 }
 
 // ------------------------------------------------------------------------------------------------------------------
@@ -701,9 +702,12 @@ extern "C" int sphb_dataset_av_switches(sphb_sim* s, size_t first, size_t last, 
     if (!(min_dt > 0.0)) { return SPHB_ERR_ARG; }
     SPHB_TRY(importBound(*s, {"vx", "vy", "vz", "xm", "kx", "c", "prho", "c11", "c12", "c13", "c22", "c23", "c33",
                               "divv", "alpha"}));
-    SPHB_TRY(packRecords(*s, true));
-    s->minDt = min_dt;
-    SPHB_TRY(simimpl::runStage(*s, sAV));
+    SPHB_TRY(packRecords(*s, true, true));
+    s->minDt         = min_dt;
+    s->avFromDataset = true;
+    int rc           = simimpl::runStage(*s, sAV);
+    s->avFromDataset = false;
+    SPHB_TRY(rc);
     SPHB_TRY(exportBound(*s, "alpha"));
     SPHB_CUDA_TRY(cudaStreamSynchronize(s->stream));
     return SPHB_OK;

@@ -17,6 +17,7 @@ constexpr int kModeTape    = 1;
 constexpr int kModeBatch   = 2;
 constexpr int kModeAvClean = 4;
 constexpr int kModeList    = 8; // block time steps: only the groups of a device-side list
+constexpr int kModeFullAv  = 16; // AV switches on AVFullRec records
 
 /*! Neighbour-sum accumulator. Terms are summed plainly within one list chunk of 8 neighbours, in list order, and the
  *  chunk sums are added in chunk order: FP64 plainly, FP32 with Kahan compensation (explicit round-to-nearest
@@ -428,9 +429,9 @@ template<int kSplit, bool kRolled, class F>
 __device__ __forceinline__ void overChunk(const uint32_t* nidx, const Target& t, unsigned round, F&& term);
 
 template<class T>
-__device__ __forceinline__ AVRec<T> loadAV(const AVRec<T>* p)
+__device__ __forceinline__ AVFullRec<T> loadAV(const AVFullRec<T>* p)
 {
-    AVRec<T> r;
+    AVFullRec<T> r;
     if constexpr (sizeof(T) == 8)
     {
         const double4* q = reinterpret_cast<const double4*>(p);
@@ -444,6 +445,18 @@ __device__ __forceinline__ AVRec<T> loadAV(const AVRec<T>* p)
         r = {v[0], v[1], v[2], v[3], v[4], v[5], 0.f, 0.f};
     }
     return r;
+}
+
+__device__ __forceinline__ AVRec<float> loadAV(const AVRec<float>* p)
+{
+    float2 v = __ldg(reinterpret_cast<const float2*>(p));
+    return {v.x, v.y};
+}
+
+__device__ __forceinline__ AVRec<double> loadAV(const AVRec<double>* p)
+{
+    double2 v = __ldg(reinterpret_cast<const double2*>(p));
+    return {v.x, v.y};
 }
 
 template<class T>

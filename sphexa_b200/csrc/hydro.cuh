@@ -51,10 +51,18 @@ struct alignas(8 * sizeof(T)) GradRec
     T c11, c12, c13, c22, c23, c33, divv, alpha;
 };
 
-/*! Neighbour-side record of the AV switches, written by IAD: velocity, sound speed, xm/kx and divv (one 32-byte
- *  gather per neighbour instead of three records). */
+/*! Neighbour-side record of the AV switches, written by IAD: xm/kx and divv. The signal velocity, which also needs the
+ *  neighbours' velocities and sound speeds, is found by IAD's loop, which gathers them anyway. */
 template<class T>
-struct alignas(8 * sizeof(T)) AVRec
+struct alignas(2 * sizeof(T)) AVRec
+{
+    T vol, divv;
+};
+
+/*! The same with velocity and sound speed, for AV switches that find the signal velocity themselves (the stages on a
+ *  caller's dataset, whose v and c are the caller's at the time of each stage). */
+template<class T>
+struct alignas(8 * sizeof(T)) AVFullRec
 {
     T vx, vy, vz, c, vol, divv;
     T pad0, pad1;
@@ -124,6 +132,8 @@ struct ChainArrays
     ChainTape<T> tape;
     BatchView batch;
     AVRec<T>* avrec{nullptr};
+    T* vsig{nullptr};                 // signal velocity of the AV switches per particle, written by IAD
+    AVFullRec<T>* avfull{nullptr};    // set: the AV switches read these records and find the signal velocity themselves
     // VeDefGradh leaves the velocity of the hydro record to launchPackVelocity (the velocities of a typed host load
     // still in flight)
     bool recordNoVelocity{false};

@@ -53,10 +53,10 @@ __global__ void __launch_bounds__(kChainMaxThreads, sizeof(T) == 4 && kSplit == 
     for (unsigned round = 0; round < t.rounds; ++round)
     {
         overChunk<kSplit, false>(a.nidx, t, round, [&](uint32_t j) {
-        Pos<T> pj  = posOf(a, j);
-        Sep<T> r   = separation(pi, pj, 2.0 * hiD, box, k);
-        T r2       = dot3(r.rx, r.ry, r.rz, r.rx, r.ry, r.rz);
-        rho0.add(kernelWr2(a.wh, k, r2, hInv, hh) * T(pj.m));
+            Pos<T> pj  = posOf(a, j);
+            Sep<T> r   = separation(pi, pj, 2.0 * hiD, box, k);
+            T r2       = dot3(r.rx, r.ry, r.rz, r.rx, r.ry, r.rz);
+            rho0.add(kernelWr2(a.wh, k, r2, hInv, hh) * T(pj.m));
         });
         foldChunks<kSplit>(round * kSplit, t.numChunks, rho0);
     }
@@ -90,45 +90,45 @@ __global__ void __launch_bounds__(kChainMaxThreads, sizeof(T) == 4 && kSplit == 
     for (unsigned round = 0; round < t.rounds; ++round)
     {
         overChunk<kSplit, false>(a.nidx, t, round, [&](uint32_t j) {
-        Pos<T> pj  = posOf(a, j);
-        Sep<T> r   = separation(pi, pj, 2.0 * hiD, box, k);
-        T r2       = dot3(r.rx, r.ry, r.rz, r.rx, r.ry, r.rz);
-        T w, dterh;
-        if constexpr (sizeof(T) == 4)
-        {
-            if (k.usePoly)
+            Pos<T> pj  = posOf(a, j);
+            Sep<T> r   = separation(pi, pj, 2.0 * hiD, box, k);
+            T r2       = dot3(r.rx, r.ry, r.rz, r.rx, r.ry, r.rz);
+            T w, dterh;
+            if constexpr (sizeof(T) == 4)
             {
-                // t = v^2/2 - 1 from r2 (no square root); W and dW's polynomial side by side in packed FP32
-                // (sm_100 FFMA2); v dW = v^2 P'(t) = 2 (t + 1) P'(t) (0.638 -> 0.624 ms at 128^3)
-                float tt   = fmaf(r2, hhV, -1.0f);
-                float2 acc = make_float2(k.wpoly[kPolyTerms - 1], k.dwpoly[kPolyTerms - 1]);
-#pragma unroll
-                for (int p = kPolyTerms - 2; p >= 0; --p)
+                if (k.usePoly)
                 {
-                    acc = __ffma2_rn(acc, make_float2(tt, tt), make_float2(k.wpoly[p], k.dwpoly[p]));
+                    // t = v^2/2 - 1 from r2 (no square root); W and dW's polynomial side by side in packed FP32
+                    // (sm_100 FFMA2); v dW = v^2 P'(t) = 2 (t + 1) P'(t) (0.638 -> 0.624 ms at 128^3)
+                    float tt   = fmaf(r2, hhV, -1.0f);
+                    float2 acc = make_float2(k.wpoly[kPolyTerms - 1], k.dwpoly[kPolyTerms - 1]);
+#pragma unroll
+                    for (int p = kPolyTerms - 2; p >= 0; --p)
+                    {
+                        acc = __ffma2_rn(acc, make_float2(tt, tt), make_float2(k.wpoly[p], k.dwpoly[p]));
+                    }
+                    bool in = tt < 1.0f;
+                    w       = in ? acc.x : 0.0f;
+                    dterh   = in ? -prodSum(3.0f, acc.x, 2.0f * (tt + 1.0f), acc.y) : 0.0f;
                 }
-                bool in = tt < 1.0f;
-                w       = in ? acc.x : 0.0f;
-                dterh   = in ? -prodSum(3.0f, acc.x, 2.0f * (tt + 1.0f), acc.y) : 0.0f;
+                else
+                {
+                    T vloc = T(r2 * rsqrtf(float(r2))) * hInv;
+                    w      = kernelW(a.wh, k, vloc);
+                    dterh  = -prodSum(T(3), w, vloc, kernelDW(a.whd, k, vloc));
+                }
             }
             else
             {
-                T vloc = T(r2 * rsqrtf(float(r2))) * hInv;
+                T vloc = T(sqrt(r2)) * hInv;
                 w      = kernelW(a.wh, k, vloc);
-                dterh  = -prodSum(T(3), w, vloc, kernelDW(a.whd, k, vloc));
+                T dw   = kernelDW(a.whd, k, vloc);
+                dterh  = -prodSum(T(3), w, vloc, dw);
             }
-        }
-        else
-        {
-            T vloc = T(sqrt(r2)) * hInv;
-            w      = kernelW(a.wh, k, vloc);
-            T dw   = kernelDW(a.whd, k, vloc);
-            dterh  = -prodSum(T(3), w, vloc, dw);
-        }
-        T xmassj   = __ldg(a.xm + j);
-        kxS.add(w * xmassj);
-        whomegaS.add(dterh * xmassj);
-        wrho0S.add(dterh * T(pj.m));
+            T xmassj   = __ldg(a.xm + j);
+            kxS.add(w * xmassj);
+            whomegaS.add(dterh * xmassj);
+            wrho0S.add(dterh * T(pj.m));
         });
         foldChunks<kSplit>(round * kSplit, t.numChunks, kxS, whomegaS, wrho0S);
     }
@@ -211,6 +211,8 @@ __global__ void __launch_bounds__(kChainMaxThreads, sizeof(T) == 4 && kSplit == 
     double divvOut   = -INFINITY;
     BlockSum<T> s11, s12, s13, s22, s23, s33;
     BlockSum<T> mxx, mxy, mxz, myx, myy, myz, mzx, mzy, mzz;
+    T vsigI = T(0);
+    [[maybe_unused]] int vsigJ = -1;
     if (kSplit > 1 || valid)
     {
         Pos<T> pi      = posOf(a, t.i);
@@ -219,38 +221,59 @@ __global__ void __launch_bounds__(kChainMaxThreads, sizeof(T) == 4 && kSplit == 
         T hiInv        = T(1) / hi;
         T hh           = T(0.5) * hiInv * hiInv;
         HydroRec<T> hr = a.hrec[t.i];
+        vsigI          = T(1.e-40) * hr.c;
         for (unsigned round = 0; round < t.rounds; ++round)
         {
             overChunk<kSplit, false>(a.nidx, t, round, [&](uint32_t j) {
-            Pos<T> pj      = posOf(a, j);
-            HydroRec<T> hj = loadHydro(a.hrec + j);
-            Sep<T> r       = separation(pi, pj, 2.0 * hiD, box, k);
-            T r2           = dot3(r.rx, r.ry, r.rz, r.rx, r.ry, r.rz);
-            T w            = kernelWr2(a.wh, k, r2, hiInv, hh);
-            T voljW        = hj.vol * w;
-            s11.add(r.rx * r.rx * voljW);
-            s12.add(r.rx * r.ry * voljW);
-            s13.add(r.rx * r.rz * voljW);
-            s22.add(r.ry * r.ry * voljW);
-            s23.add(r.ry * r.rz * voljW);
-            s33.add(r.rz * r.rz * voljW);
-            T xw = hj.xm * w;
-            T fx = (hj.vx - hr.vx) * xw;
-            T fy = (hj.vy - hr.vy) * xw;
-            T fz = (hj.vz - hr.vz) * xw;
-            mxx.add(fx * r.rx);
-            mxy.add(fx * r.ry);
-            mxz.add(fx * r.rz);
-            myx.add(fy * r.rx);
-            myy.add(fy * r.ry);
-            myz.add(fy * r.rz);
-            mzx.add(fz * r.rx);
-            mzy.add(fz * r.ry);
-            mzz.add(fz * r.rz);
+                Pos<T> pj      = posOf(a, j);
+                HydroRec<T> hj = loadHydro(a.hrec + j);
+                Sep<T> r       = separation(pi, pj, 2.0 * hiD, box, k);
+                T r2           = dot3(r.rx, r.ry, r.rz, r.rx, r.ry, r.rz);
+                T dvx = hj.vx - hr.vx, dvy = hj.vy - hr.vy, dvz = hj.vz - hr.vz;
+                T rv  = dot3(r.rx, r.ry, r.rz, dvx, dvy, dvz);
+                T rinv, w;
+                if constexpr (sizeof(T) == 4)
+                {
+                    rinv = rsqrtf(r2);
+                    w    = kernelWr2(a.wh, k, r2, hiInv, hh);
+                }
+                else
+                {
+                    rinv = rsqrt(r2);
+                    w    = kernelW(a.wh, k, r2 * rinv * hiInv);
+                }
+                // the AV switches' signal velocity c_i + c_j - 3 r.v_ij / r over approaching pairs
+                T vsig = rv > T(0) ? fma(T(3) * rv, rinv, hr.c + hj.c) : T(0);
+                if constexpr (kMode & kModeTape)
+                {
+                    if (!(vsigI > vsig)) { vsigJ = int(j); }
+                }
+                vsigI   = vsigI > vsig ? vsigI : vsig;
+                T voljW = hj.vol * w;
+                s11.add(r.rx * r.rx * voljW);
+                s12.add(r.rx * r.ry * voljW);
+                s13.add(r.rx * r.rz * voljW);
+                s22.add(r.ry * r.ry * voljW);
+                s23.add(r.ry * r.rz * voljW);
+                s33.add(r.rz * r.rz * voljW);
+                T xw = hj.xm * w;
+                T fx = dvx * xw;
+                T fy = dvy * xw;
+                T fz = dvz * xw;
+                mxx.add(fx * r.rx);
+                mxy.add(fx * r.ry);
+                mxz.add(fx * r.rz);
+                myx.add(fy * r.rx);
+                myy.add(fy * r.ry);
+                myz.add(fy * r.rz);
+                mzx.add(fz * r.rx);
+                mzy.add(fz * r.ry);
+                mzz.add(fz * r.rz);
             });
             foldChunks<kSplit>(round * kSplit, t.numChunks, s11, s12, s13, s22, s23, s33, mxx, mxy, mxz, myx, myy, myz,
                                mzx, mzy, mzz);
         }
+        vsigI = maxOverSplit<kSplit>(vsigI);
     }
     if (valid && t.sub == 0)
     {
@@ -324,7 +347,9 @@ __global__ void __launch_bounds__(kChainMaxThreads, sizeof(T) == 4 && kSplit == 
         a.divv[t.i]   = divv;
         a.curlv[t.i]  = curlv;
         a.grec[t.i]   = GradRec<T>{c11i, c12i, c13i, c22i, c23i, c33i, divv, T(a.alpha[t.i])};
-        a.avrec[t.i]  = AVRec<T>{hr.vx, hr.vy, hr.vz, hr.c, hr.vol, divv, T(0), T(0)};
+        a.avrec[t.i]  = AVRec<T>{hr.vol, divv};
+        a.vsig[t.i]   = vsigI;
+        if constexpr (kMode & kModeTape) { a.tape.vsigJ[t.i] = vsigJ; }
         divvOut       = double(divv);
     }
     reduceOrdered<true, (kMode & kModeBatch) != 0>(divvOut, a.n, a.reduce + 0, a.batch, 0);
@@ -333,10 +358,11 @@ __global__ void __launch_bounds__(kChainMaxThreads, sizeof(T) == 4 && kSplit == 
 // ---------------------------------------------------------------------------------------------------------------
 // AV switches (sph/include/sph/hydro_ve/av_switches_kern.hpp:43-137)
 // ---------------------------------------------------------------------------------------------------------------
-// FP32: up to 384 threads, run in 384-thread blocks (12 consecutive groups sharing their neighbours in L1), measured
-// 0.817 -> 0.795 ms at 128^3 against 256; at most 56 registers for three such blocks per SM. FP64 keeps the common
-// bound with no block minimum (0): an explicit minimum of 1 raised it from 96 to 108 registers and slowed it from
-// 2.45 to 2.64 ms at 128 threads.
+// The signal velocity comes from IAD's loop, so a neighbour costs a 16-byte position and an 8-byte record here instead of
+// a 32-byte one with velocity and sound speed (the loop was bound by its gathers, at 90 % of the L1's throughput): FP32
+// 0.760 -> 0.476 ms at 128^3 for 0.142 ms more in IAD, FP64 1.24 -> 0.70 ms at 101^3 for 0.02.
+// FP32: up to 384 threads, run in 384-thread blocks (12 consecutive groups sharing their neighbours in L1); at most 56
+// registers for three such blocks per SM. FP64 keeps the common bound with no block minimum.
 template<class T, int kMode, int kSplit>
 __global__ void __launch_bounds__(sizeof(T) == 4 ? kAvMaxThreads : kChainMaxThreads, sizeof(T) == 4 && kSplit == 1 ? 3 : 0)
     avSwitchesKernel(ChainArrays<T> a, HydroConsts<T> k, DevBox box, double dt)
@@ -350,7 +376,7 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? kAvMaxThreads : kChainMaxThre
     GradRec<T> gr  = a.grec[t.i];
     T hi           = T(hiD);
     T ci           = hr.c;
-    T vijsignalI   = T(1.e-40) * ci;
+    T vijsignalI   = (kMode & kModeFullAv) ? T(1.e-40) * ci : a.vsig[t.i];
     T hiInv        = T(1) / hi;
     T hiInv3       = hiInv * hiInv * hiInv;
     T KhiInv3      = k.K * hiInv3;
@@ -358,42 +384,41 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? kAvMaxThreads : kChainMaxThre
     T divvI        = gr.divv;
 
     BlockSum<T> gx, gy, gz;
-    int vsigJ = -1;
     for (unsigned round = 0; round < t.rounds; ++round)
     {
         overChunk<kSplit, false>(a.nidx, t, round, [&](uint32_t j) {
-        Pos<T> pj      = posOf(a, j);
-        AVRec<T> hj    = loadAV(a.avrec + j);
-        T divvJ        = hj.divv;
-        Sep<T> r       = separation(pi, pj, 2.0 * hiD, box, k);
-        T r2           = dot3(r.rx, r.ry, r.rz, r.rx, r.ry, r.rz);
-        T rv           = dot3(r.rx, r.ry, r.rz, hr.vx - hj.vx, hr.vy - hj.vy, hr.vz - hj.vz);
-        // 1/r from one rsqrt: 3 r.v / r without a division, and in FP64 r itself for the kernel's table
-        T vsig = T(0);
-        [[maybe_unused]] T rinv = T(0);
-        if constexpr (sizeof(T) == 8) { rinv = rsqrt(r2); }
-        if (rv < T(0))
-        {
-            if constexpr (sizeof(T) == 4) { rinv = rsqrtf(r2); }
-            vsig = fma(T(-3) * rv, rinv, ci + hj.c);
-        }
-        if constexpr (kMode & kModeTape)
-        {
-            if (!(vijsignalI > vsig)) { vsigJ = int(j); }
-        }
-        vijsignalI = vijsignalI > vsig ? vijsignalI : vsig;
-        T W;
-        if constexpr (sizeof(T) == 4) { W = kernelWr2(a.wh, k, r2, hiInv, hh); }
-        else { W = kernelW(a.wh, k, r2 * rinv * hiInv); }
-        // sum fac W r and apply -C_i once after the loop (the same vector, 9 FMAs less per pair)
-        T sw = hj.vol * (divvI - divvJ) * (KhiInv3 * W);
-        gx.add(sw * r.rx);
-        gy.add(sw * r.ry);
-        gz.add(sw * r.rz);
+            Pos<T> pj = posOf(a, j);
+            T volJ, divvJ;
+            Sep<T> r  = separation(pi, pj, 2.0 * hiD, box, k);
+            T r2      = dot3(r.rx, r.ry, r.rz, r.rx, r.ry, r.rz);
+            if constexpr (kMode & kModeFullAv)
+            {
+                AVFullRec<T> hj = loadAV(a.avfull + j);
+                volJ            = hj.vol;
+                divvJ           = hj.divv;
+                T rv            = dot3(r.rx, r.ry, r.rz, hj.vx - hr.vx, hj.vy - hr.vy, hj.vz - hr.vz);
+                T rinv;
+                if constexpr (sizeof(T) == 4) { rinv = rsqrtf(r2); }
+                else { rinv = rsqrt(r2); }
+                T vsig     = rv > T(0) ? fma(T(3) * rv, rinv, ci + hj.c) : T(0);
+                vijsignalI = vijsignalI > vsig ? vijsignalI : vsig;
+            }
+            else
+            {
+                AVRec<T> hj = loadAV(a.avrec + j);
+                volJ        = hj.vol;
+                divvJ       = hj.divv;
+            }
+            T W = kernelWr2(a.wh, k, r2, hiInv, hh);
+            // sum fac W r and apply -C_i once after the loop (the same vector, 9 FMAs less per pair)
+            T sw = volJ * (divvI - divvJ) * (KhiInv3 * W);
+            gx.add(sw * r.rx);
+            gy.add(sw * r.ry);
+            gz.add(sw * r.rz);
         });
         foldChunks<kSplit>(round * kSplit, t.numChunks, gx, gy, gz);
     }
-    vijsignalI = maxOverSplit<kSplit>(vijsignalI);
+    if constexpr (kMode & kModeFullAv) { vijsignalI = maxOverSplit<kSplit>(vijsignalI); }
     if (kSplit > 1 && (!valid || t.sub != 0)) { return; }
     T gdx = gx.get(), gdy = gy.get(), gdz = gz.get();
     {
@@ -409,7 +434,6 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? kAvMaxThreads : kChainMaxThre
         a.tape.gy[t.i]    = gdy;
         a.tape.gz[t.i]    = gdz;
         a.tape.vsig[t.i]  = vijsignalI;
-        a.tape.vsigJ[t.i] = vsigJ;
     }
     T alphaI   = T(a.alpha[t.i]);
     T alphaloc = T(0);
@@ -840,7 +864,12 @@ template<class T>
 int launchAVswitches(const ChainArrays<T>& a, const HydroConsts<T>& k, const DevBox& box, double dt, cudaStream_t s)
 {
     if (a.n == 0 || (a.groupList && a.numListed == 0)) { return kOk; }
-    SPHB_DISPATCH(avSwitchesKernel, a, k, box, dt)
+    if (a.avfull)
+    {
+        if (chainMode(a) != 0) { return kErrArg; }
+        SPHB_LAUNCH_SPLIT(avSwitchesKernel, kModeFullAv, a, k, box, dt)
+    }
+    else { SPHB_DISPATCH(avSwitchesKernel, a, k, box, dt) }
     countLaunch();
     SPHB_CUDA_TRY(cudaGetLastError());
     return kOk;

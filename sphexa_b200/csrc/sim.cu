@@ -39,7 +39,8 @@ int allocateSim(sphb_sim& s)
     SPHB_TRY(s.du.reserve(n));
     SPHB_TRY(s.hrec.reserve(n * 8 * s.elemBytes()));
     SPHB_TRY(s.grec.reserve(n * 8 * s.elemBytes()));
-    SPHB_TRY(s.avrec.reserve(n * 8 * s.elemBytes()));
+    SPHB_TRY(s.avrec.reserve(n * 2 * s.elemBytes()));
+    SPHB_TRY(s.vsig.reserve(n * s.elemBytes()));
     if (s.p.av_clean)
     {
         SPHB_TRY(s.dvrec.reserve(n * 8 * s.elemBytes()));
@@ -271,6 +272,8 @@ ChainArrays<T> chainArrays(sphb_sim& s)
     a.grec   = reinterpret_cast<GradRec<T>*>(s.grec.data());
     a.reduce = s.reduce.data();
     a.avrec  = reinterpret_cast<AVRec<T>*>(s.avrec.data());
+    a.vsig   = reinterpret_cast<T*>(s.vsig.data());
+    if (s.avFromDataset) { a.avfull = reinterpret_cast<AVFullRec<T>*>(s.avfull.data()); }
     if (s.p.av_clean)
     {
         a.dvrec = reinterpret_cast<DVRec<T>*>(s.dvrec.data());
@@ -1053,7 +1056,6 @@ std::vector<std::pair<void*, size_t>> tapedBuffers(sphb_sim& s)
     b.push_back({s.du.data(), n * sizeof(double)});
     b.push_back({s.hrec.data(), n * 8 * e});
     b.push_back({s.grec.data(), n * 8 * e});
-    b.push_back({s.avrec.data(), n * 8 * e});
     b.push_back({s.tapeT.data(), 8 * n * e});
     b.push_back({s.tapeJ.data(), n * sizeof(int)});
     b.push_back({s.hPre.data(), n * sizeof(double)});

@@ -68,7 +68,9 @@ struct sphb_sim
     DeviceBuffer<unsigned> nc;
     DeviceBuffer<char> derived[kNumDerived];
     DeviceBuffer<double> du;
-    DeviceBuffer<char> hrec, grec, avrec;
+    DeviceBuffer<char> hrec, grec, avrec, vsig;
+    DeviceBuffer<char> avfull;  // stages on a caller's dataset only: the AV switches' records with velocity and c
+    bool avFromDataset{false};  // the AV stage that runs next is a dataset's
     DeviceBuffer<char> dvrec, dv; // AV cleaning only: symmetrised velocity gradients (record + 6 arrays)
     DeviceBuffer<double> whD, whdD;
     DeviceBuffer<float> whF, whdF;
