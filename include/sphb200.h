@@ -168,7 +168,7 @@ int sphb_build_octree(const uint64_t* leaves, size_t num_leaves, uint64_t* prefi
 int sphb_ideal_gas_eos(size_t first, size_t last, double mui, double gamma, const sphb_field* fields, int num_fields,
                        void* stream);
 
-/*! Fully converged cornerstone leaf array for sorted keys (host-blocking: loops until no node splits or merges).
+/*! Fully converged cornerstone leaf array for sorted keys, built in one go (host-blocking: reads back the leaf count).
  *  Writes num_leaves + 1 keys to leaves and num_leaves counts, if num_leaves + 1 <= capacity.
  *  Replaces cstone::computeOctree / updateOctree (domain/include/cstone/tree/csarray.hpp:409-440) and their GPU
  *  counterparts computeNodeCountsGpu / rebalanceTreeGpu (csarray_gpu.cu:85-213). */

@@ -1054,7 +1054,6 @@ extern "C" int sphb_compute_octree(const uint64_t* sorted_keys, size_t n, unsign
 {
     using namespace sphb;
     if (!num_leaves || bucket == 0 || (n && !sorted_keys)) { return SPHB_ERR_ARG; }
-    if (n >= (size_t(1) << 30)) { return SPHB_ERR_ARG; }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     size_t numTiles = (n + 1 + kConvTile - 1) / kConvTile;
     // per tile: the level clamp (two ints), the leaves opened, and the scan's scratch

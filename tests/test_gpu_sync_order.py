@@ -119,3 +119,54 @@ def test_linked_octree(cuda_device, n, bucket):
     i2l, l2i = i2l.cpu().numpy(), l2i.cpu().numpy()
     assert np.array_equal(np.sort(l2i), np.arange(nn))
     assert np.array_equal(i2l[l2i], np.arange(nn) - (nl - 1) // 7)
+
+
+def _canonical(keys, bucket):
+    """leaf starts of the cornerstone tree of sorted keys: a node with more than bucket keys splits, down to level 21"""
+    leaves = []
+    todo = [(0, 0, 0, len(keys))]
+    while todo:
+        start, level, a, b = todo.pop()
+        if b - a <= bucket or level == 21:
+            leaves.append(start)
+            continue
+        width = 1 << (63 - 3 * (level + 1))
+        cuts = [start + d * width for d in range(9)]
+        at = [a + int(np.searchsorted(keys[a:b], np.uint64(c))) for c in cuts[:8]] + [b]
+        todo.extend((cuts[d], level + 1, at[d], at[d + 1]) for d in range(8))
+    return np.array(sorted(leaves) + [1 << 63], dtype=np.uint64)
+
+
+@pytest.mark.parametrize("bucket", [1, 8])
+@pytest.mark.parametrize("kind", ["spread", "clustered", "equal", "deepest", "last"])
+@pytest.mark.parametrize("n", [0, 1, 8, 9, 2049, 20_000])
+def test_converged_leaves(cuda_device, n, kind, bucket):
+    import torch
+    from sphexa_b200 import lib as L
+    lib = L.load()
+    rng = np.random.default_rng(n)
+    k = rng.integers(0, 1 << 63, n, dtype=np.uint64)
+    if kind == "clustered":
+        k[: n // 2] >>= np.uint64(20)
+    if kind == "equal":
+        k[: n // 2] = np.uint64(0x123456789abcdef)
+    if kind == "deepest":  # neighbouring cells of the deepest level
+        k[: n // 2] = np.uint64(0x3fffffffffffffff) + rng.integers(0, 4, n // 2, dtype=np.uint64)
+    if kind == "last":
+        k[: n // 2] = np.uint64((1 << 63) - 1)
+    k = np.sort(k)
+    want = _canonical(k, bucket)
+    keys = torch.from_numpy(k.view(np.int64)).cuda()
+    cap = want.size + 7
+    leaves = torch.full((cap,), -1, dtype=torch.int64, device="cuda")
+    counts = torch.zeros(cap, dtype=torch.int32, device="cuda")
+    num = C.c_size_t()
+    torch.cuda.synchronize()
+    L.check(lib.sphb_compute_octree(L.ptr(keys), n, bucket, L.ptr(leaves), L.ptr(counts), cap, C.byref(num), None), "t")
+    assert num.value == want.size - 1
+    assert np.array_equal(leaves.cpu().numpy()[:want.size].view(np.uint64), want)
+    assert np.all(leaves.cpu().numpy()[want.size:] == -1)
+    assert np.array_equal(counts.cpu().numpy()[:num.value], np.diff(np.searchsorted(k, want[:-1], "left"), append=n))
+    # no room, or only the count asked for: the number of leaves all the same
+    rc = lib.sphb_compute_octree(L.ptr(keys), n, bucket, L.ptr(leaves), L.ptr(counts), num.value, C.byref(num), None)
+    assert rc == L.SPHB_ERR_CAPACITY and num.value == want.size - 1
