@@ -182,6 +182,40 @@ __device__ __forceinline__ void scatterPos(const AdjArrays<T>& g, uint32_t j, co
     atomicAdd(g.z + j, -rb.z);
 }
 
+/*! The same with one more scalar for the neighbour, x into field[j]. FP32: one vector atomic {x, y, z, x} into plane 0 of
+ *  the neighbour sums (jacc + j) instead of four scalar ones; foldScatterKernel adds the plane into the fields. */
+template<class T>
+__device__ __forceinline__ void scatterPos(const AdjArrays<T>& g, uint32_t j, const V3<T>& rb, T x, T* field)
+{
+    if constexpr (sizeof(T) == 4)
+    {
+        if (g.jacc)
+        {
+            atomicAdd(g.jacc + j, make_float4(-rb.x, -rb.y, -rb.z, x));
+            return;
+        }
+    }
+    scatterPos(g, j, rb);
+    if (field) { atomicAdd(field + j, x); }
+}
+
+//! scatter the adjoint of a neighbour's velocity: plane 1 of the neighbour sums, as above
+template<class T>
+__device__ __forceinline__ void scatterVel(const AdjArrays<T>& g, size_t n, uint32_t j, T bx, T by, T bz)
+{
+    if constexpr (sizeof(T) == 4)
+    {
+        if (g.jacc)
+        {
+            atomicAdd(g.jacc + n + j, make_float4(bx, by, bz, 0.0f));
+            return;
+        }
+    }
+    atomicAdd(g.vx + j, bx);
+    atomicAdd(g.vy + j, by);
+    atomicAdd(g.vz + j, bz);
+}
+
 template<class T>
 __device__ __forceinline__ V3<T> sepV(const Sep<T>& r)
 {
@@ -197,8 +231,13 @@ __global__ void foldNeighbourSumsKernel(size_t n, AdjArrays<T> g)
 {
     size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
     if (i >= n) { return; }
-    const float4* q = g.jacc + i * 5;
+    float4* q = g.jacc + i * 5;
     float4 a = q[0], b = q[1], c = q[2], d = q[3], e = q[4];
+#pragma unroll
+    for (int s = 0; s < 5; ++s)
+    {
+        q[s] = make_float4(0.f, 0.f, 0.f, 0.f); // for the planes of the later kernels
+    }
     g.x[i] += a.x;
     g.y[i] += a.y;
     g.z[i] += a.z;
@@ -217,6 +256,30 @@ __global__ void foldNeighbourSumsKernel(size_t n, AdjArrays<T> g)
     g.prho[i] += d.w;
     g.xm[i] += e.x;
     g.vol[i] += e.y;
+}
+
+/*! add the planes of neighbour sums of scatterPos (x, y, z and, if set, one more field) and scatterVel into the
+ *  per-field adjoints, and clear them. The pair loops' adjoints are bound by their atomics: one float4 per pair and plane
+ *  instead of a scalar per field (48^3 FP32, us by the profiler: divv 272 -> 124, VeDefGradh 184 -> 86, IAD 177 -> 88,
+ *  XMass 139 -> 70, AV switches 157 -> 101; a fold takes 12). */
+template<class T>
+__global__ void foldScatterKernel(size_t n, AdjArrays<T> g, T* extra, bool velocity)
+{
+    size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
+    if (i >= n) { return; }
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 a          = g.jacc[i];
+    g.jacc[i]         = zero;
+    g.x[i] += a.x;
+    g.y[i] += a.y;
+    g.z[i] += a.z;
+    if (extra) { extra[i] += a.w; }
+    if (!velocity) { return; }
+    float4 b      = g.jacc[n + i];
+    g.jacc[n + i] = zero;
+    g.vx[i] += b.x;
+    g.vy[i] += b.y;
+    g.vz[i] += b.z;
 }
 
 template<class T>
@@ -674,7 +737,7 @@ __global__ void __launch_bounds__(kChainThreads) avSwitchesVjpKernel(ChainArrays
                     T f       = hj.vol * (divvI - divvJ);
                     T fB      = dot3(gB, tA);
                     V3<T> tAB = {f * gB.x, f * gB.y, f * gB.z};
-                    atomicAdd(g.vol + j, fB * (divvI - divvJ));
+                    T volB    = fB * (divvI - divvJ);
                     divviB += fB * hj.vol;
                     atomicAdd(g.divv + j, -fB * hj.vol);
                     T WiB     = -dot3(cr, tAB);
@@ -693,7 +756,7 @@ __global__ void __launch_bounds__(kChainThreads) avSwitchesVjpKernel(ChainArrays
                     xiB.x += rB.x;
                     xiB.y += rB.y;
                     xiB.z += rB.z;
-                    scatterPos(g, j, rB);
+                    scatterPos(g, j, rB, volB, g.vol);
                 }
             }
         }
@@ -781,13 +844,11 @@ __global__ void __launch_bounds__(kChainThreads) divvVjpKernel(ChainArrays<T> a,
             // term = xm_j dv . tA
             V3<T> fB  = {DB * tA.x, DB * tA.y, DB * tA.z};
             V3<T> tAB = {DB * dv.x * hj.xm, DB * dv.y * hj.xm, DB * dv.z * hj.xm};
-            atomicAdd(g.vx + j, fB.x * hj.xm);
-            atomicAdd(g.vy + j, fB.y * hj.xm);
-            atomicAdd(g.vz + j, fB.z * hj.xm);
+            scatterVel(g, a.n, j, fB.x * hj.xm, fB.y * hj.xm, fB.z * hj.xm);
             viB.x -= fB.x * hj.xm;
             viB.y -= fB.y * hj.xm;
             viB.z -= fB.z * hj.xm;
-            atomicAdd(g.xm + j, DB * dot3(dv, tA));
+            T xmB     = DB * dot3(dv, tA);
             T wB      = -dot3(cr, tAB);
             V3<T> ctb = symMul(ci6, tAB);
             V3<T> rB  = {-wk * ctb.x, -wk * ctb.y, -wk * ctb.z};
@@ -804,7 +865,7 @@ __global__ void __launch_bounds__(kChainThreads) divvVjpKernel(ChainArrays<T> a,
             xiB.x += rB.x;
             xiB.y += rB.y;
             xiB.z += rB.z;
-            scatterPos(g, j, rB);
+            scatterPos(g, j, rB, xmB, g.xm);
         }
     }
     atomicAdd(g.x + t.i, xiB.x);
@@ -896,7 +957,6 @@ __global__ void __launch_bounds__(kChainThreads) iadVjpKernel(ChainArrays<T> a, 
                         tb[2][0] * r.x + tb[2][1] * r.y + tb[2][2] * r.z};
             T wB     = dot3(r, tr);
             V3<T> rB = {T(2) * w * tr.x, T(2) * w * tr.y, T(2) * w * tr.z};
-            atomicAdd(g.vol + j, wB * wk);
             T vB = wB * hj.vol * dwk;
             hiB -= vB * v * hiInv;
             if (dist > T(0))
@@ -909,7 +969,7 @@ __global__ void __launch_bounds__(kChainThreads) iadVjpKernel(ChainArrays<T> a, 
             xiB.x += rB.x;
             xiB.y += rB.y;
             xiB.z += rB.z;
-            scatterPos(g, j, rB);
+            scatterPos(g, j, rB, wB * wk, g.vol);
         }
     }
     atomicAdd(g.x + t.i, xiB.x);
@@ -1003,20 +1063,16 @@ __global__ void __launch_bounds__(kChainThreads) veDefGradhVjpKernel(ChainArrays
             T dterh  = -(T(3) * w + v * d);
             T xmassj = __ldg(a.xm + j);
             T mj     = T(pj.m);
-            atomicAdd(g.xm + j, kxSB * w + whSB * dterh);
             T wB     = kxSB * xmassj;
             T dterhB = whSB * xmassj + wrSB * mj;
             T vB     = wB * dw - dterhB * (T(3) * dw + d + v * dd);
             hiB -= vB * v * hInv;
-            if (dist > T(0))
-            {
-                T fd     = overDist(vB * hInv, dist, rinv);
-                V3<T> rB = {fd * r.x, fd * r.y, fd * r.z};
-                xiB.x += rB.x;
-                xiB.y += rB.y;
-                xiB.z += rB.z;
-                scatterPos(g, j, rB);
-            }
+            T fd     = dist > T(0) ? overDist(vB * hInv, dist, rinv) : T(0);
+            V3<T> rB = {fd * r.x, fd * r.y, fd * r.z};
+            xiB.x += rB.x;
+            xiB.y += rB.y;
+            xiB.z += rB.z;
+            scatterPos(g, j, rB, kxSB * w + whSB * dterh, g.xm);
         }
     }
     atomicAdd(g.x + t.i, xiB.x);
@@ -1071,7 +1127,7 @@ __global__ void __launch_bounds__(kChainThreads) xmassVjpKernel(ChainArrays<T> a
                 xiB.x += rB.x;
                 xiB.y += rB.y;
                 xiB.z += rB.z;
-                scatterPos(g, j, rB);
+                scatterPos(g, j, rB, T(0), static_cast<T*>(nullptr));
             }
         }
     }
@@ -1130,28 +1186,46 @@ int stepVjp(const ChainArrays<T>& a, const HydroConsts<T>& k, const DevBox& box,
     T* fields[kNumAdjFields] = {g.x,      g.y,      g.z,      g.vx,     g.vy,     g.vz,    g.h,    g.c,  g.prho,
                                 g.alpha,  g.cij[0], g.cij[1], g.cij[2], g.cij[3], g.cij[4], g.cij[5], g.divv, g.xm,
                                 g.vol,    g.kx,     g.gradh,  g.ax,     g.ay,     g.az,     g.du};
-    for (T* f : fields)
+    // neighbouring arrays in one memset
+    for (int q = 0; q < kNumAdjFields;)
     {
-        SPHB_CUDA_TRY(cudaMemsetAsync(f, 0, s.n * sizeof(T), stream));
+        int e = q + 1;
+        while (e < kNumAdjFields && fields[e] == fields[e - 1] + s.n)
+        {
+            ++e;
+        }
+        SPHB_CUDA_TRY(cudaMemsetAsync(fields[q], 0, size_t(e - q) * s.n * sizeof(T), stream));
+        q = e;
     }
+    const bool vectorSums = sizeof(T) == 4 && g.jacc;
+    auto fold             = [&](T* extra, bool velocity) {
+        if (!vectorSums) { return; }
+        foldScatterKernel<T><<<ceilDiv(a.n, 256), 256, 0, stream>>>(a.n, g, extra, velocity);
+        countLaunch();
+    };
     integrationVjpKernel<T><<<nb, kChainThreads, 0, stream>>>(s, a.nc, post, work, g);
-    if (sizeof(T) == 4 && g.jacc)
+    if (vectorSums)
     {
         SPHB_CUDA_TRY(cudaMemsetAsync(g.jacc, 0, a.n * 5 * sizeof(float4), stream));
     }
     momentumEnergyVjpKernel<T><<<nb, kChainThreads, 0, stream>>>(a, k, box, g);
-    if (sizeof(T) == 4 && g.jacc)
+    if (vectorSums)
     {
         foldNeighbourSumsKernel<T><<<ceilDiv(a.n, 256), 256, 0, stream>>>(a.n, g);
         countLaunch();
     }
     avSwitchesVjpKernel<T><<<nb, kChainThreads, 0, stream>>>(a, k, box, s.dtAV, s.alphaPre, g, work.f[13],
                                                               s.alphamaxBar);
+    fold(g.vol, false);
     divvVjpKernel<T><<<nb, kChainThreads, 0, stream>>>(a, k, box, g);
+    fold(g.xm, true);
     iadVjpKernel<T><<<nb, kChainThreads, 0, stream>>>(a, k, box, g);
+    fold(g.vol, false);
     volEosVjpKernel<T><<<nb, kChainThreads, 0, stream>>>(a, s, g, work);
     veDefGradhVjpKernel<T><<<nb, kChainThreads, 0, stream>>>(a, k, box, g);
+    fold(g.xm, false);
     xmassVjpKernel<T><<<nb, kChainThreads, 0, stream>>>(a, k, box, g);
+    fold(nullptr, false);
     finalizeVjpKernel<T><<<nb, kChainThreads, 0, stream>>>(a, s, g, work, pre);
     for (int q = 0; q < 9; ++q)
     {
