@@ -13,6 +13,8 @@
 // (depth-first octree traversal over SFC-ordered leaves), including which neighbours are kept when more than ngmax
 // qualify. The smoothing-length iteration of sph/include/sph/find_neighbors.hpp:10-41 is fused: lanes whose count
 // left [ng0/4, ngmax+1] update h and search again, at most maxIterations times; settled lanes keep their lists.
+#include <algorithm>
+
 #include "neighbors.cuh"
 #include "primitives.cuh"
 
@@ -27,8 +29,23 @@ constexpr int kNbThreads = kNbWarps * kWarp;
 constexpr int kStackCap  = 176; // depth-first stack: <= 7 pending siblings per level + 8
 constexpr int kLeafCap   = 256; // candidate leaves buffered before they are streamed
 
+/*! Lanes that share a target. One lane per target tests and appends for its own particle, 32 targets per warp. A group's
+ *  traversal, staging and tests run one after another, so a launch of few groups takes as long as its slowest one, with
+ *  most of the GPU idle. With four lanes per target a warp serves eight targets: each lane tests and appends a quarter of
+ *  the staged candidates, and the smaller search box admits about half of them. But each box is traversed and staged by
+ *  itself, so a launch that fills the GPU is slower with it: hence the limits below.
+ *  Whole searches, us for one and for four lanes: 16^3 particles 117 and 75, 30^3 167 and 122, 36^3 203 and 144; 50^3 327
+ *  and 426, 63^3 394 and 579, 81^3 702 and 939. Searches of listed groups, a small part of all: block time steps of 64^3
+ *  509 and 452; 128^3 1569 and 1690 (with the rest of the phase). */
+constexpr int kSharedLanes          = 4;
+constexpr size_t kSharedLanesAll    = 40000;
+constexpr size_t kSharedLanesListed = 300000;
+
+template<int kPer>
 struct NbShared
 {
+    //! list entries a target buffers: the chunk being filled; where lanes share it, up to 32 more neighbours at a time
+    static constexpr int kRing = kPer == 1 ? kNbChunk : 5 * kNbChunk;
     int stack[kNbWarps][kStackCap];
     int leafFirst[kNbWarps][kLeafCap]; // first particle of each buffered leaf
     int leafEnd[kNbWarps][kLeafCap];   // one past its last particle
@@ -41,10 +58,10 @@ struct NbShared
     alignas(16) float cy[kNbWarps][kWarp];
     alignas(16) float cz[kNbWarps][kWarp];
     int cj[kNbWarps][kWarp];
-    // per lane: the neighbours of the list chunk being filled, written out as one 32-byte sector when full; lane
-    // minor, so that the lanes' appends fall into distinct banks
-    uint32_t nbuf[kNbWarps][kNbChunk][kWarp];
-    uint16_t dbuf[kNbWarps][kNbChunk][kWarp]; // skin rows: the quantised build distance of each entry
+    // per target: the neighbours of the list chunks being filled, written out as 32-byte sectors when full; target minor,
+    // so that the appends of a warp fall into distinct banks
+    uint32_t nbuf[kNbWarps][kRing * kWarp / kPer];
+    uint16_t dbuf[kNbWarps][kRing * kWarp / kPer]; // skin rows: the quantised build distance of each entry
 };
 
 /*! Half width of the band |d^2 - (2h)^2| < band * (2h)^2 in which the FP32 distance cannot decide and the exact FP64
@@ -128,7 +145,7 @@ struct SearchExtras
     unsigned gateMask;
 };
 
-template<bool kBatched, int kKind>
+template<bool kBatched, int kKind, int kPer>
 __global__ void __launch_bounds__(kNbThreads, 8) findNeighborsKernel(const double* __restrict__ x,
                                                                   const double* __restrict__ y,
                                                                   const double* __restrict__ z,
@@ -139,24 +156,25 @@ __global__ void __launch_bounds__(kNbThreads, 8) findNeighborsKernel(const doubl
                                                                   const TreeView* __restrict__ views,
                                                                   const uint8_t* __restrict__ inst, SearchExtras ex)
 {
-    __shared__ NbShared sh;
+    __shared__ NbShared<kPer> sh;
     if (ex.gate && !((ex.gateMask >> __ldg(ex.gate)) & 1u)) { return; }
+    constexpr int kTargets = kWarp / kPer; // targets of a warp
     const int warp         = threadIdx.x / kWarp;
     const int lane         = threadIdx.x & (kWarp - 1);
+    const int piece        = lane % kPer; // which of the lanes that share the target
     const size_t numGroups = (n + kWarp - 1) / kWarp;
-    size_t group           = size_t(blockIdx.x) * kNbWarps + warp;
-    if constexpr (kKind == kSearchListed)
-    {
-        if (group >= *ex.numListed) { return; }
-        group = ex.groups[group];
-    }
+    // kPer warps per group of 32
+    auto searchUnit = [&](size_t unit) {
+    size_t group = unit / kPer;
+    if constexpr (kKind == kSearchListed) { group = ex.groups[group]; }
     if (group >= numGroups) { return; }
+    const unsigned slot = unsigned(unit % kPer) * kTargets + lane / kPer; // the target's place in its group
     constexpr bool kSkin = kKind == kSearchSkin;
     // the lists written: neighbour lists (ngmax entries) or skin rows (cap entries)
     uint32_t* const outList  = kSkin ? ex.sl.rows : nidx;
     const unsigned listCap   = kSkin ? ex.sl.cap : prm.ngmax;
 
-    const size_t i = group * kWarp + lane;
+    const size_t i = group * kWarp + slot;
     // an ensemble: the group's instance (its first slot is never padding) selects the tree; padding slots idle
     TreeView tv = tree;
     if constexpr (kBatched) { tv = views[inst[group * kWarp]]; }
@@ -236,9 +254,12 @@ __global__ void __launch_bounds__(kNbThreads, 8) findNeighborsKernel(const doubl
         if (active) { count = 0; }
         int numLeaves = 0;
 
-        // this lane's chunk buffer and its store to the chunked list layout (nidxAt)
-        uint32_t* chunk     = &sh.nbuf[warp][0][lane];
-        uint16_t* dchunk    = &sh.dbuf[warp][0][lane];
+        // this target's ring of list chunks, entry e at ring[(e mod kRing) * kStride], and the store of a full chunk to the
+        // chunked list layout (nidxAt)
+        constexpr int kRing   = NbShared<kPer>::kRing;
+        constexpr int kStride = kTargets;
+        uint32_t* ring        = &sh.nbuf[warp][lane / kPer];
+        uint16_t* dring       = &sh.dbuf[warp][lane / kPer];
         // skin rows: distance -> units of R / kSkinDistUnits. The FP32 distance of the pair serves where it is known
         // to kSkinDistSlack units: both coordinates are rounded once relative to the group centre, 2^-24 reach each,
         // and the FP32 arithmetic adds at most 4 * 2^-24 R, together 2^-24 (3.5 reach + 4 R) < 1.3e-6 R = 0.084 units
@@ -247,38 +268,65 @@ __global__ void __launch_bounds__(kNbThreads, 8) findNeighborsKernel(const doubl
         const float qScaleF  = float(qScale);
         const bool exactDist = wrapTest || reach > 5.f * twoH;
         auto storeChunk = [&](unsigned c) {
-            uint32_t* dst = outList + nidxAt(group, ngPad, c * kNbChunk, lane);
+            uint32_t* dst         = outList + nidxAt(group, ngPad, c * kNbChunk, slot);
+            const uint32_t* chunk = ring + (c * kNbChunk % kRing) * kStride;
             if constexpr (kSkin)
             {
+                const uint16_t* dchunk = dring + (c * kNbChunk % kRing) * kStride;
                 uint4 d;
-                d.x = unsigned(dchunk[0]) | (unsigned(dchunk[kWarp]) << 16);
-                d.y = unsigned(dchunk[2 * kWarp]) | (unsigned(dchunk[3 * kWarp]) << 16);
-                d.z = unsigned(dchunk[4 * kWarp]) | (unsigned(dchunk[5 * kWarp]) << 16);
-                d.w = unsigned(dchunk[6 * kWarp]) | (unsigned(dchunk[7 * kWarp]) << 16);
-                *reinterpret_cast<uint4*>(ex.sl.dist + nidxAt(group, ngPad, c * kNbChunk, lane)) = d;
+                d.x = unsigned(dchunk[0]) | (unsigned(dchunk[kStride]) << 16);
+                d.y = unsigned(dchunk[2 * kStride]) | (unsigned(dchunk[3 * kStride]) << 16);
+                d.z = unsigned(dchunk[4 * kStride]) | (unsigned(dchunk[5 * kStride]) << 16);
+                d.w = unsigned(dchunk[6 * kStride]) | (unsigned(dchunk[7 * kStride]) << 16);
+                *reinterpret_cast<uint4*>(ex.sl.dist + nidxAt(group, ngPad, c * kNbChunk, slot)) = d;
             }
             // one 256-bit streaming store of the whole sector (the lists are next read once per J-loop)
             asm volatile("st.global.cs.v8.u32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(chunk[0]),
-                         "r"(chunk[kWarp]), "r"(chunk[2 * kWarp]), "r"(chunk[3 * kWarp]), "r"(chunk[4 * kWarp]),
-                         "r"(chunk[5 * kWarp]), "r"(chunk[6 * kWarp]), "r"(chunk[7 * kWarp])
+                         "r"(chunk[kStride]), "r"(chunk[2 * kStride]), "r"(chunk[3 * kStride]), "r"(chunk[4 * kStride]),
+                         "r"(chunk[5 * kStride]), "r"(chunk[6 * kStride]), "r"(chunk[7 * kStride])
                          : "memory");
         };
+        // neighbour k of the staged candidates as entry e of the list
+        auto put = [&](int k, int j, unsigned e) {
+            if constexpr (kSkin)
+            {
+                // the build distance, for the refilter's bounds
+                uint16_t q16;
+                if (exactDist)
+                {
+                    double4 pj = ldPos(pos + j);
+                    double q   = rint(sqrt(exactDistSq(pj.x, pj.y, pj.z, xi, yi, zi, box)) * qScale);
+                    q16        = uint16_t(fmin(q, kSkinDistUnits));
+                }
+                else
+                {
+                    float dx = sh.cx[warp][k] - rix, dy = sh.cy[warp][k] - riy, dz = sh.cz[warp][k] - riz;
+                    float q  = rintf(sqrtf(fmaf(dz, dz, fmaf(dy, dy, dx * dx))) * qScaleF);
+                    q16      = uint16_t(fminf(q, float(kSkinDistUnits)));
+                }
+                dring[(e % kRing) * kStride] = q16;
+            }
+            ring[(e % kRing) * kStride] = uint32_t(j);
+        };
 
-        // test the staged 32 candidates against this lane's particle and append the neighbours in index order
+        // test the staged 32 candidates (this lane's quarter of them where lanes share a target) against the target and
+        // append the neighbours in index order
+        constexpr int kShare = kWarp / kPer; // candidates per lane
         auto testStaged = [&](int numReal) {
             if (!active) { return; }
-            // bit k of sure: candidate k lies inside the sphere by its FP32 distance (below the band); of maybe: it
-            // may (below the upper edge of the band)
+            // bit k of sure: candidate first + k lies inside the sphere by its FP32 distance (below the band); of maybe:
+            // it may (below the upper edge of the band)
+            const int first = piece * kShare;
             unsigned maybe = 0u, sure = 0u;
             if (!wrapTest)
             {
                 const float2 mx = make_float2(-rix, -rix), my = make_float2(-riy, -riy), mz = make_float2(-riz, -riz);
 #pragma unroll
-                for (int k = 0; k < kWarp; k += 2)
+                for (int k = 0; k < kShare; k += 2)
                 {
-                    float2 X  = *reinterpret_cast<const float2*>(&sh.cx[warp][k]);
-                    float2 Y  = *reinterpret_cast<const float2*>(&sh.cy[warp][k]);
-                    float2 Z  = *reinterpret_cast<const float2*>(&sh.cz[warp][k]);
+                    float2 X  = *reinterpret_cast<const float2*>(&sh.cx[warp][first + k]);
+                    float2 Y  = *reinterpret_cast<const float2*>(&sh.cy[warp][first + k]);
+                    float2 Z  = *reinterpret_cast<const float2*>(&sh.cz[warp][first + k]);
                     float2 dx = __fadd2_rn(X, mx);
                     float2 dy = __fadd2_rn(Y, my);
                     float2 dz = __fadd2_rn(Z, mz);
@@ -291,7 +339,8 @@ __global__ void __launch_bounds__(kNbThreads, 8) findNeighborsKernel(const doubl
             {
                 // every real candidate of the chunk goes through the exact FP64 test below, which folds the pair
                 // difference itself (padding sits at the end of the last chunk)
-                maybe = numReal >= kWarp ? 0xffffffffu : ((1u << numReal) - 1u);
+                int real = min(max(numReal - first, 0), kShare);
+                maybe    = real >= 32 ? 0xffffffffu : ((1u << real) - 1u);
             }
             // candidates too close to the search radius for FP32: the exact test of the reference (rare)
             unsigned band = maybe & ~sure;
@@ -299,39 +348,61 @@ __global__ void __launch_bounds__(kNbThreads, 8) findNeighborsKernel(const doubl
             {
                 int k = __ffs(band) - 1;
                 band &= band - 1u;
-                int j      = sh.cj[warp][k];
+                int j      = sh.cj[warp][first + k];
                 double4 pj = ldPos(pos + j);
                 if (exactDistSq(pj.x, pj.y, pj.z, xi, yi, zi, box) < radiusSq) { sure |= 1u << k; }
             }
-            // append the neighbours in candidate (= index) order
-            while (sure)
+            if constexpr (kPer == 1)
             {
-                int k = __ffs(sure) - 1;
-                sure &= sure - 1u;
-                int j = sh.cj[warp][k];
-                if (size_t(j) == i) { continue; }
-                if (count < listCap)
+                // append the neighbours in candidate (= index) order
+                while (sure)
                 {
-                    if constexpr (kSkin)
+                    int k = __ffs(sure) - 1;
+                    sure &= sure - 1u;
+                    int j = sh.cj[warp][k];
+                    if (size_t(j) == i) { continue; }
+                    if (count < listCap)
                     {
-                        // the build distance, for the refilter's bounds
-                        if (exactDist)
-                        {
-                            double4 pj = ldPos(pos + j);
-                            double q   = rint(sqrt(exactDistSq(pj.x, pj.y, pj.z, xi, yi, zi, box)) * qScale);
-                            dchunk[(count % kNbChunk) * kWarp] = uint16_t(fmin(q, kSkinDistUnits));
-                        }
-                        else
-                        {
-                            float dx = sh.cx[warp][k] - rix, dy = sh.cy[warp][k] - riy, dz = sh.cz[warp][k] - riz;
-                            float q  = rintf(sqrtf(fmaf(dz, dz, fmaf(dy, dy, dx * dx))) * qScaleF);
-                            dchunk[(count % kNbChunk) * kWarp] = uint16_t(fminf(q, float(kSkinDistUnits)));
-                        }
+                        put(k, j, count);
+                        if (count % kNbChunk == kNbChunk - 1) { storeChunk(count / kNbChunk); }
                     }
-                    chunk[(count % kNbChunk) * kWarp] = uint32_t(j);
-                    if (count % kNbChunk == kNbChunk - 1) { storeChunk(count / kNbChunk); }
+                    ++count;
                 }
-                ++count;
+            }
+            else
+            {
+                // every lane of the target appends its own, after those of the lanes before it
+                const unsigned team = ((1u << kPer) - 1u) << (lane - piece);
+#pragma unroll
+                for (int k = 0; k < kShare; ++k)
+                {
+                    if (((sure >> k) & 1u) && size_t(sh.cj[warp][first + k]) == i) { sure &= ~(1u << k); }
+                }
+                unsigned hits = __popc(sure), before = 0u, all = hits;
+#pragma unroll
+                for (int off = 1; off < kPer; off <<= 1)
+                {
+                    unsigned o = __shfl_xor_sync(team, all, off);
+                    before += (piece & off) ? o : 0u;
+                    all += o;
+                }
+                unsigned e = count + before;
+                while (sure)
+                {
+                    int k = __ffs(sure) - 1;
+                    sure &= sure - 1u;
+                    if (e < listCap) { put(first + k, sh.cj[warp][first + k], e); }
+                    ++e;
+                }
+                __syncwarp(team);
+                // the chunks that filled up: at most five, and no entry past the list's capacity is stored
+                const unsigned now = min(count + all, listCap);
+                for (unsigned c = min(count, listCap) / kNbChunk + piece; c < now / kNbChunk; c += kPer)
+                {
+                    storeChunk(c);
+                }
+                __syncwarp(team);
+                count += all;
             }
         };
 
@@ -504,7 +575,7 @@ __global__ void __launch_bounds__(kNbThreads, 8) findNeighborsKernel(const doubl
         if (active)
         {
             unsigned kept = min(count, listCap);
-            if (kept % kNbChunk != 0) { storeChunk(kept / kNbChunk); }
+            if (kept % kNbChunk != 0 && piece == 0) { storeChunk(kept / kNbChunk); }
         }
 
         // smoothing-length iteration (skin rows: one pass at the given h)
@@ -527,7 +598,7 @@ __global__ void __launch_bounds__(kNbThreads, 8) findNeighborsKernel(const doubl
         if (lane == 0) { atomicOr(status, 1u); }
         return;
     }
-    if (valid)
+    if (valid && piece == 0)
     {
         if constexpr (kSkin)
         {
@@ -540,6 +611,19 @@ __global__ void __launch_bounds__(kNbThreads, 8) findNeighborsKernel(const doubl
             h[i]     = hi;
         }
     }
+    };
+    size_t unit = size_t(blockIdx.x) * kNbWarps + warp;
+    if constexpr (kKind == kSearchListed)
+    {
+        // as many blocks as stay resident walk the list, whose length only the device knows
+        const size_t units = size_t(*ex.numListed) * kPer;
+        for (; unit < units; unit += size_t(gridDim.x) * kNbWarps)
+        {
+            searchUnit(unit);
+            __syncwarp();
+        }
+    }
+    else { searchUnit(unit); }
 }
 
 //! bounding box of each run of kBlockSize consecutive particles, relative to the box corner, rounded outwards
@@ -578,6 +662,31 @@ int computeBlockBoxes(const double* x, const double* y, const double* z, size_t 
     return kOk;
 }
 
+namespace
+{
+unsigned searchBlocks(size_t n, int per)
+{
+    size_t units = (n + kWarp - 1) / kWarp * size_t(per);
+    return unsigned((units + kNbWarps - 1) / kNbWarps);
+}
+
+//! blocks of a listed search: at most those that stay resident
+unsigned listedBlocks(size_t n, int per) { return std::min(searchBlocks(n, per), unsigned(smCount()) * 8u); }
+
+//! KERNEL<batched, kind, lanes per target> with one tree or the members' trees
+#define SPHB_SEARCH(KIND, PER, BLOCKS, H, NIDX, NC)                                                                    \
+    if (views)                                                                                                          \
+    {                                                                                                                   \
+        findNeighborsKernel<true, KIND, PER><<<BLOCKS, kNbThreads, 0, stream>>>(x, y, z, pos, H, n, tree, box, prm,     \
+                                                                                NIDX, NC, status, views, inst, ex);     \
+    }                                                                                                                   \
+    else                                                                                                                \
+    {                                                                                                                   \
+        findNeighborsKernel<false, KIND, PER><<<BLOCKS, kNbThreads, 0, stream>>>(                                       \
+            x, y, z, pos, H, n, tree, box, prm, NIDX, NC, status, nullptr, nullptr, ex);                                \
+    }
+} // namespace
+
 int findNeighbors(const double* x, const double* y, const double* z, const double4* pos, double* h, size_t n,
                   const TreeView& tree, const DevBox& box, NeighborParams prm, uint32_t* nidx, unsigned* nc,
                   unsigned* status, cudaStream_t stream, const TreeView* views, const uint8_t* inst,
@@ -585,21 +694,11 @@ int findNeighbors(const double* x, const double* y, const double* z, const doubl
 {
     if (n == 0) { return kOk; }
     if ((views == nullptr) != (inst == nullptr)) { return kErrArg; }
-    size_t numGroups = (n + kWarp - 1) / kWarp;
-    unsigned blocks  = unsigned((numGroups + kNbWarps - 1) / kNbWarps);
     SearchExtras ex{};
     ex.gate     = gate;
     ex.gateMask = gateMask;
-    if (views)
-    {
-        findNeighborsKernel<true, kSearchAll><<<blocks, kNbThreads, 0, stream>>>(x, y, z, pos, h, n, tree, box, prm,
-                                                                                 nidx, nc, status, views, inst, ex);
-    }
-    else
-    {
-        findNeighborsKernel<false, kSearchAll><<<blocks, kNbThreads, 0, stream>>>(x, y, z, pos, h, n, tree, box, prm,
-                                                                                  nidx, nc, status, nullptr, nullptr, ex);
-    }
+    if (n <= kSharedLanesAll) { SPHB_SEARCH(kSearchAll, kSharedLanes, searchBlocks(n, kSharedLanes), h, nidx, nc) }
+    else { SPHB_SEARCH(kSearchAll, 1, searchBlocks(n, 1), h, nidx, nc) }
     countLaunch();
     SPHB_CUDA_TRY(cudaGetLastError());
     return kOk;
@@ -612,22 +711,14 @@ int findNeighborsListed(const double* x, const double* y, const double* z, const
 {
     if (n == 0) { return kOk; }
     if (!groups || !numListed || (views == nullptr) != (inst == nullptr)) { return kErrArg; }
-    size_t numGroups = (n + kWarp - 1) / kWarp;
-    unsigned blocks  = unsigned((numGroups + kNbWarps - 1) / kNbWarps);
     SearchExtras ex{};
     ex.groups    = groups;
     ex.numListed = numListed;
-    if (views)
+    if (n <= kSharedLanesListed)
     {
-        findNeighborsKernel<true, kSearchListed><<<blocks, kNbThreads, 0, stream>>>(x, y, z, pos, h, n, tree, box,
-                                                                                    prm, nidx, nc, status, views, inst,
-                                                                                    ex);
+        SPHB_SEARCH(kSearchListed, kSharedLanes, listedBlocks(n, kSharedLanes), h, nidx, nc)
     }
-    else
-    {
-        findNeighborsKernel<false, kSearchListed><<<blocks, kNbThreads, 0, stream>>>(
-            x, y, z, pos, h, n, tree, box, prm, nidx, nc, status, nullptr, nullptr, ex);
-    }
+    else { SPHB_SEARCH(kSearchListed, 1, listedBlocks(n, 1), h, nidx, nc) }
     countLaunch();
     SPHB_CUDA_TRY(cudaGetLastError());
     return kOk;
@@ -643,24 +734,15 @@ int buildSkinLists(const double* x, const double* y, const double* z, const doub
     {
         return kErrArg;
     }
-    size_t numGroups = (n + kWarp - 1) / kWarp;
-    unsigned blocks  = unsigned((numGroups + kNbWarps - 1) / kNbWarps);
     SearchExtras ex{};
     ex.sl          = sl;
     ex.onePlusSkin = 1.0 + skin;
     ex.gate        = gate;
     ex.gateMask    = gateMask;
     // the kernel writes h only in the iterating kinds, never in this one
-    if (views)
-    {
-        findNeighborsKernel<true, kSearchSkin><<<blocks, kNbThreads, 0, stream>>>(
-            x, y, z, pos, const_cast<double*>(h), n, tree, box, prm, nullptr, nullptr, status, views, inst, ex);
-    }
-    else
-    {
-        findNeighborsKernel<false, kSearchSkin><<<blocks, kNbThreads, 0, stream>>>(
-            x, y, z, pos, const_cast<double*>(h), n, tree, box, prm, nullptr, nullptr, status, nullptr, nullptr, ex);
-    }
+    double* hRead = const_cast<double*>(h);
+    if (n <= kSharedLanesAll) { SPHB_SEARCH(kSearchSkin, kSharedLanes, searchBlocks(n, kSharedLanes), hRead, nullptr, nullptr) }
+    else { SPHB_SEARCH(kSearchSkin, 1, searchBlocks(n, 1), hRead, nullptr, nullptr) }
     countLaunch();
     SPHB_CUDA_TRY(cudaGetLastError());
     return kOk;
