@@ -26,7 +26,8 @@ namespace
 
 constexpr int kNbWarps   = 4;
 constexpr int kNbThreads = kNbWarps * kWarp;
-constexpr int kStackCap  = 176; // depth-first stack: <= 7 pending siblings per level + 8
+constexpr int kStackWide = 80;  // entries up to which the traversal takes four of them at a time
+constexpr int kStackCap  = 256; // kStackWide + 28, and 7 per level for those taken one at a time
 constexpr int kLeafCap   = 256; // candidate leaves buffered before they are streamed
 
 /*! Lanes that share a target. One lane per target tests and appends for its own particle, 32 targets per warp. A group's
@@ -34,9 +35,9 @@ constexpr int kLeafCap   = 256; // candidate leaves buffered before they are str
  *  most of the GPU idle. With four lanes per target a warp serves eight targets: each lane tests and appends a quarter of
  *  the staged candidates, and the smaller search box admits about half of them. But each box is traversed and staged by
  *  itself, so a launch that fills the GPU is slower with it: hence the limits below.
- *  Whole searches, us for one and for four lanes: 16^3 particles 117 and 75, 30^3 167 and 122, 36^3 203 and 144; 50^3 327
- *  and 426, 63^3 394 and 579, 81^3 702 and 939. Searches of listed groups, a small part of all: block time steps of 64^3
- *  509 and 452; 128^3 1569 and 1690 (with the rest of the phase). */
+ *  Neighbour phase before the traversal took four nodes a round, us for one and for four lanes: 16^3 particles 117 and 75,
+ *  30^3 167 and 122, 36^3 203 and 144; 50^3 327 and 426, 63^3 394 and 579, 81^3 702 and 939. Searches of listed groups,
+ *  a small part of all: block time steps of 64^3 509 and 452; 128^3 1569 and 1690. */
 constexpr int kSharedLanes          = 4;
 constexpr size_t kSharedLanesAll    = 40000;
 constexpr size_t kSharedLanesListed = 300000;
@@ -47,7 +48,7 @@ struct NbShared
     //! list entries a target buffers: the chunk being filled; where lanes share it, up to 32 more neighbours at a time
     static constexpr int kRing = kPer == 1 ? kNbChunk : 5 * kNbChunk;
     int stack[kNbWarps][kStackCap];
-    int leafFirst[kNbWarps][kLeafCap]; // first particle of each buffered leaf
+    int leafFirst[kNbWarps][kLeafCap]; // the buffered leaves, then the first particle of each
     int leafEnd[kNbWarps][kLeafCap];   // one past its last particle
     int blkPre[kNbWarps][kLeafCap + 1]; // exclusive prefix of the number of blocks per buffered leaf
     int pStart[kNbWarps][kWarp];       // surviving pieces (block and leaf intersections) of one round
@@ -417,7 +418,11 @@ __global__ void __launch_bounds__(kNbThreads, 8) findNeighborsKernel(const doubl
                 int nbk = 0;
                 if (t < numLeaves)
                 {
-                    int b = leafFirst[t], e = leafEnd[t];
+                    int leaf = leafFirst[t];
+                    int b    = tv.layout[leaf];
+                    int e    = tv.layout[leaf + 1];
+                    leafFirst[t] = b;
+                    leafEnd[t]   = e;
                     nbk   = e > b ? (e - 1) / kBlockSize - b / kBlockSize + 1 : 0;
                 }
                 local[q] = nbk;
@@ -516,56 +521,57 @@ __global__ void __launch_bounds__(kNbThreads, 8) findNeighborsKernel(const doubl
             numLeaves = 0;
         };
 
-        // depth-first traversal in SFC order
-        int sp = 0;
-        if (lane == 0) { stack[0] = 0; }
-        sp = 1;
+        // Depth-first traversal in SFC order, the lowest key on top of the stack: an entry is the first child of an internal
+        // node or the complement of a leaf. Every round takes the top four entries, tests the children of the internal ones,
+        // one per lane, and buffers the leaves that come before the first internal node; the rest goes back in order. A node a
+        // round, tested by eight lanes and its leaves looked up by one, took the search of 81^3 Noh particles from 525 to 716 us.
+        const int rootChild = tv.childOffsets[0];
+        int sp              = 1;
+        if (lane == 0) { stack[0] = rootChild ? rootChild : ~tv.nodeToLeaf[0]; }
         __syncwarp();
         while (sp > 0)
         {
-            int node = stack[sp - 1];
-            --sp;
-            int child0 = tv.childOffsets[node];
-            if (child0 == 0)
+            const int take = sp > kStackWide ? 1 : min(sp, kWarp / 8);
+            int entry      = 0;
+            bool ov        = false;
+            if (lane / 8 < take)
             {
-                if (numLeaves == kLeafCap) { flush(); }
-                if (lane == 0)
+                entry = stack[sp - 1 - lane / 8];
+                ov    = lane % 8 == 0;
+                if (entry > 0)
                 {
-                    int leaf             = tv.nodeToLeaf[node];
-                    leafFirst[numLeaves] = tv.layout[leaf];
-                    leafEnd[numLeaves]   = tv.layout[leaf + 1];
-                }
-                ++numLeaves;
-                __syncwarp();
-                continue;
-            }
-            bool ov = false;
-            if (lane < 8)
-            {
-                int c = child0 + lane;
-                ov    = true;
+                    int c     = entry + lane % 8;
+                    int child = tv.childOffsets[c];
+                    int leaf  = tv.nodeToLeaf[c];
+                    ov        = true;
 #pragma unroll
-                for (int k = 0; k < 3; ++k)
-                {
-                    double d = tv.centers[3 * c + k] - gc[k];
-                    if (box.periodic[k]) { d -= box.len[k] * rint(d * box.ilen[k]); }
-                    ov = ov && fabs(d) <= gs[k] + tv.sizes[3 * c + k] * (1.0 + 1e-12) + tv.ext;
+                    for (int k = 0; k < 3; ++k)
+                    {
+                        double d = tv.centers[3 * c + k] - gc[k];
+                        if (box.periodic[k]) { d -= box.len[k] * rint(d * box.ilen[k]); }
+                        ov = ov && fabs(d) <= gs[k] + tv.sizes[3 * c + k] * (1.0 + 1e-12) + tv.ext;
+                    }
+                    entry = child ? child : ~leaf;
                 }
             }
-            unsigned m = __ballot_sync(0xffffffffu, ov) & 0xffu;
-            int pushes = __popc(m);
+            __syncwarp();
+            sp -= take;
+            unsigned found    = __ballot_sync(0xffffffffu, ov);
+            unsigned internal = __ballot_sync(0xffffffffu, ov && entry > 0);
+            unsigned ready    = internal ? found & ((internal & (0u - internal)) - 1u) : found;
+            int numReady      = __popc(ready);
+            if (numLeaves + numReady > kLeafCap) { flush(); }
+            if ((ready >> lane) & 1u) { leafFirst[numLeaves + __popc(ready & ((1u << lane) - 1u))] = ~entry; }
+            numLeaves += numReady;
+            unsigned later = found & ~ready;
+            int pushes     = __popc(later);
             if (sp + pushes > kStackCap)
             {
                 overflow = true;
                 break;
             }
-            __syncwarp();
-            if (ov)
-            {
-                // children are pushed in reverse so that the lowest key is popped first
-                int pos         = __popc(m >> (lane + 1));
-                stack[sp + pos] = child0 + lane;
-            }
+            // in reverse, so that the lowest key is on top
+            if ((later >> lane) & 1u) { stack[sp + __popc(later >> lane >> 1)] = entry; }
             sp += pushes;
             __syncwarp();
         }
