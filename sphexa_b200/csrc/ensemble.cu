@@ -514,8 +514,7 @@ int rebuildTrees(sphb_ensemble& e)
             f.firstCall = false;
         }
         SPHB_TRY(focusUpdateTree(f, g, e.ts, st, &converged));
-        SPHB_TRY(focusUpdateCounts(f, keys, nk, st));
-        SPHB_TRY(computeGeoCenters(f.tree, e.box, st));
+        SPHB_TRY(focusUpdateCounts(f, keys, nk, st, &e.box));
         SPHB_TRY(e.layouts[k]->reserve(size_t(f.numLeaves) + 1));
         TreeView tv;
         tv.childOffsets = f.tree.childOffsets.data();

@@ -222,6 +222,44 @@ __global__ void linkKernel(const uint64_t* prefixes, const int* nodeToLeaf, int 
 
 constexpr int kCountThreads = 256;
 
+/*! Trees of at most this many leaves are updated by single blocks that do several of the steps below one after another: a
+ *  step over a few thousand nodes takes about 3 us, most of it launch, and eleven launches become three. Sync of 16^3
+ *  particles 157 -> 127 us, of 30^3 164 -> 137 us. Beyond 2,048 leaves a phase is several rounds of one SM. */
+constexpr int kSmallTree    = 2048;
+constexpr int kSmallThreads = 1024;
+
+/*! data[0 .. n) -> its exclusive scan, in place, and the sum to data[n], by one block of kSmallThreads */
+__device__ void blockScanInPlace(int* data, int n)
+{
+    __shared__ int warpSum[kSmallThreads / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int carry = 0;
+    for (int base = 0; base < n; base += kSmallThreads)
+    {
+        int i    = base + threadIdx.x;
+        int v    = i < n ? data[i] : 0;
+        int incl = v;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1)
+        {
+            int t = __shfl_up_sync(0xffffffffu, incl, off);
+            if (lane >= off) { incl += t; }
+        }
+        if (lane == 31) { warpSum[warp] = incl; }
+        __syncthreads();
+        int before = 0, all = 0;
+        for (int w = 0; w < kSmallThreads / 32; ++w)
+        {
+            before += w < warp ? warpSum[w] : 0;
+            all += warpSum[w];
+        }
+        if (i < n) { data[i] = carry + before + incl - v; }
+        carry += all;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) { data[n] = carry; }
+}
+
 /*! counts[i] = keys in [leaves[i], leaves[i + 1]), the layout first[i] = keys below leaves[i] (i <= numLeaves; the
  *  exclusive scan of the counts, since the leaves start at key 0), and the largest count into *maxCount; first and
  *  maxCount may be null. One binary search per boundary: a leaf takes its end from the next thread. */
@@ -251,12 +289,11 @@ __global__ void __launch_bounds__(kCountThreads) leafCountsKernel(const uint64_t
     }
 }
 
-//! counts of every node: a leaf's own, or the layout at the ends of the leaves an internal node covers
-__global__ void nodeCountsKernel(const uint64_t* prefixes, const int* nodeToLeaf, int numNodes, const uint64_t* leaves,
-                                 int numLeaves, const unsigned* leafCounts, const int* layout, unsigned* nodeCounts)
+//! count of node p: a leaf's own, or the layout at the ends of the leaves an internal node covers
+__device__ __forceinline__ void nodeCountOf(int p, const uint64_t* prefixes, const int* nodeToLeaf,
+                                            const uint64_t* leaves, int numLeaves, const unsigned* leafCounts,
+                                            const int* layout, unsigned* nodeCounts)
 {
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= numNodes) { return; }
     int leaf = nodeToLeaf[p];
     if (leaf >= 0)
     {
@@ -272,10 +309,15 @@ __global__ void nodeCountsKernel(const uint64_t* prefixes, const int* nodeToLeaf
     nodeCounts[p]   = unsigned(layout[e] - layout[b]);
 }
 
-__global__ void geoKernel(const uint64_t* prefixes, int numNodes, DevBox box, double* centers, double* sizes)
+__global__ void nodeCountsKernel(const uint64_t* prefixes, const int* nodeToLeaf, int numNodes, const uint64_t* leaves,
+                                 int numLeaves, const unsigned* leafCounts, const int* layout, unsigned* nodeCounts)
 {
     int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= numNodes) { return; }
+    if (p < numNodes) { nodeCountOf(p, prefixes, nodeToLeaf, leaves, numLeaves, leafCounts, layout, nodeCounts); }
+}
+
+__device__ __forceinline__ void geoOf(int p, const uint64_t* prefixes, const DevBox& box, double* centers, double* sizes)
+{
     uint64_t prefix = prefixes[p];
     unsigned level  = prefixLevel(prefix);
     unsigned ixyz[3];
@@ -292,15 +334,61 @@ __global__ void geoKernel(const uint64_t* prefixes, int numNodes, DevBox box, do
     }
 }
 
+__global__ void geoKernel(const uint64_t* prefixes, int numNodes, DevBox box, double* centers, double* sizes)
+{
+    int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p < numNodes) { geoOf(p, prefixes, box, centers, sizes); }
+}
+
+/*! the number of keys below every leaf boundary into bound (shared, kSmallTree + 1 entries), and the leaves' counts, by one
+ *  block; returns this thread's largest count */
+__device__ unsigned blockLeafCounts(const uint64_t* leaves, int numLeaves, const uint64_t* keys, size_t n,
+                                    unsigned* counts, unsigned* bound)
+{
+    for (int i = threadIdx.x; i <= numLeaves; i += kSmallThreads)
+    {
+        bound[i] = unsigned(lowerBound(keys, n, leaves[i]));
+    }
+    __syncthreads();
+    unsigned largest = 0;
+    for (int i = threadIdx.x; i < numLeaves; i += kSmallThreads)
+    {
+        unsigned c = bound[i + 1] - bound[i];
+        counts[i]  = c;
+        largest    = max(largest, c);
+    }
+    return largest;
+}
+
+//! leaf counts, layout, node counts and, if centers is set, the node geometry of a small tree
+__global__ void __launch_bounds__(kSmallThreads) smallCountsKernel(const uint64_t* leaves, int numLeaves,
+                                                                  const uint64_t* keys, size_t n, unsigned* counts,
+                                                                  int* layout, const uint64_t* prefixes,
+                                                                  const int* nodeToLeaf, int numNodes,
+                                                                  unsigned* nodeCounts, DevBox box, double* centers,
+                                                                  double* sizes)
+{
+    __shared__ unsigned bound[kSmallTree + 1];
+    blockLeafCounts(leaves, numLeaves, keys, n, counts, bound);
+    for (int i = threadIdx.x; i <= numLeaves; i += kSmallThreads)
+    {
+        layout[i] = int(bound[i]);
+    }
+    __syncthreads();
+    for (int p = threadIdx.x; p < numNodes; p += kSmallThreads)
+    {
+        nodeCountOf(p, prefixes, nodeToLeaf, leaves, numLeaves, counts, layout, nodeCounts);
+        if (centers) { geoOf(p, prefixes, box, centers, sizes); }
+    }
+}
+
 // ---------------------------------------------------------------------------------------------------------------
 // global tree: csarray rebalance (cstone/tree/csarray.hpp:248-389)
 // ---------------------------------------------------------------------------------------------------------------
 
-__global__ void csNodeOpsKernel(const uint64_t* leaves, const unsigned* counts, int numLeaves, unsigned bucket,
-                                int* ops, unsigned* flags)
+__device__ __forceinline__ void csNodeOp(int i, const uint64_t* leaves, const unsigned* counts, int numLeaves,
+                                         unsigned bucket, int* ops, unsigned* flags)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > numLeaves) { return; }
     if (i == numLeaves)
     {
         ops[i] = 0;
@@ -340,6 +428,31 @@ __global__ void csNodeOpsKernel(const uint64_t* leaves, const unsigned* counts, 
     }
     ops[i] = op;
     if (op != 1) { atomicOr(flags, 1u); }
+}
+
+__global__ void csNodeOpsKernel(const uint64_t* leaves, const unsigned* counts, int numLeaves, unsigned bucket,
+                                int* ops, unsigned* flags)
+{
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i <= numLeaves) { csNodeOp(i, leaves, counts, numLeaves, bucket, ops, flags); }
+}
+
+//! globalTreeStep's ops, their scan and the counts of the current leaves for a small tree; flags cleared before
+__global__ void __launch_bounds__(kSmallThreads) smallGlobalStepKernel(const uint64_t* leaves, unsigned* counts,
+                                                                      int numLeaves, unsigned bucket, int* ops,
+                                                                      unsigned* flags, const uint64_t* keys, size_t n)
+{
+    __shared__ unsigned bound[kSmallTree + 1];
+    if (threadIdx.x < 4) { flags[threadIdx.x] = 0; }
+    __syncthreads();
+    for (int i = threadIdx.x; i <= numLeaves; i += kSmallThreads)
+    {
+        csNodeOp(i, leaves, counts, numLeaves, bucket, ops, flags);
+    }
+    __syncthreads();
+    blockScanInPlace(ops, numLeaves + 1);
+    unsigned largest = blockLeafCounts(leaves, numLeaves, keys, n, counts, bound);
+    if (largest) { atomicMax(flags + 1, largest); }
 }
 
 //! new leaves from scanned ops (processNode, cstone/tree/csarray.hpp:340-366)
@@ -382,11 +495,9 @@ enum Resolution : unsigned
 
 /*! mergeCountAndMacOp (rebalance.hpp:31-75) with the whole key range in focus: every node is inside the focus and
  *  every sibling group is in the fringe, so the MAC never decides and only particle counts do. */
-__global__ void focusOpsKernel(const uint64_t* prefixes, const int* childOffsets, const int* parents,
-                               const unsigned* counts, int numNodes, unsigned bucket, int* ops)
+__device__ __forceinline__ void focusOp(int p, const uint64_t* prefixes, const int* childOffsets, const int* parents,
+                                        const unsigned* counts, unsigned bucket, int* ops)
 {
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= numNodes) { return; }
     if (p > 0)
     {
         int parent = parents[(p - 1) / 8];
@@ -409,6 +520,13 @@ __global__ void focusOpsKernel(const uint64_t* prefixes, const int* childOffsets
     ops[p] = op;
 }
 
+__global__ void focusOpsKernel(const uint64_t* prefixes, const int* childOffsets, const int* parents,
+                               const unsigned* counts, int numNodes, unsigned bucket, int* ops)
+{
+    int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p < numNodes) { focusOp(p, prefixes, childOffsets, parents, counts, bucket, ops); }
+}
+
 //! smallest existing node containing the node with placeholder-bit key `want` (octree.hpp:199-216)
 __device__ int containingNodeOf(uint64_t want, const uint64_t* prefixes, const int* childOffsets)
 {
@@ -425,12 +543,9 @@ __device__ int containingNodeOf(uint64_t want, const uint64_t* prefixes, const i
 
 /*! enforceKeySingle (rebalance.hpp:161-212) for every mandatory key in parallel. Sibling resets only ever turn 0
  *  into 1 and splits take the maximum, so the final ops and the maximum status do not depend on key order. */
-__global__ void enforceKeysKernel(const uint64_t* keys, int numKeys, const uint64_t* prefixes, const int* childOffsets,
-                                  const int* parents, int* ops, unsigned* status)
+__device__ __forceinline__ void enforceKey(uint64_t key, const uint64_t* prefixes, const int* childOffsets,
+                                           const int* parents, int* ops, unsigned* status)
 {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= numKeys) { return; }
-    uint64_t key = keys[t];
     if (key == 0 || key == kRootRange) { return; }
 
     unsigned lastNz    = kMaxLevel - unsigned(__ffsll((long long)key) - 1) / 3u;
@@ -465,12 +580,17 @@ __global__ void enforceKeysKernel(const uint64_t* keys, int numKeys, const uint6
     if (st != kConverged) { atomicMax(status, st); }
 }
 
-//! nzAncestorOp (rebalance.hpp:96-116): merged nodes are kept only as the left-most descendant of a kept ancestor
-__global__ void protectKernel(const uint64_t* prefixes, const int* parents, const int* opsIn, int numNodes,
-                              int* opsOut, unsigned* numChanges)
+__global__ void enforceKeysKernel(const uint64_t* keys, int numKeys, const uint64_t* prefixes, const int* childOffsets,
+                                  const int* parents, int* ops, unsigned* status)
 {
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= numNodes) { return; }
+    int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < numKeys) { enforceKey(keys[t], prefixes, childOffsets, parents, ops, status); }
+}
+
+//! nzAncestorOp (rebalance.hpp:96-116): merged nodes are kept only as the left-most descendant of a kept ancestor
+__device__ __forceinline__ void protectOp(int p, const uint64_t* prefixes, const int* parents, const int* opsIn,
+                                          int* opsOut, unsigned* numChanges)
+{
     int res;
     if (p == 0) { res = opsIn[0]; }
     else
@@ -486,11 +606,16 @@ __global__ void protectKernel(const uint64_t* prefixes, const int* parents, cons
     if (res != 1) { atomicAdd(numChanges, 1u); }
 }
 
-__global__ void leafOpsKernel(const int* nodeOps, const int* leafToNode, int numLeaves, int* leafOps,
-                              unsigned* numNotOne)
+__global__ void protectKernel(const uint64_t* prefixes, const int* parents, const int* opsIn, int numNodes,
+                              int* opsOut, unsigned* numChanges)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > numLeaves) { return; }
+    int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p < numNodes) { protectOp(p, prefixes, parents, opsIn, opsOut, numChanges); }
+}
+
+__device__ __forceinline__ void leafOp(int i, const int* nodeOps, const int* leafToNode, int numLeaves, int* leafOps,
+                                       unsigned* numNotOne)
+{
     if (i == numLeaves)
     {
         leafOps[i] = 0;
@@ -499,6 +624,45 @@ __global__ void leafOpsKernel(const int* nodeOps, const int* leafToNode, int num
     int op     = nodeOps[leafToNode[i]];
     leafOps[i] = op;
     if (op != 1) { atomicAdd(numNotOne, 1u); }
+}
+
+__global__ void leafOpsKernel(const int* nodeOps, const int* leafToNode, int numLeaves, int* leafOps,
+                              unsigned* numNotOne)
+{
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i <= numLeaves) { leafOp(i, nodeOps, leafToNode, numLeaves, leafOps, numNotOne); }
+}
+
+//! focusUpdateTree's ops of nodes and leaves and their scan for a small tree; flags cleared before
+__global__ void __launch_bounds__(kSmallThreads) smallFocusOpsKernel(const uint64_t* prefixes, const int* childOffsets,
+                                                                    const int* parents, const unsigned* counts,
+                                                                    int numNodes, unsigned bucket,
+                                                                    const uint64_t* keys, int numKeys,
+                                                                    const int* leafToNode, int numLeaves, int* ops,
+                                                                    int* opsOut, unsigned* flags)
+{
+    if (threadIdx.x < 4) { flags[threadIdx.x] = 0; }
+    for (int p = threadIdx.x; p < numNodes; p += kSmallThreads)
+    {
+        focusOp(p, prefixes, childOffsets, parents, counts, bucket, ops);
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < numKeys; t += kSmallThreads)
+    {
+        enforceKey(keys[t], prefixes, childOffsets, parents, ops, flags);
+    }
+    __syncthreads();
+    for (int p = threadIdx.x; p < numNodes; p += kSmallThreads)
+    {
+        protectOp(p, prefixes, parents, ops, opsOut, flags + 1);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i <= numLeaves; i += kSmallThreads)
+    {
+        leafOp(i, opsOut, leafToNode, numLeaves, ops, flags + 2);
+    }
+    __syncthreads();
+    blockScanInPlace(ops, numLeaves + 1);
 }
 
 __global__ void setLeavesKernel(uint64_t* leaves, unsigned* counts, unsigned initialCount)
@@ -598,7 +762,6 @@ int initGlobalTree(GlobalTree& g, unsigned bucket, cudaStream_t stream)
     g.bucket    = bucket;
     g.numLeaves = 1;
     g.firstCall = true;
-    g.hostStale = true;
     SPHB_TRY(g.leaves.reserve(2));
     SPHB_TRY(g.counts.reserve(1));
     setLeavesKernel<<<1, 1, 0, stream>>>(g.leaves.data(), g.counts.data(), bucket - 1);
@@ -614,14 +777,24 @@ int globalTreeStep(GlobalTree& g, const uint64_t* keys, size_t n, TreeScratch& s
     SPHB_TRY(s.ints.reserve(L + 2));
     SPHB_TRY(s.scanTmp.reserve(scanTempInts(L + 1) + 1));
     SPHB_TRY(s.flags.reserve(4));
-    SPHB_CUDA_TRY(cudaMemsetAsync(s.flags.data(), 0, 4 * sizeof(unsigned), stream));
-    csNodeOpsKernel<<<ceilDiv(L + 1, 256), 256, 0, stream>>>(g.leaves.data(), g.counts.data(), L, g.bucket,
-                                                             s.ints.data(), s.flags.data());
-    countLaunch();
-    SPHB_TRY(exclusiveScan(s.ints.data(), s.ints.data(), L + 1, s.scanTmp.data(), stream));
-    // the counts of the current leaves, before knowing whether they change: in the steady state nothing splits or
+    // with the counts of the current leaves, before knowing whether they change: in the steady state nothing splits or
     // merges and one read back serves both decisions
-    SPHB_TRY(computeLeafCounts(g.leaves.data(), L, keys, n, g.counts.data(), stream, nullptr, s.flags.data() + 1));
+    if (L <= kSmallTree && n <= UINT32_MAX)
+    {
+        smallGlobalStepKernel<<<1, kSmallThreads, 0, stream>>>(g.leaves.data(), g.counts.data(), L, g.bucket,
+                                                               s.ints.data(), s.flags.data(), keys, n);
+        countLaunch();
+        SPHB_CUDA_TRY(cudaGetLastError());
+    }
+    else
+    {
+        SPHB_CUDA_TRY(cudaMemsetAsync(s.flags.data(), 0, 4 * sizeof(unsigned), stream));
+        csNodeOpsKernel<<<ceilDiv(L + 1, 256), 256, 0, stream>>>(g.leaves.data(), g.counts.data(), L, g.bucket,
+                                                                 s.ints.data(), s.flags.data());
+        countLaunch();
+        SPHB_TRY(exclusiveScan(s.ints.data(), s.ints.data(), L + 1, s.scanTmp.data(), stream));
+        SPHB_TRY(computeLeafCounts(g.leaves.data(), L, keys, n, g.counts.data(), stream, nullptr, s.flags.data() + 1));
+    }
     unsigned msg[3]; // new leaf count, any op, largest count
     SPHB_TRY(readBack(stream, {{msg, s.ints.data() + L, sizeof(int)}, {msg + 1, s.flags.data(), 2 * sizeof(unsigned)}}));
     int newL       = int(msg[0]);
@@ -636,7 +809,6 @@ int globalTreeStep(GlobalTree& g, const uint64_t* keys, size_t n, TreeScratch& s
         SPHB_CUDA_TRY(cudaGetLastError());
         g.leaves.swap(g.leavesAlt);
         g.numLeaves = newL;
-        g.hostStale = true;
         SPHB_TRY(g.counts.reserve(newL));
         SPHB_CUDA_TRY(cudaMemsetAsync(s.flags.data() + 1, 0, sizeof(unsigned), stream));
         SPHB_TRY(computeLeafCounts(g.leaves.data(), newL, keys, n, g.counts.data(), stream, nullptr,
@@ -649,7 +821,6 @@ int globalTreeStep(GlobalTree& g, const uint64_t* keys, size_t n, TreeScratch& s
 
 int updateGlobalTree(GlobalTree& g, const uint64_t* keys, size_t n, TreeScratch& s, cudaStream_t stream)
 {
-    if (g.hostLeaves.empty()) { g.hostStale = true; }
     unsigned maxCount = 0;
     SPHB_TRY(globalTreeStep(g, keys, n, s, stream, &maxCount));
     if (g.firstCall || maxCount >= 8 * g.bucket)
@@ -661,15 +832,6 @@ int updateGlobalTree(GlobalTree& g, const uint64_t* keys, size_t n, TreeScratch&
             SPHB_TRY(globalTreeStep(g, keys, n, s, stream, &maxCount));
             if (++guard > 64) { return kErrNotConverged; }
         } while (maxCount > g.bucket);
-    }
-    if (g.hostStale)
-    {
-        // the host copy of the leaves (mandatory keys of a failed focus update) follows only changes
-        g.hostLeaves.resize(g.numLeaves + 1);
-        SPHB_CUDA_TRY(cudaMemcpyAsync(g.hostLeaves.data(), g.leaves.data(), (g.numLeaves + 1) * sizeof(uint64_t),
-                                      cudaMemcpyDeviceToHost, stream));
-        SPHB_CUDA_TRY(cudaStreamSynchronize(stream));
-        g.hostStale = false;
     }
     return kOk;
 }
@@ -706,22 +868,32 @@ int focusUpdateTree(FocusTree& f, const GlobalTree& g, TreeScratch& s, cudaStrea
     SPHB_TRY(s.flags.reserve(4));
     int* ops    = s.ints.data();
     int* opsOut = s.ints2.data();
-    SPHB_CUDA_TRY(cudaMemsetAsync(s.flags.data(), 0, 4 * sizeof(unsigned), stream));
-
-    focusOpsKernel<<<ceilDiv(nn, 256), 256, 0, stream>>>(t.prefixes.data(), t.childOffsets.data(), t.parents.data(),
-                                                         t.nodeCounts.data(), nn, f.bucket, ops);
-    // mandatory keys: the global leaves (the focus start 0 and end 2^63 are always converged)
-    enforceKeysKernel<<<ceilDiv(g.numLeaves + 1, 128), 128, 0, stream>>>(
-        g.leaves.data(), g.numLeaves + 1, t.prefixes.data(), t.childOffsets.data(), t.parents.data(), ops,
-        s.flags.data());
-    protectKernel<<<ceilDiv(nn, 256), 256, 0, stream>>>(t.prefixes.data(), t.parents.data(), ops, nn, opsOut,
-                                                        s.flags.data() + 1);
     int* leafOps = ops; // node ops no longer needed
-    leafOpsKernel<<<ceilDiv(L + 1, 256), 256, 0, stream>>>(opsOut, t.leafToNode.data(), L, leafOps,
-                                                           s.flags.data() + 2);
-    countLaunch(4);
-    SPHB_CUDA_TRY(cudaGetLastError());
-    SPHB_TRY(exclusiveScan(leafOps, leafOps, L + 1, s.scanTmp.data(), stream));
+    // mandatory keys: the global leaves (the focus start 0 and end 2^63 are always converged)
+    if (L <= kSmallTree && g.numLeaves <= kSmallTree)
+    {
+        smallFocusOpsKernel<<<1, kSmallThreads, 0, stream>>>(
+            t.prefixes.data(), t.childOffsets.data(), t.parents.data(), t.nodeCounts.data(), nn, f.bucket,
+            g.leaves.data(), g.numLeaves + 1, t.leafToNode.data(), L, ops, opsOut, s.flags.data());
+        countLaunch();
+        SPHB_CUDA_TRY(cudaGetLastError());
+    }
+    else
+    {
+        SPHB_CUDA_TRY(cudaMemsetAsync(s.flags.data(), 0, 4 * sizeof(unsigned), stream));
+        focusOpsKernel<<<ceilDiv(nn, 256), 256, 0, stream>>>(t.prefixes.data(), t.childOffsets.data(),
+                                                             t.parents.data(), t.nodeCounts.data(), nn, f.bucket, ops);
+        enforceKeysKernel<<<ceilDiv(g.numLeaves + 1, 128), 128, 0, stream>>>(
+            g.leaves.data(), g.numLeaves + 1, t.prefixes.data(), t.childOffsets.data(), t.parents.data(), ops,
+            s.flags.data());
+        protectKernel<<<ceilDiv(nn, 256), 256, 0, stream>>>(t.prefixes.data(), t.parents.data(), ops, nn, opsOut,
+                                                            s.flags.data() + 1);
+        leafOpsKernel<<<ceilDiv(L + 1, 256), 256, 0, stream>>>(opsOut, t.leafToNode.data(), L, leafOps,
+                                                               s.flags.data() + 2);
+        countLaunch(4);
+        SPHB_CUDA_TRY(cudaGetLastError());
+        SPHB_TRY(exclusiveScan(leafOps, leafOps, L + 1, s.scanTmp.data(), stream));
+    }
     int newL = 0;
     unsigned flags[3];
     SPHB_TRY(readBack(stream, {{&newL, leafOps + L, sizeof(int)}, {flags, s.flags.data(), sizeof(flags)}}));
@@ -748,10 +920,12 @@ int focusUpdateTree(FocusTree& f, const GlobalTree& g, TreeScratch& s, cudaStrea
         // injectKeys (cstone/focus/inject.hpp): merge the spanning tree of the mandatory keys into the leaves
         conv = false;
         std::vector<uint64_t> leaves(newL + 1);
+        std::vector<uint64_t> mand(g.numLeaves + 1);
         SPHB_CUDA_TRY(cudaMemcpyAsync(leaves.data(), f.leaves.data(), (newL + 1) * sizeof(uint64_t),
                                       cudaMemcpyDeviceToHost, stream));
+        SPHB_CUDA_TRY(cudaMemcpyAsync(mand.data(), g.leaves.data(), (g.numLeaves + 1) * sizeof(uint64_t),
+                                      cudaMemcpyDeviceToHost, stream));
         SPHB_CUDA_TRY(cudaStreamSynchronize(stream));
-        std::vector<uint64_t> mand(g.hostLeaves.begin(), g.hostLeaves.end());
         mand.push_back(0);
         mand.push_back(kRootRange);
         std::sort(mand.begin(), mand.end());
@@ -777,14 +951,25 @@ int focusUpdateTree(FocusTree& f, const GlobalTree& g, TreeScratch& s, cudaStrea
     return kOk;
 }
 
-int focusUpdateCounts(FocusTree& f, const uint64_t* keys, size_t n, cudaStream_t stream)
+int focusUpdateCounts(FocusTree& f, const uint64_t* keys, size_t n, cudaStream_t stream, const DevBox* box)
 {
     int L = f.numLeaves;
     SPHB_TRY(f.leafCounts.reserve(L));
     SPHB_TRY(f.layout.reserve(L + 1));
+    if (L <= kSmallTree && n <= UINT32_MAX)
+    {
+        LinkedOctree& t = f.tree;
+        smallCountsKernel<<<1, kSmallThreads, 0, stream>>>(
+            f.leaves.data(), L, keys, n, f.leafCounts.data(), f.layout.data(), t.prefixes.data(), t.nodeToLeaf.data(),
+            t.numNodes, t.nodeCounts.data(), box ? *box : DevBox{}, box ? t.centers.data() : nullptr,
+            box ? t.sizes.data() : nullptr);
+        countLaunch();
+        SPHB_CUDA_TRY(cudaGetLastError());
+        return kOk;
+    }
     SPHB_TRY(computeLeafCounts(f.leaves.data(), L, keys, n, f.leafCounts.data(), stream, f.layout.data()));
     SPHB_TRY(computeNodeCounts(f.leaves.data(), f.leafCounts.data(), f.layout.data(), f.tree, stream));
-    return kOk;
+    return box ? computeGeoCenters(f.tree, *box, stream) : int(kOk);
 }
 
 } // namespace sphb

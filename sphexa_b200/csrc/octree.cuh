@@ -62,8 +62,6 @@ struct GlobalTree
     int numLeaves{0};
     unsigned bucket{0};
     bool firstCall{true};
-    std::vector<uint64_t> hostLeaves;
-    bool hostStale{true}; // hostLeaves lag the device leaves
 };
 
 int initGlobalTree(GlobalTree& g, unsigned bucket, cudaStream_t stream);
@@ -96,7 +94,8 @@ int initFocusTree(FocusTree& f, unsigned bucket, TreeScratch& s, cudaStream_t st
  *  global leaves, ancestor protection, rebalance, forced injection if needed. *converged = tree unchanged. */
 int focusUpdateTree(FocusTree& f, const GlobalTree& g, TreeScratch& s, cudaStream_t stream, bool* converged);
 
-/*! FocusedOctree::updateCounts at one rank (octree_focus_mpi.hpp:192-251) + layout (cstone/domain/layout.hpp) */
-int focusUpdateCounts(FocusTree& f, const uint64_t* keys, size_t n, cudaStream_t stream);
+/*! FocusedOctree::updateCounts at one rank (octree_focus_mpi.hpp:192-251) + layout (cstone/domain/layout.hpp); with a box,
+ *  also the node geometry (computeGeoCenters) */
+int focusUpdateCounts(FocusTree& f, const uint64_t* keys, size_t n, cudaStream_t stream, const DevBox* box = nullptr);
 
 } // namespace sphb

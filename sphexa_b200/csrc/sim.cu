@@ -220,8 +220,7 @@ int syncDomain(sphb_sim& s)
         s.ftree.firstCall = false;
     }
     SPHB_TRY(focusUpdateTree(s.ftree, s.gtree, s.ts, st, &converged));
-    SPHB_TRY(focusUpdateCounts(s.ftree, s.keys.data(), s.n, st));
-    SPHB_TRY(computeGeoCenters(s.ftree.tree, s.box, st));
+    SPHB_TRY(focusUpdateCounts(s.ftree, s.keys.data(), s.n, st, &s.box));
     SPHB_TRY(packPositionsAndBoxes(s.f[fX].data(), s.f[fY].data(), s.f[fZ].data(), s.f[fM].data(), s.n,
                                    s.pos.data(), s.mixed ? s.posq.data() : nullptr, s.box, s.blockLo.data(),
                                    s.blockHi.data(), st));

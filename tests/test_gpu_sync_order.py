@@ -170,3 +170,26 @@ def test_converged_leaves(cuda_device, n, kind, bucket):
     # no room, or only the count asked for: the number of leaves all the same
     rc = lib.sphb_compute_octree(L.ptr(keys), n, bucket, L.ptr(leaves), L.ptr(counts), num.value, C.byref(num), None)
     assert rc == L.SPHB_ERR_CAPACITY and num.value == want.size - 1
+
+
+@pytest.mark.parametrize("side", [4, 13, 27, 34, 36])
+@pytest.mark.parametrize("move", ["cells", "crowded", "equal keys"])
+def test_repeated_syncs_reach_the_converged_tree(cuda_device, side, move):
+    """trees of up to and above the 2,048 leaves that single blocks update: splits, merges and forced leaves end at the
+    tree in which a node with more than bucket_focus particles is split"""
+    from sphexa_b200 import ic as icm
+    from sphexa_b200 import lib as L
+    from sphexa_b200.simulation import Simulation
+    ic = icm.sedov(side)
+    sim = Simulation(ic, "mixed")
+    sim.sync()
+    rng = np.random.default_rng(side)
+    p = np.stack([sim.get(f) for f in ("x", "y", "z")])
+    for f, v in zip(("x", "y", "z"), MOVES[move](p, rng)):
+        sim.set(f, v - np.round(v))
+    for _ in range(25):
+        sim.sync()
+    leaves, counts, layout = sim.tree()
+    keys = sim.keys()
+    assert np.array_equal(leaves, _canonical(keys, 64))
+    assert np.array_equal(counts, np.diff(np.searchsorted(keys, leaves[:-1]), append=keys.size))
