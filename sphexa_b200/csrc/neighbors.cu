@@ -32,21 +32,24 @@ constexpr int kLeafCap   = 256; // candidate leaves buffered before they are str
 
 /*! Lanes that share a target. One lane per target tests and appends for its own particle, 32 targets per warp. A group's
  *  traversal, staging and tests run one after another, so a launch of few groups takes as long as its slowest one, with
- *  most of the GPU idle. With four lanes per target a warp serves eight targets: each lane tests and appends a quarter of
- *  the staged candidates, and the smaller search box admits about half of them. But each box is traversed and staged by
- *  itself, so a launch that fills the GPU is slower with it: hence the limits below.
- *  Neighbour phase before the traversal took four nodes a round, us for one and for four lanes: 16^3 particles 117 and 75,
- *  30^3 167 and 122, 36^3 203 and 144; 50^3 327 and 426, 63^3 394 and 579, 81^3 702 and 939. Searches of listed groups,
- *  a small part of all: block time steps of 64^3 509 and 452; 128^3 1569 and 1690. */
-constexpr int kSharedLanes          = 4;
-constexpr size_t kSharedLanesAll    = 40000;
-constexpr size_t kSharedLanesListed = 300000;
+ *  most of the GPU idle. With four (eight) lanes per target a warp serves eight (four) targets: each lane tests and
+ *  appends its part of the staged candidates, and the smaller search box admits fewer of them. But each box is traversed
+ *  and staged by itself, so a launch that fills the GPU is slower with it: hence the limits below.
+ *  Neighbour phase, us. Whole searches with four and eight lanes: 16^3 particles 64 and 49, 36^3 (a sphere of them)
+ *  99 and 108, 30^3 FP64 103 and 117; with one and four, before the traversal took four nodes a round: 30^3 167 and 122,
+ *  50^3 327 and 426, 63^3 394 and 579. Searches of listed groups, a small part of all, with one, four and eight: block
+ *  time steps of 64^3 450, 320 and 298; 128^3 with one and four 1569 and 1690. */
+constexpr int kFewLanes             = 4;
+constexpr int kManyLanes            = 8;
+constexpr size_t kManyLanesAll      = 10000;
+constexpr size_t kFewLanesAll       = 40000;
+constexpr size_t kManyLanesListed   = 300000;
 
-template<int kPer>
+template<int kPer, bool kSkin>
 struct NbShared
 {
-    //! list entries a target buffers: the chunk being filled; where lanes share it, up to 32 more neighbours at a time
-    static constexpr int kRing = kPer == 1 ? kNbChunk : 5 * kNbChunk;
+    //! list entries a target buffers: the chunk being filled and up to 8 more neighbours (kPer 1) or 32
+    static constexpr int kRing = (kPer == 1 ? 2 : 5) * kNbChunk;
     int stack[kNbWarps][kStackCap];
     int leafFirst[kNbWarps][kLeafCap]; // the buffered leaves, then the first particle of each
     int leafEnd[kNbWarps][kLeafCap];   // one past its last particle
@@ -62,7 +65,7 @@ struct NbShared
     // per target: the neighbours of the list chunks being filled, written out as 32-byte sectors when full; target minor,
     // so that the appends of a warp fall into distinct banks
     uint32_t nbuf[kNbWarps][kRing * kWarp / kPer];
-    uint16_t dbuf[kNbWarps][kRing * kWarp / kPer]; // skin rows: the quantised build distance of each entry
+    uint16_t dbuf[kNbWarps][kSkin ? kRing * kWarp / kPer : 1]; // skin rows: the quantised build distance of each entry
 };
 
 /*! Half width of the band |d^2 - (2h)^2| < band * (2h)^2 in which the FP32 distance cannot decide and the exact FP64
@@ -157,7 +160,7 @@ __global__ void __launch_bounds__(kNbThreads, 8) findNeighborsKernel(const doubl
                                                                   const TreeView* __restrict__ views,
                                                                   const uint8_t* __restrict__ inst, SearchExtras ex)
 {
-    __shared__ NbShared<kPer> sh;
+    __shared__ NbShared<kPer, kKind == kSearchSkin> sh;
     if (ex.gate && !((ex.gateMask >> __ldg(ex.gate)) & 1u)) { return; }
     constexpr int kTargets = kWarp / kPer; // targets of a warp
     const int warp         = threadIdx.x / kWarp;
@@ -257,7 +260,7 @@ __global__ void __launch_bounds__(kNbThreads, 8) findNeighborsKernel(const doubl
 
         // this target's ring of list chunks, entry e at ring[(e mod kRing) * kStride], and the store of a full chunk to the
         // chunked list layout (nidxAt)
-        constexpr int kRing   = NbShared<kPer>::kRing;
+        constexpr int kRing   = NbShared<kPer, kSkin>::kRing;
         constexpr int kStride = kTargets;
         uint32_t* ring        = &sh.nbuf[warp][lane / kPer];
         uint16_t* dring       = &sh.dbuf[warp][lane / kPer];
@@ -310,7 +313,7 @@ __global__ void __launch_bounds__(kNbThreads, 8) findNeighborsKernel(const doubl
             ring[(e % kRing) * kStride] = uint32_t(j);
         };
 
-        // test the staged 32 candidates (this lane's quarter of them where lanes share a target) against the target and
+        // test the staged 32 candidates (this lane's part of them where lanes share a target) against the target and
         // append the neighbours in index order
         constexpr int kShare = kWarp / kPer; // candidates per lane
         auto testStaged = [&](int numReal) {
@@ -355,19 +358,23 @@ __global__ void __launch_bounds__(kNbThreads, 8) findNeighborsKernel(const doubl
             }
             if constexpr (kPer == 1)
             {
-                // append the neighbours in candidate (= index) order
+                // append the neighbours in candidate (= index) order, up to eight before the chunk that filled up is
+                // stored: the warp's lanes store together instead of at every append that fills a chunk (neighbour phase of
+                // 101^3 FP64 1096 -> 1052 us, of 63^3 332 -> 315)
                 while (sure)
                 {
-                    int k = __ffs(sure) - 1;
-                    sure &= sure - 1u;
-                    int j = sh.cj[warp][k];
-                    if (size_t(j) == i) { continue; }
-                    if (count < listCap)
+                    const unsigned from = count;
+                    while (sure && count - from < kNbChunk)
                     {
-                        put(k, j, count);
-                        if (count % kNbChunk == kNbChunk - 1) { storeChunk(count / kNbChunk); }
+                        int k = __ffs(sure) - 1;
+                        sure &= sure - 1u;
+                        int j = sh.cj[warp][k];
+                        if (size_t(j) == i) { continue; }
+                        if (count < listCap) { put(k, j, count); }
+                        ++count;
                     }
-                    ++count;
+                    const unsigned c = min(from, listCap) / kNbChunk;
+                    if (min(count, listCap) / kNbChunk != c) { storeChunk(c); }
                 }
             }
             else
@@ -523,8 +530,8 @@ __global__ void __launch_bounds__(kNbThreads, 8) findNeighborsKernel(const doubl
 
         // Depth-first traversal in SFC order, the lowest key on top of the stack: an entry is the first child of an internal
         // node or the complement of a leaf. Every round takes the top four entries, tests the children of the internal ones,
-        // one per lane, and buffers the leaves that come before the first internal node; the rest goes back in order. A node a
-        // round, tested by eight lanes and its leaves looked up by one, took the search of 81^3 Noh particles from 525 to 716 us.
+        // one per lane, and buffers the leaves that come before the first internal node; the rest goes back in order. With a node
+        // a round, tested by eight lanes and its leaves looked up by one, the search of 81^3 Noh particles took 716 us, now 525.
         const int rootChild = tv.childOffsets[0];
         int sp              = 1;
         if (lane == 0) { stack[0] = rootChild ? rootChild : ~tv.nodeToLeaf[0]; }
@@ -703,7 +710,8 @@ int findNeighbors(const double* x, const double* y, const double* z, const doubl
     SearchExtras ex{};
     ex.gate     = gate;
     ex.gateMask = gateMask;
-    if (n <= kSharedLanesAll) { SPHB_SEARCH(kSearchAll, kSharedLanes, searchBlocks(n, kSharedLanes), h, nidx, nc) }
+    if (n <= kManyLanesAll) { SPHB_SEARCH(kSearchAll, kManyLanes, searchBlocks(n, kManyLanes), h, nidx, nc) }
+    else if (n <= kFewLanesAll) { SPHB_SEARCH(kSearchAll, kFewLanes, searchBlocks(n, kFewLanes), h, nidx, nc) }
     else { SPHB_SEARCH(kSearchAll, 1, searchBlocks(n, 1), h, nidx, nc) }
     countLaunch();
     SPHB_CUDA_TRY(cudaGetLastError());
@@ -720,10 +728,7 @@ int findNeighborsListed(const double* x, const double* y, const double* z, const
     SearchExtras ex{};
     ex.groups    = groups;
     ex.numListed = numListed;
-    if (n <= kSharedLanesListed)
-    {
-        SPHB_SEARCH(kSearchListed, kSharedLanes, listedBlocks(n, kSharedLanes), h, nidx, nc)
-    }
+    if (n <= kManyLanesListed) { SPHB_SEARCH(kSearchListed, kManyLanes, listedBlocks(n, kManyLanes), h, nidx, nc) }
     else { SPHB_SEARCH(kSearchListed, 1, listedBlocks(n, 1), h, nidx, nc) }
     countLaunch();
     SPHB_CUDA_TRY(cudaGetLastError());
@@ -747,7 +752,8 @@ int buildSkinLists(const double* x, const double* y, const double* z, const doub
     ex.gateMask    = gateMask;
     // the kernel writes h only in the iterating kinds, never in this one
     double* hRead = const_cast<double*>(h);
-    if (n <= kSharedLanesAll) { SPHB_SEARCH(kSearchSkin, kSharedLanes, searchBlocks(n, kSharedLanes), hRead, nullptr, nullptr) }
+    if (n <= kManyLanesAll) { SPHB_SEARCH(kSearchSkin, kManyLanes, searchBlocks(n, kManyLanes), hRead, nullptr, nullptr) }
+    else if (n <= kFewLanesAll) { SPHB_SEARCH(kSearchSkin, kFewLanes, searchBlocks(n, kFewLanes), hRead, nullptr, nullptr) }
     else { SPHB_SEARCH(kSearchSkin, 1, searchBlocks(n, 1), hRead, nullptr, nullptr) }
     countLaunch();
     SPHB_CUDA_TRY(cudaGetLastError());
