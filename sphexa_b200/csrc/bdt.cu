@@ -267,12 +267,16 @@ __device__ inline unsigned lowerBound(const uint64_t* sortedKeys, unsigned num, 
     return lo;
 }
 
+//! one thread per rung
 __global__ void rungInfoKernel(const uint64_t* keys, unsigned num, unsigned fastIdx, uint32_t* out)
 {
     float minDt = __uint_as_float(unsigned(keys[0]));
-    out[0]      = unsigned(keys[0]);
-    out[1]      = unsigned(keys[min(fastIdx, num - 1)]);
-    for (int r = 1; r < kMaxRungs; ++r)
+    if (threadIdx.x == 0)
+    {
+        out[0] = unsigned(keys[0]);
+        out[1] = unsigned(keys[min(fastIdx, num - 1)]);
+    }
+    for (int r = 1 + threadIdx.x; r < kMaxRungs; r += 32)
     {
         float maxDtRung = float(1 << r) * minDt;
         out[1 + r]      = lowerBound(keys, num, maxDtRung);
@@ -395,7 +399,7 @@ int launchSortedDt(const uint64_t* keys, unsigned num, unsigned fastIdx, float* 
 {
     if (num == 0) { return kErrArg; }
     sortedDtKernel<<<ceilDiv(num, kBdtThreads), kBdtThreads, 0, s>>>(keys, num, groupDt);
-    rungInfoKernel<<<1, 1, 0, s>>>(keys, num, fastIdx, out);
+    rungInfoKernel<<<1, 32, 0, s>>>(keys, num, fastIdx, out);
     countLaunch();
     countLaunch();
     SPHB_CUDA_TRY(cudaGetLastError());

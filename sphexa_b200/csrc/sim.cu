@@ -858,8 +858,12 @@ int sortGroupDt(sphb_sim& s, unsigned num, float* minDt, float* fastDt, uint32_t
 {
     cudaStream_t st = s.stream;
     SPHB_TRY(launchDtKeys(s.groupDt.data(), num, s.dtKeys.data(), s.groupIdx.data(), st));
-    SPHB_TRY(sortByKeyAsync(s.dtKeys.data(), s.groupIdx.data(), num, false, s.sortScratch.data(),
-                            s.sortScratch.capacity(), 0x0fu, s.status.data() + 2, st));
+    if (num <= kSortShortMax) { SPHB_TRY(sortShortKeysAsync(s.dtKeys.data(), s.groupIdx.data(), num, st)); }
+    else
+    {
+        SPHB_TRY(sortByKeyAsync(s.dtKeys.data(), s.groupIdx.data(), num, false, s.sortScratch.data(),
+                                s.sortScratch.capacity(), 0x0fu, s.status.data() + 2, st));
+    }
     unsigned fastIdx = unsigned(0.4f * float(num)); // LocalIndex(fastFraction * numGroups), ts_rungs.hpp:86,102
     SPHB_TRY(launchSortedDt(s.dtKeys.data(), num, fastIdx, s.groupDt.data(), s.rungInfo.data(), st));
     uint32_t info[1 + kMaxRungs];

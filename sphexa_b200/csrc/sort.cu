@@ -530,6 +530,130 @@ int sortNearlySorted(uint64_t* keys, uint32_t* values, size_t n, void* scratch, 
     return sortByKey(keys, values, n, false, scratch, scratchBytes, stream);
 }
 
+namespace
+{
+
+constexpr int kBlockSortThreads = 1024;
+constexpr int kBlockSortItems   = 16;
+constexpr int kBlockSortWarps   = kBlockSortThreads / kWarp;
+constexpr int kBlockSortMax     = kBlockSortThreads * kBlockSortItems;
+static_assert(kBlockSortMax == int(kSortShortMax), "sort.cuh");
+
+struct BlockSortShared
+{
+    uint32_t key[kBlockSortMax];
+    uint32_t val[kBlockSortMax];
+    uint16_t warpCount[kBlockSortWarps][kRadix]; // keys of a digit per warp, then those of the warps before it
+    uint32_t digitBase[kRadix];
+    uint32_t warpSum[kRadix / kWarp];
+};
+
+/*! stable LSD sort of up to kBlockSortMax keys of 32 bits by one block in shared memory, ranked as in onesweepKernel; a
+ *  digit that all keys share is skipped */
+__global__ void __launch_bounds__(kBlockSortThreads) blockSortKernel(uint64_t* keys, uint32_t* values, int n)
+{
+    extern __shared__ __align__(16) char raw[];
+    BlockSortShared& sh = *reinterpret_cast<BlockSortShared*>(raw);
+    const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
+    const int base = warp * kBlockSortItems * kWarp + lane;
+
+    for (int i = threadIdx.x; i < n; i += kBlockSortThreads)
+    {
+        sh.key[i] = uint32_t(keys[i]);
+        sh.val[i] = values[i];
+    }
+    for (int shift = 0; shift < 32; shift += kRadixBits)
+    {
+        for (int t = threadIdx.x; t < kBlockSortWarps * kRadix; t += kBlockSortThreads)
+        {
+            (&sh.warpCount[0][0])[t] = 0;
+        }
+        __syncthreads();
+        uint32_t key[kBlockSortItems], val[kBlockSortItems];
+        uint16_t rank[kBlockSortItems];
+#pragma unroll
+        for (int k = 0; k < kBlockSortItems; ++k)
+        {
+            const int idx    = base + k * kWarp;
+            const bool valid = idx < n;
+            key[k]           = valid ? sh.key[idx] : 0u;
+            val[k]           = valid ? sh.val[idx] : 0u;
+            uint32_t digit   = (key[k] >> shift) & (kRadix - 1);
+            uint32_t peers   = __match_any_sync(0xffffffffu, valid ? digit : 0xffffffffu);
+            uint32_t before  = valid ? sh.warpCount[warp][digit] : 0u;
+            uint32_t lower   = peers & ((1u << lane) - 1u);
+            rank[k]          = uint16_t(before + __popc(lower));
+            __syncwarp();
+            if (valid && lower == 0) { sh.warpCount[warp][digit] = uint16_t(before + __popc(peers)); }
+            __syncwarp();
+        }
+        __syncthreads();
+        // per digit: the warps' counts, then the digits' first positions (thread d owns digit d)
+        uint32_t total = 0, incl = 0;
+        if (threadIdx.x < kRadix)
+        {
+            for (int w = 0; w < kBlockSortWarps; ++w)
+            {
+                uint32_t c                    = sh.warpCount[w][threadIdx.x];
+                sh.warpCount[w][threadIdx.x] = uint16_t(total);
+                total += c;
+            }
+            incl = total;
+#pragma unroll
+            for (int off = 1; off < kWarp; off <<= 1)
+            {
+                uint32_t t = __shfl_up_sync(0xffffffffu, incl, off);
+                if (lane >= off) { incl += t; }
+            }
+            if (lane == kWarp - 1) { sh.warpSum[warp] = incl; }
+        }
+        const bool shared = __syncthreads_or(threadIdx.x < kRadix && total == uint32_t(n));
+        if (shared) { continue; }
+        if (threadIdx.x < kRadix)
+        {
+            uint32_t before = 0;
+            for (int w = 0; w < warp; ++w)
+            {
+                before += sh.warpSum[w];
+            }
+            sh.digitBase[threadIdx.x] = before + incl - total;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kBlockSortItems; ++k)
+        {
+            if (base + k * kWarp < n)
+            {
+                uint32_t digit = (key[k] >> shift) & (kRadix - 1);
+                uint32_t pos   = sh.digitBase[digit] + sh.warpCount[warp][digit] + rank[k];
+                sh.key[pos]    = key[k];
+                sh.val[pos]    = val[k];
+            }
+        }
+        __syncthreads();
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += kBlockSortThreads)
+    {
+        keys[i]   = sh.key[i];
+        values[i] = sh.val[i];
+    }
+}
+
+} // namespace
+
+int sortShortKeysAsync(uint64_t* keys, uint32_t* values, size_t n, cudaStream_t stream)
+{
+    if (n == 0) { return kOk; }
+    if (n > kSortShortMax) { return kErrArg; }
+    SPHB_CUDA_TRY(cudaFuncSetAttribute(blockSortKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       int(sizeof(BlockSortShared))));
+    blockSortKernel<<<1, kBlockSortThreads, sizeof(BlockSortShared), stream>>>(keys, values, int(n));
+    countLaunch();
+    SPHB_CUDA_TRY(cudaGetLastError());
+    return kOk;
+}
+
 int sortByKeyAsync(uint64_t* keys, uint32_t* values, size_t n, bool initValues, void* scratch, size_t scratchBytes,
                    unsigned passMask, uint32_t* errorOut, cudaStream_t stream, const uint32_t* gate)
 {

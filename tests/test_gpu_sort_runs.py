@@ -45,3 +45,32 @@ def test_sort_by_key_matches_the_stable_sort(cuda_device, kind, n):
     torch.cuda.synchronize()
     assert np.array_equal(dk.cpu().numpy().view(np.uint64), keys[order])
     assert np.array_equal(dv.cpu().numpy(), values[order])
+
+
+@pytest.mark.parametrize("n", [1, 2, 511, 513, 8193, 16_384, 16_385])
+@pytest.mark.parametrize("kind", ["floats", "few", "equal", "one digit"])
+def test_one_block_sort(cuda_device, kind, n):
+    """the sort of the groups' time steps, at the edges of a warp's part and of the block's capacity"""
+    import ctypes as C
+    import torch
+    from sphexa_b200 import lib as L
+    sort = L.load()["_ZN4sphb18sortShortKeysAsyncEPmPjmP11CUstream_st"]  # internal: no C entry of its own
+    sort.argtypes = [C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p]
+    rng = np.random.default_rng(n)
+    if kind == "floats":
+        keys = rng.uniform(1e-7, 1e-3, n).astype(np.float32).view(np.uint32).astype(np.uint64)
+    else:
+        keys = rng.integers(0, {"few": 7, "equal": 1, "one digit": 256}[kind], n, dtype=np.uint64)
+        keys = keys << U(16) if kind == "one digit" else keys + U(0xfffffff0)
+    dk = torch.from_numpy(keys.view(np.int64)).cuda()
+    dv = torch.arange(n, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    rc = sort(dk.data_ptr(), dv.data_ptr(), n, None)
+    torch.cuda.synchronize()
+    if n > 16_384:
+        assert rc == L.SPHB_ERR_ARG
+        return
+    assert rc == L.SPHB_OK
+    order = np.argsort(keys, kind="stable")
+    assert np.array_equal(dk.cpu().numpy().view(np.uint64), keys[order])
+    assert np.array_equal(dv.cpu().numpy(), order.astype(np.int32))
