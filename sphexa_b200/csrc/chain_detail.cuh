@@ -100,15 +100,18 @@ __device__ __forceinline__ T maxOverSplit(T v)
 __device__ __forceinline__ double fdiv(double a, double b) { return a / b; }
 __device__ __forceinline__ float fdiv(float a, float b) { return __fdividef(a, b); }
 
-// Sums of products with the rounding written out. Left to the compiler, which product of a sum becomes the FMA's can
-// differ between the instances of a kernel (one lane or several per target, a single simulation or an ensemble), and
-// with it the last bit of their results.
+// Sums of products with the rounding written out. Left to the compiler, which product of a sum becomes the FMA's differs
+// between the instances of a kernel (one lane or several per target, a single simulation or an ensemble), and with it the
+// last bit of their results. A last bit counts: the AV switches jump where divv changes its sign, by the full range of
+// alpha for such a particle. So every FP32 sum keeps the order that the one-lane instances had when the compiler chose
+// it, and where that is not the order of these functions the sum is written with fma; tests/test_gpu_mixed_bits.py holds
+// the results to it.
 
-//! a . b
+//! a . b: y first, then x, then z
 template<class T>
 __device__ __forceinline__ T dot3(T ax, T ay, T az, T bx, T by, T bz)
 {
-    return fma(az, bz, fma(ay, by, ax * bx));
+    return fma(az, bz, fma(ax, bx, ay * by));
 }
 
 //! a b + c d

@@ -301,7 +301,7 @@ __global__ void __launch_bounds__(kChainMaxThreads, sizeof(T) == 4 && kSplit == 
         T c13i = prodDiff(tau12, tau23, tau22, tau13) * factor;
         T c22i = prodDiff(tau11, tau33, tau13, tau13) * factor;
         T c23i = prodDiff(tau13, tau12, tau11, tau23) * factor;
-        T c33i = prodDiff(tau11, tau22, tau12, tau12) * factor;
+        T c33i = fma(-tau12, tau12, tau11 * tau22) * factor;
 
         // dV_ab = -sum_c C_bc M_ac
         T M[3][3] = {{mxx.get(), mxy.get(), mxz.get()}, {myx.get(), myy.get(), myz.get()},
@@ -423,9 +423,9 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? kAvMaxThreads : kChainMaxThre
     T gdx = gx.get(), gdy = gy.get(), gdz = gz.get();
     {
         T sx = gdx, sy = gdy, sz = gdz;
-        gdx  = -dot3(gr.c11, gr.c12, gr.c13, sx, sy, sz);
-        gdy  = -dot3(gr.c12, gr.c22, gr.c23, sx, sy, sz);
-        gdz  = -dot3(gr.c13, gr.c23, gr.c33, sx, sy, sz);
+        gdx  = -fma(gr.c13, sz, fma(gr.c12, sy, gr.c11 * sx));
+        gdy  = -fma(gr.c23, sz, fma(gr.c22, sy, gr.c12 * sx));
+        gdz  = -fma(gr.c33, sz, fma(gr.c23, sy, gr.c13 * sx));
     }
     T graddivv = sqrt(dot3(gdx, gdy, gdz, gdx, gdy, gdz));
     if constexpr (kMode & kModeTape)
@@ -572,8 +572,8 @@ __global__ void __launch_bounds__(kChainMaxThreads, (sizeof(T) == 4 && kSplit ==
                 {
                     float sigma = k.ramp * (fdiv(dRho, sRho) - k.Atmin);
                     float lxj   = log2f(xmassj);
-                    aMom        = exp2f(prodSum(2.0f - sigma, lxi, sigma, lxj));
-                    bMom        = exp2f(prodSum(2.0f - sigma, lxj, sigma, lxi));
+                    aMom        = exp2f(prodSum(sigma, lxj, 2.0f - sigma, lxi));
+                    bMom        = exp2f(prodSum(sigma, lxi, 2.0f - sigma, lxj));
                 }
                 float aVisc = mj * invRhoi * visc;
                 float bVisc = hj.vol * visc;
@@ -583,8 +583,8 @@ __global__ void __launch_bounds__(kChainMaxThreads, (sizeof(T) == 4 && kSplit ==
                                                   __fmul2_rn(tA1, make_float2(vxij, vxij))));
                 aViscE.add(0.5f * prodSum(aVisc, dv.x, bVisc, dv.y));
                 energyS.add(mj * aMom * dv.x);
-                float cI = prodSum(mj * prhoi, aMom, 0.5f, aVisc);
-                float cJ = prodSum(mj * hj.prho, bMom, 0.5f, bVisc);
+                float cI = prodSum(0.5f, aVisc, mj * prhoi, aMom);
+                float cJ = prodSum(0.5f, bVisc, mj * hj.prho, bMom);
                 momX.add(prodSum(cI, tA1.x, cJ, tA1.y));
                 momY.add(prodSum(cI, tA2.x, cJ, tA2.y));
                 momZ.add(prodSum(cI, tA3.x, cJ, tA3.y));
@@ -640,10 +640,21 @@ __global__ void __launch_bounds__(kChainMaxThreads, (sizeof(T) == 4 && kSplit ==
                 T vijsignal = T(0.5) * (ci + cj) - T(2) * wij;
                 maxvsignalI = vijsignal > maxvsignalI ? vijsignal : maxvsignalI;
 
-                // |rho_i - rho_j| against A (rho_i + rho_j), both times vol_j = m_j / rho_j
+                // |rho_i - rho_j| against A (rho_i + rho_j); FP64: both times vol_j = m_j / rho_j, without a division
                 T aMom, bMom;
-                T rhoiVol = rhoi * hj.vol;
-                T dRho = fabs(rhoiVol - mj), sRho = rhoiVol + mj;
+                T dRho, sRho;
+                if constexpr (sizeof(T) == 4)
+                {
+                    T rhoj = fdiv(mj, hj.vol);
+                    dRho   = fabs(rhoi - rhoj);
+                    sRho   = rhoi + rhoj;
+                }
+                else
+                {
+                    T rhoiVol = rhoi * hj.vol;
+                    dRho      = fabs(rhoiVol - mj);
+                    sRho      = rhoiVol + mj;
+                }
                 if (dRho < k.Atmin * sRho)
                 {
                     aMom = xmassi * xmassi;
@@ -660,8 +671,8 @@ __global__ void __launch_bounds__(kChainMaxThreads, (sizeof(T) == 4 && kSplit ==
                     if constexpr (sizeof(T) == 4)
                     {
                         T lxj = log2f(xmassj);
-                        aMom  = exp2f(prodSum(T(2) - sigma, lxi, sigma, lxj));
-                        bMom  = exp2f(prodSum(T(2) - sigma, lxj, sigma, lxi));
+                        aMom  = exp2f(prodSum(sigma, lxj, T(2) - sigma, lxi));
+                        bMom  = exp2f(prodSum(sigma, lxi, T(2) - sigma, lxj));
                     }
                     else
                     {
@@ -675,16 +686,16 @@ __global__ void __launch_bounds__(kChainMaxThreads, (sizeof(T) == 4 && kSplit ==
 
                 T aVisc  = mj * invRhoi * visc;
                 T bVisc  = hj.vol * visc;
-                T aViscX = T(0.5) * prodSum(aVisc, tA1i, bVisc, tA1j);
-                T aViscY = T(0.5) * prodSum(aVisc, tA2i, bVisc, tA2j);
-                T aViscZ = T(0.5) * prodSum(aVisc, tA3i, bVisc, tA3j);
-                aViscE.add(dot3(aViscX, aViscY, aViscZ, vxij, vyij, vzij));
+                T viscX = prodSum(aVisc, tA1i, bVisc, tA1j);
+                T viscY = prodSum(aVisc, tA2i, bVisc, tA2j);
+                T viscZ = prodSum(aVisc, tA3i, bVisc, tA3j);
+                aViscE.add(dot3(T(0.5) * viscX, T(0.5) * viscY, T(0.5) * viscZ, vxij, vyij, vzij));
                 energyS.add(mj * aMom * dot3(vxij, vyij, vzij, tA1i, tA2i, tA3i));
                 T momI = mj * prhoi * aMom;
                 T momJ = mj * hj.prho * bMom;
-                momX.add(fma(momI, tA1i, fma(momJ, tA1j, aViscX)));
-                momY.add(fma(momI, tA2i, fma(momJ, tA2j, aViscY)));
-                momZ.add(fma(momI, tA3i, fma(momJ, tA3j, aViscZ)));
+                momX.add(fma(T(0.5), viscX, prodSum(momI, tA1i, momJ, tA1j)));
+                momY.add(fma(T(0.5), viscY, prodSum(momI, tA2i, momJ, tA2j)));
+                momZ.add(fma(T(0.5), viscZ, prodSum(momI, tA3i, momJ, tA3j)));
             }
         };
         // one pair per iteration: the unrolled 8-pair body overflowed the instruction cache (FP32 2.04 -> 1.71 ms at
