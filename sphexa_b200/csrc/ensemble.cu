@@ -429,29 +429,31 @@ void swapState(sphb_ensemble& e)
 /*! keys, segmented sort, gather of 16 fields into the other buffer set, which then becomes the current one (a
  *  captured step records the buffers of its set; the two captured steps alternate). The particles are sorted by the
  *  leaves of their member's tree, as in a single simulation; the trees stay those of the last rebuild, so a leaf can
- *  outgrow a warp: then the full segmented radix sort (by key over all slots, then stably by instance) takes its
- *  place, decided on the device (every one of its kernels reads that flag and returns at once when it is zero). Before
- *  the first trees the radix sort runs. The result is the same stable sort either way. */
+ *  grow past 2,048 particles: then the full segmented radix sort (by key over all slots, then stably by instance) takes
+ *  its place, decided on the device (every one of its kernels reads that flag and returns at once when it is zero). It
+ *  runs alone before the first trees and for buckets that the first step could fill that far. The result is the same
+ *  stable sort either way. */
 int syncBatched(sphb_ensemble& e, bool withLayout)
 {
     cudaStream_t st = e.stream;
     size_t n        = e.slots;
     SPHB_TRY(launchSfcKeys(e.f[0].data(), e.f[1].data(), e.f[2].data(), e.keys.data(), n, e.box, st));
     SPHB_CUDA_TRY(cudaMemcpyAsync(e.keysTmp.data(), e.keys.data(), n * sizeof(uint64_t), cudaMemcpyDeviceToDevice, st));
-    const uint32_t* remaining = nullptr;
-    if (withLayout)
+    const uint32_t* overflow = nullptr;
+    const bool byLeaves      = withLayout && e.p.bucket_focus <= 1024;
+    if (byLeaves)
     {
         SPHB_TRY(sortSegmentsByLeavesAsync(e.keys.data(), e.keysTmp.data(), e.order.data(), n, e.segOfSlot.data(),
                                            e.leafSets.data(), e.numBuckets, e.leafSort, e.sortScratch.data(),
-                                           e.sortScratch.capacity(), &remaining, st));
+                                           e.sortScratch.capacity(), &overflow, st));
     }
-    SPHB_TRY(sortByKeyAsync(e.keysTmp.data(), e.order.data(), n, !withLayout, e.sortScratch.data(),
-                            e.sortScratch.capacity(), 0xffu, e.status.data() + 2, st, remaining));
+    SPHB_TRY(sortByKeyAsync(e.keysTmp.data(), e.order.data(), n, !byLeaves, e.sortScratch.data(),
+                            e.sortScratch.capacity(), 0xffu, e.status.data() + 2, st, overflow));
     const void* segSrc[1] = {e.segOfSlot.data()};
     void* segDst[1]       = {e.segKey.data()};
     SPHB_TRY(gather8(e.order.data(), n, 1, segSrc, segDst, st));
     SPHB_TRY(sortByKeyAsync(e.segKey.data(), e.order.data(), n, false, e.sortScratch.data(),
-                            e.sortScratch.capacity(), 0x1u, e.status.data() + 2, st, remaining));
+                            e.sortScratch.capacity(), 0x1u, e.status.data() + 2, st, overflow));
     const void* src[16];
     void* dst[16];
     for (int k = 0; k < kFields; ++k)
@@ -538,7 +540,7 @@ int rebuildTrees(sphb_ensemble& e)
     SPHB_TRY(e.leafSets.reserve(e.num));
     SPHB_CUDA_TRY(cudaMemcpyAsync(e.leafSets.data(), sets.data(), e.num * sizeof(LeafSet), cudaMemcpyHostToDevice, st));
     SPHB_TRY(e.leafSort.slot.reserve(e.slots));
-    SPHB_TRY(e.leafSort.first.reserve(e.numBuckets + 3));
+    SPHB_TRY(e.leafSort.first.reserve(leafSortInts(e.numBuckets)));
     SPHB_TRY(e.leafSort.scanTmp.reserve(scanTempInts(e.numBuckets) + 1));
     dim3 grid(unsigned(ceilDiv(size_t(e.maxLeaves) + 1, 256)), unsigned(e.num));
     forestLayoutKernel<<<grid, 256, 0, st>>>(e.leafDescs.data(), e.keys.data());

@@ -741,15 +741,27 @@ int runPasses(uint64_t* keys, uint32_t* values, size_t n, const SortScratch& s, 
 // moves by up to n, and then both repair passes (45 us each at 4,096 particles, 91 us at 128^3) were followed by the
 // radix sort (eight passes of 18 to 38 us and an 8 KB host read). Sync of a step with such a motion: 16^3 235 -> 154 us,
 // 30^3 510 -> 168 us, 81^3 (Noh) 663 -> 263 us, 128^3 0.95 -> 0.43 ms. A warp sorts a leaf in registers, at most
-// 128 keys (four per lane): the tree splits leaves of more than 64, so only a sudden compression exceeds it. An ensemble
-// of 663,000 particles in 16 members (its trees stay those of the last rebuild) 0.69 -> 0.21 ms.
+// 128 keys (four per lane): the tree splits leaves of more than 64, so only a sudden compression exceeds it, or trees
+// that stay those of the last rebuild (an ensemble's; 663,000 particles in 16 members 0.69 -> 0.21 ms): a block sorts
+// such a leaf, up to 2,048 keys. Beyond that the radix sort runs.
 // ---------------------------------------------------------------------------------------------------------------
 
 namespace
 {
 
-//! the largest leaf a warp sorts (four elements per lane)
-constexpr int kLeafSortCap = 128;
+//! the largest leaf a warp sorts (four elements per lane), and the largest one a block sorts
+constexpr int kLeafSortCap  = 128;
+constexpr int kLeafBlockCap = 2048;
+
+//! words before the bucket counts
+enum LeafFlag
+{
+    kLeafInversions, // an adjacent pair is out of order (one tree only)
+    kLeafOverflow,   // a bucket exceeds kLeafBlockCap: nothing is sorted
+    kLeafLarge,      // a bucket exceeds kLeafSortCap
+    kLeafListed,     // number of such buckets, listed by leafSortKernel
+    kNumLeafFlags
+};
 
 //! largest l with leaves[l] <= key (leaves[0] = 0; l = numLeaves for keys past the last leaf)
 __device__ __forceinline__ int leafOf(const uint64_t* __restrict__ leaves, int numLeaves, uint64_t key)
@@ -774,8 +786,7 @@ __device__ __forceinline__ LeafSet leafSetOf(const LeafSet& one, const LeafSet* 
 }
 
 /*! values = 0..n-1; slot[i] = {bucket (leaf) of key i, its place among the bucket's keys in arrival order}, counts[l] =
- *  keys per bucket (zero on entry); flags[0] = 1 if any adjacent pair is out of order (one tree only), flags[1] = 1 if
- *  a bucket exceeds kLeafSortCap. The lanes of a bucket (most of a warp: the keys are nearly in order) share one
+ *  keys per bucket (zero on entry), and the flags (zero on entry). The lanes of a bucket (most of a warp: the keys are nearly in order) share one
  *  atomic. */
 template<bool kSeg>
 __global__ void __launch_bounds__(256) leafSlotKernel(const uint64_t* __restrict__ keys, size_t n, LeafSet one,
@@ -803,10 +814,12 @@ __global__ void __launch_bounds__(256) leafSlotKernel(const uint64_t* __restrict
     base      = __shfl_sync(0xffffffffu, base, leader);
     int place = base + __popc(peers & ((1u << lane) - 1u));
     if (valid) { slot[i] = make_uint2(unsigned(bucket), unsigned(place)); }
-    unsigned anyInv  = __ballot_sync(0xffffffffu, inv);
-    unsigned anyFull = __ballot_sync(0xffffffffu, valid && place >= kLeafSortCap);
-    if (lane == 0 && anyInv) { flags[0] = 1u; }
-    if (lane == 0 && anyFull) { flags[1] = 1u; }
+    unsigned anyInv   = __ballot_sync(0xffffffffu, inv);
+    unsigned anyLarge = __ballot_sync(0xffffffffu, valid && place >= kLeafSortCap);
+    unsigned anyOver  = __ballot_sync(0xffffffffu, valid && place >= kLeafBlockCap);
+    if (lane == 0 && anyInv) { flags[kLeafInversions] = 1u; }
+    if (lane == 0 && anyLarge) { flags[kLeafLarge] = 1u; }
+    if (lane == 0 && anyOver) { flags[kLeafOverflow] = 1u; }
 }
 
 /*! composite[first[bucket] + place] = (the upper 32 bits of the key within its leaf, index): what a warp sorts. A leaf
@@ -819,7 +832,7 @@ __global__ void __launch_bounds__(256) leafScatterKernel(const uint64_t* __restr
                                                          uint64_t* __restrict__ composite, const unsigned* flags)
 {
     size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
-    if (i >= n || (kSeg && flags[1] != 0)) { return; }
+    if (i >= n || (kSeg && flags[kLeafOverflow] != 0)) { return; }
     uint2 s        = slot[i];
     LeafSet t      = leafSetOf<kSeg>(one, many, seg, i);
     int leaf       = int(s.x - t.bucket0);
@@ -942,23 +955,93 @@ __device__ __forceinline__ void sortLeaf(const uint64_t* composite, const uint64
     }
 }
 
-//! one warp per bucket; with gate set, nothing runs if *gate is not 0
+//! one warp per bucket; larger ones are listed for leafBlockKernel (flags zero in kLeafListed on entry)
 __global__ void __launch_bounds__(256) leafSortKernel(const uint64_t* __restrict__ composite,
                                                       const uint64_t* __restrict__ keysIn, int numBuckets,
                                                       const int* __restrict__ first, uint64_t* __restrict__ keysOut,
-                                                      uint32_t* __restrict__ values, const unsigned* gate)
+                                                      uint32_t* __restrict__ values, unsigned* flags, uint32_t* large)
 {
     int bucket = int((blockIdx.x * size_t(blockDim.x) + threadIdx.x) / kWarp);
     int lane   = threadIdx.x & (kWarp - 1);
-    if (bucket >= numBuckets || (gate && *gate != 0)) { return; }
+    if (bucket >= numBuckets || flags[kLeafOverflow] != 0) { return; }
     int b = first[bucket], m = first[bucket + 1] - b;
     if (m <= 0) { return; }
     if (m <= 32) { sortLeaf<1>(composite, keysIn, b, m, lane, keysOut, values); }
     else if (m <= 64) { sortLeaf<2>(composite, keysIn, b, m, lane, keysOut, values); }
-    else { sortLeaf<4>(composite, keysIn, b, min(m, kLeafSortCap), lane, keysOut, values); }
+    else if (m <= kLeafSortCap) { sortLeaf<4>(composite, keysIn, b, m, lane, keysOut, values); }
+    else if (lane == 0) { large[atomicAdd(flags + kLeafListed, 1u)] = uint32_t(bucket); }
 }
 
+constexpr int kLeafBlockThreads = 512;
+
+/*! One block per listed bucket: bitonic network on (key, index) in shared memory. An ensemble's trees stay those of the
+ *  last rebuild, and a contracting member outgrows the warps for the rest of a run; the radix sort of all slots that took
+ *  over before cost 140 us a step for 512,000 of them (sync 315 us, with this kernel 185, 176 before the leaf grew). */
+__global__ void __launch_bounds__(kLeafBlockThreads) leafBlockKernel(const uint64_t* __restrict__ composite,
+                                                                     const uint64_t* __restrict__ keysIn,
+                                                                     const int* __restrict__ first,
+                                                                     uint64_t* __restrict__ keysOut,
+                                                                     uint32_t* __restrict__ values,
+                                                                     const unsigned* flags, const uint32_t* large)
+{
+    __shared__ uint64_t key[kLeafBlockCap];
+    __shared__ uint32_t val[kLeafBlockCap];
+    if (flags[kLeafOverflow] != 0) { return; }
+    const unsigned num = flags[kLeafListed];
+    for (unsigned l = blockIdx.x; l < num; l += gridDim.x)
+    {
+        const int b = first[large[l]];
+        const int m = min(first[large[l] + 1] - b, kLeafBlockCap);
+        int width   = 2 * kLeafSortCap;
+        while (width < m)
+        {
+            width <<= 1;
+        }
+        for (int e = threadIdx.x; e < width; e += kLeafBlockThreads)
+        {
+            val[e] = e < m ? uint32_t(composite[b + e]) : 0xffffffffu;
+            key[e] = e < m ? __ldg(keysIn + val[e]) : ~uint64_t(0);
+        }
+        __syncthreads();
+        for (int size = 2; size <= width; size <<= 1)
+        {
+            for (int stride = size >> 1; stride > 0; stride >>= 1)
+            {
+                // pair t of the stage: its lower element has a zero at the stride's bit
+                for (int t = threadIdx.x; t < width / 2; t += kLeafBlockThreads)
+                {
+                    int q        = 2 * t - (t & (stride - 1));
+                    int p        = q + stride;
+                    bool up      = (q & size) == 0;
+                    bool greater = key[q] > key[p] || (key[q] == key[p] && val[q] > val[p]);
+                    if (greater == up)
+                    {
+                        uint64_t k = key[q];
+                        key[q]     = key[p];
+                        key[p]     = k;
+                        uint32_t v = val[q];
+                        val[q]     = val[p];
+                        val[p]     = v;
+                    }
+                }
+                __syncthreads();
+            }
+        }
+        for (int e = threadIdx.x; e < m; e += kLeafBlockThreads)
+        {
+            keysOut[b + e] = key[e];
+            values[b + e]  = val[e];
+        }
+        __syncthreads();
+    }
+}
+
+//! blocks of leafBlockKernel: every one may find a bucket, none has many
+unsigned leafBlocks(size_t n) { return unsigned(std::min<size_t>(ceilDiv(n, kLeafSortCap), size_t(smCount()) * 2)); }
+
 } // namespace
+
+size_t leafSortInts(size_t numBuckets) { return kNumLeafFlags + numBuckets + 1; }
 
 int sortByLeaves(uint64_t* keys, uint64_t* keysOut, uint32_t* values, size_t n, const uint64_t* leaves, int numLeaves,
                  LeafSortScratch& ls, void* scratch, size_t scratchBytes, LeafSort* result, cudaStream_t stream)
@@ -973,31 +1056,38 @@ int sortByLeaves(uint64_t* keys, uint64_t* keysOut, uint32_t* values, size_t n, 
     if (!scratch || scratchBytes < sortScratchBytes(n)) { return kErrCapacity; }
     size_t buckets = size_t(numLeaves) + 1;
     SPHB_TRY(ls.slot.reserve(n));
-    SPHB_TRY(ls.first.reserve(buckets + 1 + 2));
+    SPHB_TRY(ls.first.reserve(leafSortInts(buckets)));
     SPHB_TRY(ls.scanTmp.reserve(scanTempInts(buckets) + 1));
-    int* counts     = ls.first.data() + 2;
+    int* counts     = ls.first.data() + kNumLeafFlags;
     unsigned* flags = reinterpret_cast<unsigned*>(ls.first.data());
-    SPHB_CUDA_TRY(cudaMemsetAsync(ls.first.data(), 0, (buckets + 2) * sizeof(int), stream));
+    SPHB_CUDA_TRY(cudaMemsetAsync(ls.first.data(), 0, (kNumLeafFlags + buckets) * sizeof(int), stream));
     LeafSet one{leaves, numLeaves, 0};
     leafSlotKernel<false><<<ceilDiv(n, 256), 256, 0, stream>>>(keys, n, one, nullptr, nullptr, values, ls.slot.data(),
                                                                counts, flags);
     countLaunch();
     SPHB_CUDA_TRY(cudaGetLastError());
-    unsigned msg[2];
+    unsigned msg[kLeafLarge + 1];
     SPHB_TRY(readBack(stream, {{msg, flags, sizeof(msg)}}));
-    if (!msg[0])
+    if (!msg[kLeafInversions])
     {
         *result = LeafSort::identity;
         return kOk;
     }
-    if (msg[1]) { return sortByKey(keys, values, n, false, scratch, scratchBytes, stream); }
+    if (msg[kLeafOverflow]) { return sortByKey(keys, values, n, false, scratch, scratchBytes, stream); }
     uint64_t* composite = carve(scratch, n).keysAlt;
+    uint32_t* large     = carve(scratch, n).valsAlt;
     SPHB_TRY(exclusiveScan(counts, counts, buckets, ls.scanTmp.data(), stream));
     leafScatterKernel<false><<<ceilDiv(n, 256), 256, 0, stream>>>(keys, n, one, nullptr, nullptr, ls.slot.data(), counts,
                                                                   composite, nullptr);
     leafSortKernel<<<ceilDiv(buckets * kWarp, 256), 256, 0, stream>>>(composite, keys, int(buckets), counts, keysOut,
-                                                                      values, nullptr);
+                                                                      values, flags, large);
     countLaunch(2);
+    if (msg[kLeafLarge])
+    {
+        leafBlockKernel<<<leafBlocks(n), kLeafBlockThreads, 0, stream>>>(composite, keys, counts, keysOut, values, flags,
+                                                                         large);
+        countLaunch();
+    }
     SPHB_CUDA_TRY(cudaGetLastError());
     *result = LeafSort::keysOut;
     return kOk;
@@ -1008,16 +1098,17 @@ int sortSegmentsByLeavesAsync(const uint64_t* keys, uint64_t* keysOut, uint32_t*
                               size_t scratchBytes, const unsigned** overflow, cudaStream_t stream)
 {
     if (!scratch || scratchBytes < sortScratchBytes(n) || ls.slot.capacity() < n ||
-        ls.first.capacity() < numBuckets + 3 || ls.scanTmp.capacity() < scanTempInts(numBuckets) + 1)
+        ls.first.capacity() < leafSortInts(numBuckets) || ls.scanTmp.capacity() < scanTempInts(numBuckets) + 1)
     {
         return kErrCapacity;
     }
-    int* counts     = ls.first.data() + 2;
+    int* counts     = ls.first.data() + kNumLeafFlags;
     unsigned* flags = reinterpret_cast<unsigned*>(ls.first.data());
-    *overflow       = flags + 1;
-    SPHB_CUDA_TRY(cudaMemsetAsync(ls.first.data(), 0, (numBuckets + 2) * sizeof(int), stream));
+    *overflow       = flags + kLeafOverflow;
+    SPHB_CUDA_TRY(cudaMemsetAsync(ls.first.data(), 0, (kNumLeafFlags + numBuckets) * sizeof(int), stream));
     if (n == 0) { return kOk; }
     uint64_t* composite = carve(scratch, n).keysAlt;
+    uint32_t* large     = carve(scratch, n).valsAlt;
     LeafSet none{nullptr, 0, 0};
     leafSlotKernel<true><<<ceilDiv(n, 256), 256, 0, stream>>>(keys, n, none, sets, seg, values, ls.slot.data(), counts,
                                                               flags);
@@ -1026,8 +1117,10 @@ int sortSegmentsByLeavesAsync(const uint64_t* keys, uint64_t* keysOut, uint32_t*
     leafScatterKernel<true><<<ceilDiv(n, 256), 256, 0, stream>>>(keys, n, none, sets, seg, ls.slot.data(), counts,
                                                                  composite, flags);
     leafSortKernel<<<ceilDiv(numBuckets * kWarp, 256), 256, 0, stream>>>(composite, keys, int(numBuckets), counts,
-                                                                         keysOut, values, flags + 1);
-    countLaunch(2);
+                                                                         keysOut, values, flags, large);
+    leafBlockKernel<<<leafBlocks(n), kLeafBlockThreads, 0, stream>>>(composite, keys, counts, keysOut, values, flags,
+                                                                     large);
+    countLaunch(3);
     SPHB_CUDA_TRY(cudaGetLastError());
     return kOk;
 }

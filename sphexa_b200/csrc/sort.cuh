@@ -27,6 +27,9 @@ enum class LeafSort
     keysOut   // in keysOut
 };
 
+//! entries of LeafSortScratch::first for so many buckets (the leaves and one for the keys past the last leaf)
+size_t leafSortInts(size_t numBuckets);
+
 //! device buffers of sortByLeaves
 struct LeafSortScratch
 {
@@ -37,8 +40,8 @@ struct LeafSortScratch
 
 /*! The same stable sort (values = 0..n-1 first) with the help of a cornerstone leaf array that held few keys per leaf
  *  for keys close to these, the tree of the previous step: every key finds its leaf, a scan of the leaf counts places
- *  the leaves, and one warp sorts each leaf. One host read, of whether anything is out of order and whether a leaf
- *  grew past 128 keys (then the radix sort runs, in place). It reads and writes the keys twice whatever the particles'
+ *  the leaves, and one warp sorts each leaf, a block one of more than 128 keys. One host read, of whether anything is out
+ *  of order and whether a leaf grew past 2,048 keys (then the radix sort runs, in place). It reads and writes the keys twice whatever the particles'
  *  motion is, where the radix sort takes eight passes. */
 int sortByLeaves(uint64_t* keys, uint64_t* keysOut, uint32_t* values, size_t n, const uint64_t* leaves, int numLeaves,
                  LeafSortScratch& ls, void* scratch, size_t scratchBytes, LeafSort* result, cudaStream_t stream);
@@ -67,8 +70,8 @@ struct LeafSet
 
 /*! sortByLeaves for an array of contiguous segments (seg[i] ascending; sets[k] the leaves of segment k, numBuckets
  *  buckets over all segments), without any host synchronisation. values = 0..n-1, then the stable order by (segment,
- *  key) and the keys in it in keysOut; if a bucket grew past 128 keys, **overflow (device) is not 0 and only values =
- *  0..n-1 was written. The buffers of ls must be large enough beforehand (slot n, first numBuckets + 3, scanTmp
+ *  key) and the keys in it in keysOut; if a bucket grew past 2,048 keys, **overflow (device) is not 0 and only values =
+ *  0..n-1 was written. The buffers of ls must be large enough beforehand (slot n, first leafSortInts(numBuckets), scanTmp
  *  scanTempInts(numBuckets) + 1). */
 int sortSegmentsByLeavesAsync(const uint64_t* keys, uint64_t* keysOut, uint32_t* values, size_t n, const uint64_t* seg,
                               const LeafSet* sets, size_t numBuckets, LeafSortScratch& ls, void* scratch,
