@@ -39,8 +39,8 @@ struct SortScratch
     uint64_t* keysAlt;
     uint32_t* valsAlt;
     uint32_t* hist;       // [kPasses][kRadix] counts, then exclusive offsets
-    uint32_t* status;     // [numTiles][kRadix]
-    uint32_t* counters;   // [0] tile counter, [1] error word, [2] sortRunsKernel's flag
+    uint32_t* status;     // [numTiles][kRadix], directly behind hist
+    uint32_t* counters;   // [0] tile counter, [1] error word, [2] longRunsKernel's flag, [3] runs that sortRunsKernel listed
 };
 
 size_t alignUp(size_t x, size_t a) { return (x + a - 1) / a * a; }
@@ -63,33 +63,124 @@ SortScratch carve(void* base, size_t n)
     return s;
 }
 
-//! digit histograms of all 8 byte positions in one sweep over the keys
-__global__ void __launch_bounds__(256) histogramKernel(const uint64_t* __restrict__ keys, size_t n,
-                                                       uint32_t* __restrict__ hist, const uint32_t* gate)
+//! keys of equal upper bits that one thread puts in order, and those that a block sorts
+constexpr int kRunCap      = 32;
+constexpr int kRunBlockCap = 2048;
+
+//! passes on the upper digits before the runs are looked at: 32 bits tell nearly all of 2^30 spread keys apart
+constexpr int kUpperPasses = 4;
+
+constexpr int kHistThreads = 1024;
+constexpr int kSamples     = 4096;
+constexpr int kSampleSlots = 2 * kSamples;
+
+/*! *verdict = 1 if many keys probably lie in runs that no block sorts, else 0: counts the samples (spread evenly,
+ *  up to kSamples) that agree in the upper digits with an earlier, different one. A hash table holds 8 bits of a fingerprint, the
+ *  first sample and the count of each. A run of kRunBlockCap keys holds kRunBlockCap samples / n of them; three of spread
+ *  keys hardly ever agree. Equal keys, which are in order, do not count. The upper digits are the kUpperPasses highest
+ *  ones in which the samples differ. By one block of kHistThreads. */
+__device__ void sampleRuns(const uint64_t* __restrict__ keys, size_t n, uint32_t* slots, uint32_t* verdict)
 {
-    if (gate && *gate == 0) { return; }
-    __shared__ uint32_t sh[kPasses][kRadix];
-    for (int t = threadIdx.x; t < kPasses * kRadix; t += blockDim.x)
+    __shared__ uint32_t differ; // the digits in which the samples differ
+    if (threadIdx.x == 0) { differ = 0; }
+    // one a thread serves few keys as well
+    const size_t samples = min(min(n, size_t(kSamples)), max(n / 32, size_t(kHistThreads)));
+    uint64_t key[kSamples / kHistThreads];
+#pragma unroll
+    for (int r = 0; r < kSamples / kHistThreads; ++r)
     {
-        (&sh[0][0])[t] = 0;
+        size_t q = threadIdx.x + size_t(r) * kHistThreads;
+        key[r]   = __ldg(keys + (q < samples ? n * q / samples : 0));
+    }
+    for (int t = threadIdx.x; t < kSampleSlots; t += kHistThreads)
+    {
+        slots[t] = 0;
     }
     __syncthreads();
-    for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x)
+    uint64_t bits = 0;
+#pragma unroll
+    for (int r = 0; r < kSamples / kHistThreads; ++r)
+    {
+        bits |= key[r] ^ __ldg(keys);
+    }
+    uint32_t mine = 0;
+#pragma unroll
+    for (int p = 0; p < kPasses; ++p)
+    {
+        mine |= ((bits >> (p * kRadixBits)) & (kRadix - 1)) ? 1u << p : 0u;
+    }
+    mine = __reduce_or_sync(0xffffffffu, mine);
+    if ((threadIdx.x & (kWarp - 1)) == 0) { atomicOr(&differ, mine); }
+    __syncthreads();
+    uint32_t upper = differ;
+    while (__popc(upper) > kUpperPasses)
+    {
+        upper &= upper - 1;
+    }
+    const int shift    = upper ? (__ffs(upper) - 1) * kRadixBits : 0;
+    const size_t limit = max(size_t(3), size_t(kRunBlockCap) * samples * 3 / (4 * n));
+    unsigned most      = 0;
+#pragma unroll
+    for (int r = 0; r < kSamples / kHistThreads; ++r)
+    {
+        if (threadIdx.x + size_t(r) * kHistThreads >= samples) { continue; }
+        uint64_t h = (key[r] >> shift) * 0x9E3779B97F4A7C15ull; // multiplicative hashing (golden ratio)
+        h ^= h >> 29;
+        const uint32_t self = threadIdx.x + r * kHistThreads;
+        const uint32_t word = (uint32_t(h >> 32) & 0xff000000u) | (self << 12) | 1u;
+        for (uint32_t at = uint32_t(h >> 40) % kSampleSlots;; at = (at + 1) % kSampleSlots)
+        {
+            uint32_t old = atomicCAS(&slots[at], 0u, word);
+            if (old == 0) { break; }
+            if ((old ^ word) >> 24) { continue; }
+            // kSamples / 2 are enough for any limit, and no count reaches the sample's bits
+            bool equal = __ldg(keys + n * ((old >> 12) & 0xfffu) / samples) == key[r];
+            if (!equal && (old & 0xfffu) < kSamples / 2) { most = max(most, (atomicAdd(&slots[at], 1u) & 0xfffu) + 1u); }
+            break;
+        }
+    }
+    bool many = __syncthreads_or(most >= limit);
+    if (threadIdx.x == 0) { *verdict = many ? 1u : 0u; }
+}
+
+//! digit histograms of all 8 byte positions in one sweep over the keys; with verdict set, the first block takes a sample
+//! instead (sampleRuns), which costs nothing beside the sweep
+__global__ void __launch_bounds__(kHistThreads) histogramKernel(const uint64_t* __restrict__ keys, size_t n,
+                                                                uint32_t* __restrict__ hist, const uint32_t* gate,
+                                                                uint32_t* verdict = nullptr)
+{
+    if (gate && *gate == 0) { return; }
+    __shared__ uint32_t sh[kSampleSlots];
+    const unsigned blocks = verdict ? gridDim.x - 1 : gridDim.x;
+    const unsigned block  = verdict ? blockIdx.x - 1 : blockIdx.x;
+    if (verdict && blockIdx.x == 0)
+    {
+        sampleRuns(keys, n, sh, verdict);
+        return;
+    }
+    for (int t = threadIdx.x; t < kPasses * kRadix; t += kHistThreads)
+    {
+        sh[t] = 0;
+    }
+    __syncthreads();
+    for (size_t i = block * size_t(kHistThreads) + threadIdx.x; i < n; i += size_t(blocks) * kHistThreads)
     {
         uint64_t k = keys[i];
 #pragma unroll
         for (int p = 0; p < kPasses; ++p)
         {
-            atomicAdd(&sh[p][(k >> (p * kRadixBits)) & (kRadix - 1)], 1u);
+            atomicAdd(&sh[p * kRadix + ((k >> (p * kRadixBits)) & (kRadix - 1))], 1u);
         }
     }
     __syncthreads();
-    for (int t = threadIdx.x; t < kPasses * kRadix; t += blockDim.x)
+    for (int t = threadIdx.x; t < kPasses * kRadix; t += kHistThreads)
     {
-        uint32_t c = (&sh[0][0])[t];
+        uint32_t c = sh[t];
         if (c) { atomicAdd(hist + t, c); }
     }
 }
+
+unsigned histogramBlocks(size_t n) { return unsigned(std::min<size_t>(ceilDiv(n, 4 * kHistThreads), size_t(smCount()) * 2)); }
 
 //! exclusive scan of each pass's 256 digit counts, in place (one block per pass)
 __global__ void histScanKernel(uint32_t* hist, const uint32_t* gate)
@@ -359,39 +450,62 @@ __global__ void orErrorKernel(const uint32_t* err, uint32_t* out)
 namespace
 {
 
-//! keys of equal upper bits that one thread puts in order
-constexpr int kRunCap = 32;
+//! one past the last of the keys in [i, end) whose upper bits are those of key i
+__device__ __forceinline__ size_t runEnd(const uint64_t* keys, size_t i, size_t end, int shift)
+{
+    uint64_t up = keys[i] >> shift;
+    while (end - i > 1)
+    {
+        size_t mid = i + (end - i) / 2;
+        if ((keys[mid] >> shift) == up) { i = mid; }
+        else { end = mid; }
+    }
+    return end;
+}
 
-/*! After a stable sort by the bits from `shift` up, sets *flag if a run of more than kRunCap keys of equal upper bits is
- *  out of order. */
+//! the first of the keys in [begin, i] whose upper bits are those of key i
+__device__ __forceinline__ size_t runBegin(const uint64_t* keys, size_t begin, size_t i, int shift)
+{
+    uint64_t up = keys[i] >> shift;
+    while (i > begin)
+    {
+        size_t mid = begin + (i - begin) / 2;
+        if ((keys[mid] >> shift) == up) { i = mid; }
+        else { begin = mid + 1; }
+    }
+    return i;
+}
+
+/*! After a stable sort by the bits from `shift` up, sets *flag if a run of more than kRunBlockCap keys of equal upper bits
+ *  is out of order. */
 __global__ void __launch_bounds__(256) longRunsKernel(const uint64_t* __restrict__ keys, size_t n, int shift,
                                                       uint32_t* flag)
 {
     size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x + 1;
     if (i >= n || keys[i] >= keys[i - 1]) { return; }
     uint64_t up = keys[i] >> shift;
-    size_t b    = i - 1;
-    size_t e    = i + 1;
-    while (b > 0 && e - b <= size_t(kRunCap) && (keys[b - 1] >> shift) == up)
-    {
-        --b;
-    }
-    while (e < n && e - b <= size_t(kRunCap) && (keys[e] >> shift) == up)
-    {
-        ++e;
-    }
-    if (e - b > size_t(kRunCap)) { *flag = 1u; }
+    bool back   = i >= size_t(kRunCap) && (keys[i - kRunCap] >> shift) == up;
+    bool ahead  = i + kRunCap < n && (keys[i + kRunCap] >> shift) == up;
+    if (!back && !ahead) { return; }
+    size_t b = runBegin(keys, i > size_t(kRunBlockCap) ? i - kRunBlockCap : 0, i, shift);
+    size_t e = runEnd(keys, i, min(n, i + kRunBlockCap + 1), shift);
+    if (e - b > size_t(kRunBlockCap)) { *flag = 1u; }
 }
 
-/*! the thread of the first key of every run of equal upper bits sorts the run by insertion, stably: after longRunsKernel,
- *  which leaves only short ones to sort (a longer run is in order, *flag clear) */
+/*! the thread of the first key of every run of equal upper bits sorts the run by insertion, stably, or lists it (counters
+ *  [3], list) for runBlockKernel: after longRunsKernel, which leaves no larger one out of order (counters[2] clear) */
 __global__ void __launch_bounds__(256) sortRunsKernel(uint64_t* keys, uint32_t* values, size_t n, int shift,
-                                                      const uint32_t* flag)
+                                                      uint32_t* counters, uint32_t* list)
 {
     size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
-    if (i + 1 >= n || *flag) { return; }
+    if (i + 1 >= n || counters[2]) { return; }
     uint64_t up = keys[i] >> shift;
     if ((keys[i + 1] >> shift) != up || (i > 0 && (keys[i - 1] >> shift) == up)) { return; }
+    if (i + kRunCap < n && (keys[i + kRunCap] >> shift) == up)
+    {
+        list[atomicAdd(counters + 3, 1u)] = uint32_t(i); // at most n / (kRunCap + 1) of them
+        return;
+    }
     for (size_t a = i + 1; a < n && a - i < size_t(kRunCap); ++a)
     {
         uint64_t k = keys[a];
@@ -409,8 +523,89 @@ __global__ void __launch_bounds__(256) sortRunsKernel(uint64_t* keys, uint32_t* 
     }
 }
 
-//! passes on the upper digits before the runs are looked at: 32 bits tell nearly all of 2^30 spread keys apart
-constexpr int kUpperPasses = 4;
+constexpr int kRunBlockThreads = 256;
+
+//! bitonic network over elements 0 .. width - 1 (a power of two) by one block; exchange(q, p, up) puts the pair q < p in
+//! ascending (up) or descending order
+template<int kThreads, class F>
+__device__ __forceinline__ void blockBitonic(int width, F&& exchange)
+{
+    for (int size = 2; size <= width; size <<= 1)
+    {
+        for (int stride = size >> 1; stride > 0; stride >>= 1)
+        {
+            // pair t of the stage: its lower element has a zero at the stride's bit
+            for (int t = threadIdx.x; t < width / 2; t += kThreads)
+            {
+                int q = 2 * t - (t & (stride - 1));
+                exchange(q, q + stride, (q & size) == 0);
+            }
+            __syncthreads();
+        }
+    }
+}
+
+/*! one block per listed run (longer ones than kRunBlockCap are in order): its open lower bits, at most 32, with the
+ *  position behind them, so that equal keys keep their order */
+__global__ void __launch_bounds__(kRunBlockThreads) runBlockKernel(uint64_t* keys, uint32_t* values, size_t n, int shift,
+                                                                   const uint32_t* counters, const uint32_t* list)
+{
+    __shared__ uint64_t v[kRunBlockCap];
+    if (counters[2]) { return; }
+    const unsigned num      = counters[3];
+    const uint64_t openBits = (uint64_t(1) << shift) - 1;
+    for (unsigned l = blockIdx.x; l < num; l += gridDim.x)
+    {
+        const size_t b = list[l];
+        const size_t e = runEnd(keys, b, min(n, b + kRunBlockCap + 1), shift);
+        const int m    = int(e - b);
+        if (m > kRunBlockCap) { continue; }
+        const uint64_t up = keys[b] & ~openBits;
+        int width         = 64;
+        while (width < m)
+        {
+            width <<= 1;
+        }
+        for (int t = threadIdx.x; t < width; t += kRunBlockThreads)
+        {
+            v[t] = t < m ? ((keys[b + t] & openBits) << 11) | uint64_t(t) : ~uint64_t(0);
+        }
+        __syncthreads();
+        bool disorder = false;
+        for (int t = threadIdx.x; t + 1 < m; t += kRunBlockThreads)
+        {
+            disorder = disorder || v[t] > v[t + 1];
+        }
+        if (!__syncthreads_or(disorder)) { continue; }
+        blockBitonic<kRunBlockThreads>(width, [&](int q, int p, bool ascending) {
+            uint64_t x = v[q], y = v[p];
+            if ((x > y) == ascending)
+            {
+                v[q] = y;
+                v[p] = x;
+            }
+        });
+        uint32_t val[kRunBlockCap / kRunBlockThreads];
+#pragma unroll
+        for (int r = 0; r < kRunBlockCap / kRunBlockThreads; ++r)
+        {
+            int t  = threadIdx.x + r * kRunBlockThreads;
+            val[r] = t < m ? values[b + (v[t] & (kRunBlockCap - 1))] : 0u;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < kRunBlockCap / kRunBlockThreads; ++r)
+        {
+            int t = threadIdx.x + r * kRunBlockThreads;
+            if (t < m)
+            {
+                keys[b + t]   = up | (v[t] >> 11);
+                values[b + t] = val[r];
+            }
+        }
+        __syncthreads();
+    }
+}
 
 } // namespace
 
@@ -429,12 +624,14 @@ int sortByKey(uint64_t* keys, uint32_t* values, size_t n, bool initValues, void*
     }
 
     SPHB_CUDA_TRY(cudaMemsetAsync(s.hist, 0, kPasses * kRadix * sizeof(uint32_t), stream));
-    unsigned histBlocks = unsigned(std::min<size_t>(ceilDiv(n, 256 * 16), size_t(smCount()) * 4));
-    histogramKernel<<<histBlocks, 256, 0, stream>>>(keys, n, s.hist, nullptr);
+    unsigned histBlocks = histogramBlocks(n);
+    const bool sample = n > size_t(kRunBlockCap);
+    histogramKernel<<<histBlocks + (sample ? 1 : 0), kHistThreads, 0, stream>>>(keys, n, s.hist, nullptr,
+                                                                                sample ? s.status : nullptr);
     SPHB_CUDA_TRY(cudaGetLastError());
 
-    // decide on the host which passes are trivial (one digit holds every key)
-    uint32_t h[kPasses * kRadix];
+    // decide on the host which passes are trivial (one digit holds every key); the word behind is the sample's verdict
+    uint32_t h[kPasses * kRadix + 1];
     SPHB_CUDA_TRY(cudaMemcpyAsync(h, s.hist, sizeof(h), cudaMemcpyDeviceToHost, stream));
     SPHB_CUDA_TRY(cudaStreamSynchronize(stream));
     bool doPass[kPasses];
@@ -452,12 +649,14 @@ int sortByKey(uint64_t* keys, uint32_t* values, size_t n, bool initValues, void*
     {
         mask |= doPass[p] ? (1u << p) : 0u;
     }
-    // Space-filling-curve keys differ in all eight digits, but few agree in the upper four: half the passes and a repair of
-    // the short runs that do (sort and tree of 4,000,037 clustered keys 1.38 -> 1.04 ms, half of that gain with five
-    // passes; of 19,709 keys 0.33 -> 0.26 ms). If a run is long and out of order, the full sort follows (twelve passes
-    // instead of eight); it is stable, as what came before, so the result is the same.
+    // Space-filling-curve keys differ in all eight digits, but few agree in the upper four: half the passes and a sort of
+    // the runs that do, by a thread (up to 32 keys) or a block (up to 2,048). Keys of which many lie in longer runs are
+    // told by a sample beforehand and take all eight passes. Where the sample missed a long run that is out of order, they
+    // follow the four; they are stable, as what came before, so the result is the same.
+    // 4,000,037 keys, us, eight passes / this: spread 857 / 502, one run of 40 858 / 513, a tenth in runs of 40 845 / 604,
+    // all in runs of 64 774 / 775 or of 1,000 748 / 750, half in one cell 793 / 792, half equal 687 / 423.
     unsigned upper = mask;
-    while (__builtin_popcount(upper) > kUpperPasses)
+    while (!(sample && h[kPasses * kRadix]) && __builtin_popcount(upper) > kUpperPasses)
     {
         upper &= upper - 1;
     }
@@ -465,12 +664,14 @@ int sortByKey(uint64_t* keys, uint32_t* values, size_t n, bool initValues, void*
     // block of readBack is allocated on its first use in a thread)
     uint32_t msg[2] = {0, 0};
     SPHB_TRY(runPasses(keys, values, n, s, upper, stream));
-    SPHB_CUDA_TRY(cudaMemsetAsync(s.counters + 2, 0, sizeof(uint32_t), stream));
+    SPHB_CUDA_TRY(cudaMemsetAsync(s.counters + 2, 0, 2 * sizeof(uint32_t), stream));
     if (upper != mask)
     {
         int shift = __builtin_ctz(upper) * kRadixBits;
         longRunsKernel<<<ceilDiv(n, 256), 256, 0, stream>>>(keys, n, shift, s.counters + 2);
-        sortRunsKernel<<<ceilDiv(n, 256), 256, 0, stream>>>(keys, values, n, shift, s.counters + 2);
+        sortRunsKernel<<<ceilDiv(n, 256), 256, 0, stream>>>(keys, values, n, shift, s.counters, s.valsAlt);
+        unsigned blocks = unsigned(std::min<size_t>(ceilDiv(n, kRunCap + 1), size_t(smCount()) * 8));
+        runBlockKernel<<<blocks, kRunBlockThreads, 0, stream>>>(keys, values, n, shift, s.counters, s.valsAlt);
         SPHB_CUDA_TRY(cudaGetLastError());
     }
     SPHB_CUDA_TRY(cudaMemcpyAsync(msg, s.counters + 1, sizeof(msg), cudaMemcpyDeviceToHost, stream));
@@ -478,7 +679,7 @@ int sortByKey(uint64_t* keys, uint32_t* values, size_t n, bool initValues, void*
     if (!msg[0] && msg[1])
     {
         SPHB_CUDA_TRY(cudaMemsetAsync(s.hist, 0, kPasses * kRadix * sizeof(uint32_t), stream));
-        histogramKernel<<<histBlocks, 256, 0, stream>>>(keys, n, s.hist, nullptr);
+        histogramKernel<<<histBlocks, kHistThreads, 0, stream>>>(keys, n, s.hist, nullptr);
         SPHB_CUDA_TRY(cudaGetLastError());
         SPHB_TRY(runPasses(keys, values, n, s, mask, stream));
         SPHB_CUDA_TRY(cudaMemcpyAsync(msg, s.counters + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
@@ -667,8 +868,8 @@ int sortByKeyAsync(uint64_t* keys, uint32_t* values, size_t n, bool initValues, 
         SPHB_CUDA_TRY(cudaGetLastError());
     }
     SPHB_CUDA_TRY(cudaMemsetAsync(s.hist, 0, kPasses * kRadix * sizeof(uint32_t), stream));
-    unsigned histBlocks = unsigned(std::min<size_t>(ceilDiv(n, 256 * 16), size_t(smCount()) * 4));
-    histogramKernel<<<histBlocks, 256, 0, stream>>>(keys, n, s.hist, gate);
+    unsigned histBlocks = histogramBlocks(n);
+    histogramKernel<<<histBlocks, kHistThreads, 0, stream>>>(keys, n, s.hist, gate);
     SPHB_CUDA_TRY(cudaGetLastError());
     SPHB_TRY(runPasses(keys, values, n, s, passMask, stream, gate));
     if (errorOut) { orErrorKernel<<<1, 1, 0, stream>>>(s.counters + 1, errorOut); }
@@ -1003,30 +1204,17 @@ __global__ void __launch_bounds__(kLeafBlockThreads) leafBlockKernel(const uint6
             key[e] = e < m ? __ldg(keysIn + val[e]) : ~uint64_t(0);
         }
         __syncthreads();
-        for (int size = 2; size <= width; size <<= 1)
-        {
-            for (int stride = size >> 1; stride > 0; stride >>= 1)
+        blockBitonic<kLeafBlockThreads>(width, [&](int q, int p, bool up) {
+            if ((key[q] > key[p] || (key[q] == key[p] && val[q] > val[p])) == up)
             {
-                // pair t of the stage: its lower element has a zero at the stride's bit
-                for (int t = threadIdx.x; t < width / 2; t += kLeafBlockThreads)
-                {
-                    int q        = 2 * t - (t & (stride - 1));
-                    int p        = q + stride;
-                    bool up      = (q & size) == 0;
-                    bool greater = key[q] > key[p] || (key[q] == key[p] && val[q] > val[p]);
-                    if (greater == up)
-                    {
-                        uint64_t k = key[q];
-                        key[q]     = key[p];
-                        key[p]     = k;
-                        uint32_t v = val[q];
-                        val[q]     = val[p];
-                        val[p]     = v;
-                    }
-                }
-                __syncthreads();
+                uint64_t k = key[q];
+                key[q]     = key[p];
+                key[p]     = k;
+                uint32_t v = val[q];
+                val[q]     = val[p];
+                val[p]     = v;
             }
-        }
+        });
         for (int e = threadIdx.x; e < m; e += kLeafBlockThreads)
         {
             keysOut[b + e] = key[e];

@@ -74,3 +74,37 @@ def test_one_block_sort(cuda_device, kind, n):
     order = np.argsort(keys, kind="stable")
     assert np.array_equal(dk.cpu().numpy().view(np.uint64), keys[order])
     assert np.array_equal(dv.cpu().numpy(), order.astype(np.int32))
+
+
+@pytest.mark.parametrize("initial", [True, False])
+@pytest.mark.parametrize("n", [6_000, 70_001, 300_007])
+@pytest.mark.parametrize("length", [33, 64, 65, 1000, 2047, 2048, 2049, 5000])
+@pytest.mark.parametrize("share", ["one", "some", "all"])
+def test_runs_that_a_block_sorts(cuda_device, share, length, n, initial):
+    """runs of keys that agree in the upper half, on both sides of what a thread, a block and the sample take; equal keys
+    among them, whole runs of one key, and a run at either end"""
+    import torch
+    from sphexa_b200 import lib as L
+    lib = L.load()
+    rng = np.random.default_rng(n + length)
+    keys = rng.integers(0, 1 << 63, n, dtype=np.uint64)
+    part = {"one": length, "some": max(length, n // 5), "all": n}[share]
+    cell = np.arange(part, dtype=np.uint64) // U(length)
+    low = rng.integers(0, 1 << 32, part, dtype=np.uint64)
+    low[::7] = low[0]
+    low[cell % U(5) == 1] = U(77)
+    keys[:part] = (cell * U(0x2545f491) % U(1 << 31) << U(32)) + low
+    keys[part // 2:part] |= U(0x7fffffff00000000) if share == "some" else U(0)
+    if not initial:
+        keys = rng.permutation(keys)
+    order = np.argsort(keys, kind="stable")
+    dk = torch.from_numpy(keys.view(np.int64)).cuda()
+    values = rng.integers(0, 1 << 31, n, dtype=np.int32)
+    dv = torch.from_numpy(values).cuda()
+    size = lib.sphb_sort_by_key_scratch_bytes(n)
+    scratch = torch.empty(size, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    L.check(lib.sphb_sort_by_key(L.ptr(dk), L.ptr(dv), n, int(initial), L.ptr(scratch), size, None), "sort")
+    torch.cuda.synchronize()
+    assert np.array_equal(dk.cpu().numpy().view(np.uint64), keys[order])
+    assert np.array_equal(dv.cpu().numpy(), order if initial else values[order])
