@@ -26,8 +26,8 @@ namespace
 
 constexpr int kNbWarps   = 4;
 constexpr int kNbThreads = kNbWarps * kWarp;
-constexpr int kStackWide = 80;  // entries up to which the traversal takes four of them at a time
-constexpr int kStackCap  = 256; // kStackWide + 28, and 7 per level for those taken one at a time
+constexpr int kStackWide = 44;  // entries up to which the traversal takes four of them at a time
+constexpr int kStackCap  = 220; // kStackWide + 28, and 7 per level for those taken one at a time
 constexpr int kLeafCap   = 256; // candidate leaves buffered before they are streamed
 
 /*! Lanes that share a target. One lane per target tests and appends for its own particle, 32 targets per warp. A group's
@@ -149,16 +149,24 @@ struct SearchExtras
     unsigned gateMask;
 };
 
+/*! Blocks that stay resident on an SM: eight by their registers, fewer where the buffers do not fit into its shared memory
+ *  (228 KB, 1 KB of it per block for the system). Row builds with one lane per target keep seven. The other kinds keep
+ *  eight: a stack of 256 entries instead of 220 left them seven (neighbour phase of 101^3 FP64 1064 us, now 1029, of Noh
+ *  81^3 498, now 482, of 128^3 with a wide blast 2272, now 2191). */
+template<int kPer, bool kSkin>
+constexpr int residentBlocks()
+{
+    constexpr int fit = int(228 * 1024 / (sizeof(NbShared<kPer, kSkin>) + 1024));
+    return fit < 8 ? fit : 8;
+}
+static_assert(residentBlocks<1, false>() == 8 && residentBlocks<kFewLanes, true>() == 8, "the launches count on eight");
+
 template<bool kBatched, int kKind, int kPer>
-__global__ void __launch_bounds__(kNbThreads, 8) findNeighborsKernel(const double* __restrict__ x,
-                                                                  const double* __restrict__ y,
-                                                                  const double* __restrict__ z,
-                                                                  const double4* __restrict__ pos, double* h, size_t n,
-                                                                  TreeView tree, DevBox box, NeighborParams prm,
-                                                                  uint32_t* __restrict__ nidx,
-                                                                  unsigned* __restrict__ ncOut, unsigned* status,
-                                                                  const TreeView* __restrict__ views,
-                                                                  const uint8_t* __restrict__ inst, SearchExtras ex)
+__global__ void __launch_bounds__(kNbThreads, residentBlocks<kPer, kKind == kSearchSkin>())
+    findNeighborsKernel(const double* __restrict__ x, const double* __restrict__ y, const double* __restrict__ z,
+                        const double4* __restrict__ pos, double* h, size_t n, TreeView tree, DevBox box,
+                        NeighborParams prm, uint32_t* __restrict__ nidx, unsigned* __restrict__ ncOut, unsigned* status,
+                        const TreeView* __restrict__ views, const uint8_t* __restrict__ inst, SearchExtras ex)
 {
     __shared__ NbShared<kPer, kKind == kSearchSkin> sh;
     if (ex.gate && !((ex.gateMask >> __ldg(ex.gate)) & 1u)) { return; }
@@ -684,7 +692,11 @@ unsigned searchBlocks(size_t n, int per)
 }
 
 //! blocks of a listed search: at most those that stay resident
-unsigned listedBlocks(size_t n, int per) { return std::min(searchBlocks(n, per), unsigned(smCount()) * 8u); }
+template<int kPer>
+unsigned listedBlocks(size_t n)
+{
+    return std::min(searchBlocks(n, kPer), unsigned(smCount() * residentBlocks<kPer, false>()));
+}
 
 //! KERNEL<batched, kind, lanes per target> with one tree or the members' trees
 #define SPHB_SEARCH(KIND, PER, BLOCKS, H, NIDX, NC)                                                                    \
@@ -728,8 +740,8 @@ int findNeighborsListed(const double* x, const double* y, const double* z, const
     SearchExtras ex{};
     ex.groups    = groups;
     ex.numListed = numListed;
-    if (n <= kManyLanesListed) { SPHB_SEARCH(kSearchListed, kManyLanes, listedBlocks(n, kManyLanes), h, nidx, nc) }
-    else { SPHB_SEARCH(kSearchListed, 1, listedBlocks(n, 1), h, nidx, nc) }
+    if (n <= kManyLanesListed) { SPHB_SEARCH(kSearchListed, kManyLanes, listedBlocks<kManyLanes>(n), h, nidx, nc) }
+    else { SPHB_SEARCH(kSearchListed, 1, listedBlocks<1>(n), h, nidx, nc) }
     countLaunch();
     SPHB_CUDA_TRY(cudaGetLastError());
     return kOk;
