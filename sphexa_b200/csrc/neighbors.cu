@@ -37,13 +37,16 @@ constexpr int kLeafCap   = 256; // candidate leaves buffered before they are str
  *  and staged by itself, so a launch that fills the GPU is slower with it: hence the limits below.
  *  Neighbour phase, us. Whole searches with four and eight lanes: 16^3 particles 64 and 49, 36^3 (a sphere of them)
  *  99 and 108, 30^3 FP64 103 and 117; with one and four, before the traversal took four nodes a round: 30^3 167 and 122,
- *  50^3 327 and 426, 63^3 394 and 579. Searches of listed groups, a small part of all, with one, four and eight: block
- *  time steps of 64^3 450, 320 and 298; 128^3 with one and four 1569 and 1690. */
+ *  50^3 327 and 426, 63^3 394 and 579.
+ *  Searches of listed groups, a small part of all, choose by the length of the list, which only the device knows. Neighbour
+ *  phase with one lane, with eight, and with eight for lists of up to 1,500 groups (the same up to 100 either way): block
+ *  time steps of 64^3 334, 248 and 248, 81^3 414, 300 and 301, 90^3 378, 496 and 388, 100^3 468, 609 and 476, 100^3 with a
+ *  wide blast 757, 1480 and 760, global steps of 128^3 934, 1193 and 935. */
 constexpr int kFewLanes             = 4;
 constexpr int kManyLanes            = 8;
 constexpr size_t kManyLanesAll      = 10000;
 constexpr size_t kFewLanesAll       = 40000;
-constexpr size_t kManyLanesListed   = 300000;
+constexpr size_t kManyLanesListed   = 1500; // groups of the list
 
 template<int kPer, bool kSkin>
 struct NbShared
@@ -161,22 +164,22 @@ constexpr int residentBlocks()
 }
 static_assert(residentBlocks<1, false>() == 8 && residentBlocks<kFewLanes, true>() == 8, "the launches count on eight");
 
+/*! One warp's unit of the search: kWarp / kPer targets of a group of 32 (unit = kPer group + part; of a listed search,
+ *  group is the place in the list). */
 template<bool kBatched, int kKind, int kPer>
-__global__ void __launch_bounds__(kNbThreads, residentBlocks<kPer, kKind == kSearchSkin>())
-    findNeighborsKernel(const double* __restrict__ x, const double* __restrict__ y, const double* __restrict__ z,
-                        const double4* __restrict__ pos, double* h, size_t n, TreeView tree, DevBox box,
-                        NeighborParams prm, uint32_t* __restrict__ nidx, unsigned* __restrict__ ncOut, unsigned* status,
-                        const TreeView* __restrict__ views, const uint8_t* __restrict__ inst, SearchExtras ex)
+__device__ __forceinline__ void searchUnit(NbShared<kPer, kKind == kSearchSkin>& sh, size_t unit,
+                                           const double* __restrict__ x, const double* __restrict__ y,
+                                           const double* __restrict__ z, const double4* __restrict__ pos, double* h,
+                                           size_t n, const TreeView& tree, const DevBox& box, const NeighborParams& prm,
+                                           uint32_t* __restrict__ nidx, unsigned* __restrict__ ncOut, unsigned* status,
+                                           const TreeView* __restrict__ views, const uint8_t* __restrict__ inst,
+                                           const SearchExtras& ex)
 {
-    __shared__ NbShared<kPer, kKind == kSearchSkin> sh;
-    if (ex.gate && !((ex.gateMask >> __ldg(ex.gate)) & 1u)) { return; }
     constexpr int kTargets = kWarp / kPer; // targets of a warp
     const int warp         = threadIdx.x / kWarp;
     const int lane         = threadIdx.x & (kWarp - 1);
     const int piece        = lane % kPer; // which of the lanes that share the target
     const size_t numGroups = (n + kWarp - 1) / kWarp;
-    // kPer warps per group of 32
-    auto searchUnit = [&](size_t unit) {
     size_t group = unit / kPer;
     if constexpr (kKind == kSearchListed) { group = ex.groups[group]; }
     if (group >= numGroups) { return; }
@@ -481,15 +484,15 @@ __global__ void __launch_bounds__(kNbThreads, residentBlocks<kPer, kKind == kSea
                 }
                 unsigned m = __ballot_sync(0xffffffffu, keep);
                 int totalCand;
-                int ex = warpExclusive(keep ? plen : 0, lane, &totalCand);
+                int before = warpExclusive(keep ? plen : 0, lane, &totalCand);
                 if (keep)
                 {
                     int pos     = __popc(m & ((1u << lane) - 1u));
                     pStart[pos] = ps;
-                    pPre[pos]   = ex;
+                    pPre[pos]   = before;
                     for (int q = 0; q < plen; ++q)
                     {
-                        sh.pieceOf[warp][ex + q] = uint8_t(pos);
+                        sh.pieceOf[warp][before + q] = uint8_t(pos);
                     }
                 }
                 __syncwarp();
@@ -632,19 +635,53 @@ __global__ void __launch_bounds__(kNbThreads, residentBlocks<kPer, kKind == kSea
             h[i]     = hi;
         }
     }
-    };
-    size_t unit = size_t(blockIdx.x) * kNbWarps + warp;
-    if constexpr (kKind == kSearchListed)
+}
+
+template<bool kBatched, int kKind, int kPer>
+__global__ void __launch_bounds__(kNbThreads, residentBlocks<kPer, kKind == kSearchSkin>())
+    findNeighborsKernel(const double* __restrict__ x, const double* __restrict__ y, const double* __restrict__ z,
+                        const double4* __restrict__ pos, double* h, size_t n, TreeView tree, DevBox box,
+                        NeighborParams prm, uint32_t* __restrict__ nidx, unsigned* __restrict__ ncOut, unsigned* status,
+                        const TreeView* __restrict__ views, const uint8_t* __restrict__ inst, SearchExtras ex)
+{
+    __shared__ NbShared<kPer, kKind == kSearchSkin> sh;
+    if (ex.gate && !((ex.gateMask >> __ldg(ex.gate)) & 1u)) { return; }
+    searchUnit<kBatched, kKind, kPer>(sh, size_t(blockIdx.x) * kNbWarps + threadIdx.x / kWarp, x, y, z, pos, h, n, tree,
+                                      box, prm, nidx, ncOut, status, views, inst, ex);
+}
+
+//! the listed groups by as many blocks as stay resident: only the device knows how many they are
+template<bool kBatched>
+__global__ void __launch_bounds__(kNbThreads, residentBlocks<1, false>())
+    findListedKernel(const double* __restrict__ x, const double* __restrict__ y, const double* __restrict__ z,
+                     const double4* __restrict__ pos, double* h, size_t n, TreeView tree, DevBox box, NeighborParams prm,
+                     uint32_t* __restrict__ nidx, unsigned* __restrict__ ncOut, unsigned* status,
+                     const TreeView* __restrict__ views, const uint8_t* __restrict__ inst, SearchExtras ex)
+{
+    __shared__ union
     {
-        // as many blocks as stay resident walk the list, whose length only the device knows
-        const size_t units = size_t(*ex.numListed) * kPer;
-        for (; unit < units; unit += size_t(gridDim.x) * kNbWarps)
+        NbShared<1, false> one;
+        NbShared<kManyLanes, false> many;
+    } sh;
+    const size_t listed = *ex.numListed;
+    const size_t stride = size_t(gridDim.x) * kNbWarps;
+    size_t unit         = size_t(blockIdx.x) * kNbWarps + threadIdx.x / kWarp;
+    if (listed <= kManyLanesListed)
+    {
+        for (; unit < listed * kManyLanes; unit += stride)
         {
-            searchUnit(unit);
+            searchUnit<kBatched, kSearchListed, kManyLanes>(sh.many, unit, x, y, z, pos, h, n, tree, box, prm, nidx, ncOut,
+                                                            status, views, inst, ex);
             __syncwarp();
         }
+        return;
     }
-    else { searchUnit(unit); }
+    for (; unit < listed; unit += stride)
+    {
+        searchUnit<kBatched, kSearchListed, 1>(sh.one, unit, x, y, z, pos, h, n, tree, box, prm, nidx, ncOut, status, views,
+                                               inst, ex);
+        __syncwarp();
+    }
 }
 
 //! bounding box of each run of kBlockSize consecutive particles, relative to the box corner, rounded outwards
@@ -691,13 +728,6 @@ unsigned searchBlocks(size_t n, int per)
     return unsigned((units + kNbWarps - 1) / kNbWarps);
 }
 
-//! blocks of a listed search: at most those that stay resident
-template<int kPer>
-unsigned listedBlocks(size_t n)
-{
-    return std::min(searchBlocks(n, kPer), unsigned(smCount() * residentBlocks<kPer, false>()));
-}
-
 //! KERNEL<batched, kind, lanes per target> with one tree or the members' trees
 #define SPHB_SEARCH(KIND, PER, BLOCKS, H, NIDX, NC)                                                                    \
     if (views)                                                                                                          \
@@ -740,8 +770,17 @@ int findNeighborsListed(const double* x, const double* y, const double* z, const
     SearchExtras ex{};
     ex.groups    = groups;
     ex.numListed = numListed;
-    if (n <= kManyLanesListed) { SPHB_SEARCH(kSearchListed, kManyLanes, listedBlocks<kManyLanes>(n), h, nidx, nc) }
-    else { SPHB_SEARCH(kSearchListed, 1, listedBlocks<1>(n), h, nidx, nc) }
+    unsigned blocks = std::min(searchBlocks(n, kManyLanes), unsigned(smCount() * residentBlocks<1, false>()));
+    if (views)
+    {
+        findListedKernel<true><<<blocks, kNbThreads, 0, stream>>>(x, y, z, pos, h, n, tree, box, prm, nidx, nc, status,
+                                                                  views, inst, ex);
+    }
+    else
+    {
+        findListedKernel<false><<<blocks, kNbThreads, 0, stream>>>(x, y, z, pos, h, n, tree, box, prm, nidx, nc, status,
+                                                                   nullptr, nullptr, ex);
+    }
     countLaunch();
     SPHB_CUDA_TRY(cudaGetLastError());
     return kOk;

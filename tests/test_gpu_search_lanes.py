@@ -1,5 +1,5 @@
-"""Neighbour searches with one and with four lanes per target: the lists against a k-d tree, and listed searches against
-the full ones, on both sides of the sizes at which the number of lanes changes."""
+"""Neighbour searches with one, four and eight lanes per target: the lists against a k-d tree, and listed searches against
+the full ones, on both sides of the sizes and of the list length at which the number of lanes changes."""
 import numpy as np
 import pytest
 
@@ -11,7 +11,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("precision", ["mixed", "fp64"])
 @pytest.mark.parametrize("n,spread,ngmax", [(9, 1.0, 150), (33, 1.0, 150), (263, 0.5, 150), (4099, 0.3, 150),
-                                            (4100, 0.3, 20), (40_000, 0.3, 150), (40_001, 0.3, 150)])
+                                            (4100, 0.3, 20), (10_000, 0.3, 150), (10_001, 0.3, 150),
+                                            (40_000, 0.3, 150), (40_001, 0.3, 150)])
 def test_lists_match_a_kd_tree(cuda_device, n, spread, ngmax, precision):
     from scipy.spatial import cKDTree
     from sphexa_b200.simulation import Simulation
@@ -50,8 +51,28 @@ def test_lists_match_a_kd_tree(cuda_device, n, spread, ngmax, precision):
         assert over > 0  # truncated lists are among the tested
 
 
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
 @pytest.mark.parametrize("side", [40, 66, 68])
-def test_listed_searches(cuda_device, side):
-    a, b = _pair(_stirred(side, radius=0.15, speed=40.0), "mixed")
+def test_listed_searches(cuda_device, side, precision):
+    a, b = _pair(_stirred(side, radius=0.15, speed=40.0), precision)
     _run(a, b, 4)
     assert a.search_stats()["deferred_groups"] > 0
+
+
+def test_lists_on_both_sides_of_the_limit(cuda_device):
+    """a stirred region that spreads: few of its groups are listed first, then more than those that take eight lanes"""
+    a, b = _pair(_stirred(80, radius=0.173), "mixed")
+    lengths = []
+    for _ in range(7):
+        before = a.search_stats()["deferred_groups"]
+        _run(a, b, 1)
+        lengths.append(a.search_stats()["deferred_groups"] - before)
+    assert any(0 < n <= 1500 for n in lengths) and max(lengths) > 1500, lengths
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("n", [10_000, 10_001, 40_000, 40_001])
+def test_row_builds(cuda_device, n, precision):
+    a, b = _pair(clumps(n, 5, 0.5), precision)
+    _run(a, b, 3)
+    assert a.search_stats()["skin_builds"] >= 1
