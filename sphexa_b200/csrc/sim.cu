@@ -1472,13 +1472,20 @@ extern "C" int sphb_sim_get_field(sphb_sim* s, const char* name, double* out, in
     int src = kind == 0 ? SPHB_F64 : kind == 1 ? (s->mixed ? SPHB_F32 : SPHB_F64) : kind == 2 ? SPHB_U32 : SPHB_U64;
     int dst = src == SPHB_U64 ? SPHB_U64 : SPHB_F64; // keys and ids keep their bits
     size_t bytes = s->n * sizeof(double);
+    bool direct  = false;
     if (on_device)
     {
         // out may still be in use by work on the caller's default stream, which a copy to it would wait for
         SPHB_CUDA_TRY(cudaEventRecord(s->copyFork, cudaStreamLegacy));
         SPHB_CUDA_TRY(cudaStreamWaitEvent(s->stream, s->copyFork, 0));
-        SPHB_TRY(simimpl::convertArray(ptr, src, out, dst, s->n, s->stream));
+        cudaPointerAttributes at{};
+        int device = 0;
+        SPHB_CUDA_TRY(cudaPointerGetAttributes(&at, out));
+        SPHB_CUDA_TRY(cudaGetDevice(&device));
+        if (at.type == cudaMemoryTypeUnregistered) { return SPHB_ERR_ARG; } // a kernel would write there, a copy refuses
+        direct = at.type != cudaMemoryTypeHost && at.device == device;      // not another device's memory
     }
+    if (direct) { SPHB_TRY(simimpl::convertArray(ptr, src, out, dst, s->n, s->stream)); }
     else
     {
         const void* from = ptr;
@@ -1488,7 +1495,7 @@ extern "C" int sphb_sim_get_field(sphb_sim* s, const char* name, double* out, in
             SPHB_TRY(simimpl::convertArray(ptr, src, s->typedStage.data(), dst, s->n, s->stream));
             from = s->typedStage.data();
         }
-        SPHB_CUDA_TRY(cudaMemcpyAsync(out, from, bytes, cudaMemcpyDeviceToHost, s->stream));
+        SPHB_CUDA_TRY(cudaMemcpyAsync(out, from, bytes, on_device ? cudaMemcpyDefault : cudaMemcpyDeviceToHost, s->stream));
     }
     SPHB_CUDA_TRY(cudaStreamSynchronize(s->stream));
     return SPHB_OK;

@@ -282,3 +282,27 @@ def test_step_fields_equals_load_step_store(lib, types, precision):
         assert np.array_equal(a.get(f), b.get(f)), f
     assert a.scalars()["minDt"] == b.scalars()["minDt"]
     assert a.search_stats() == b.search_stats()
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_field_reads_by_the_kind_of_memory(cuda_device, precision):
+    """device memory, pinned and pageable host memory as host memory, pinned memory as device memory; pageable memory as
+    device memory is refused"""
+    import torch
+    from sphexa_b200 import ic as icm
+    from sphexa_b200 import lib as L
+    from sphexa_b200.simulation import Simulation
+    sim = Simulation(icm.sedov(9), precision)
+    sim.compute_forces()
+    for f in ("x", "divv", "nc", "keys"):
+        want = sim.get(f).view(np.float64) if f == "keys" else sim.get(f)
+        got = {"device": torch.zeros(sim.n, dtype=torch.float64, device="cuda"),
+               "pinned": torch.zeros(sim.n, dtype=torch.float64, pin_memory=True),
+               "pinned as device": torch.zeros(sim.n, dtype=torch.float64, pin_memory=True)}
+        for k, a in got.items():
+            on_device = int(k != "pinned")
+            L.check(sim.lib.sphb_sim_get_field(sim.h, f.encode(), a.data_ptr(), on_device), k)
+            assert np.array_equal(a.cpu().numpy().view(np.uint64), want.view(np.uint64)), (f, k)
+        pageable = np.zeros(sim.n)
+        assert sim.lib.sphb_sim_get_field(sim.h, f.encode(), pageable.ctypes.data, 1) == L.SPHB_ERR_ARG
+        assert not pageable.any()
