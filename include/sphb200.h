@@ -504,7 +504,9 @@ int sphb_ensemble_create(sphb_ensemble** ens, int num, const size_t* sizes, cons
 
 int sphb_ensemble_destroy(sphb_ensemble* ens);
 
-/*! The 14 conserved fields and ids of instance k (as sphb_sim_upload). */
+/*! The 14 conserved fields and ids of instance k (arrays as for sphb_sim_upload). The instance's time, time step and
+ *  previous time step stay what they are: those of its parameters after sphb_ensemble_create, those of the last step after
+ *  steps. */
 int sphb_ensemble_upload(sphb_ensemble* ens, int k, const double* const* fields, const uint64_t* id, int on_device);
 
 /*! Sort every instance into SFC order and build its trees (host-driven; after all uploads). */

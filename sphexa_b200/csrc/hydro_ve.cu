@@ -3,9 +3,10 @@
 // neighbour lists are read slot-major (one coalesced line per slot). Each J-loop walks the list in stored (ascending)
 // order, like the reference CPU loops, and reads neighbour data through the packed records of hydro.cuh.
 //
-// T = double: the plain FP64 drop-in. Positions are FP64, the periodic shift is the reference's and sums run in list
-// order. The pair terms are the reference's up to algebra that keeps FP64 rounding (a reciprocal for a division, a
-// constant factor taken out of a sum), so results differ from the reference CPU by rounding, 1e-15 of a force.
+// T = double: the plain FP64 drop-in. Positions are FP64 and the periodic shift is the reference's. Sums run over blocks of
+// 8 neighbours in list order, whose partial sums are added in list order. The pair terms are the reference's up to
+// algebra that keeps FP64 rounding (a reciprocal for a division, a constant factor taken out of a sum), so results differ
+// from the reference CPU by rounding, 1e-15 of a force.
 //
 // T = float: the mixed form. Pair separations come from 32-bit fixed-point coordinates (exact integer differences,
 // periodic wrap by overflow; one unit = L / 2^32), all pair arithmetic is FP32, the kernel W is a degree-12

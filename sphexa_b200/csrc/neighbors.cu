@@ -39,7 +39,7 @@ constexpr int kLeafCap   = 256; // candidate leaves buffered before they are str
  *  99 and 108, 30^3 FP64 103 and 117; with one and four, before the traversal took four nodes a round: 30^3 167 and 122,
  *  50^3 327 and 426, 63^3 394 and 579.
  *  Searches of listed groups, a small part of all, choose by the length of the list, which only the device knows. Neighbour
- *  phase with one lane, with eight, and with eight for lists of up to 1,500 groups (the same up to 100 either way): block
+ *  phase with one lane, with eight, and with eight for lists of up to 1,500 groups (1,350 to 1,700 do the same): block
  *  time steps of 64^3 334, 248 and 248, 81^3 414, 300 and 301, 90^3 378, 496 and 388, 100^3 468, 609 and 476, 100^3 with a
  *  wide blast 757, 1480 and 760, global steps of 128^3 934, 1193 and 935. */
 constexpr int kFewLanes             = 4;

@@ -984,8 +984,9 @@ int focusUpdateCounts(FocusTree& f, const uint64_t* keys, size_t n, cudaStream_t
 // p is then on level D_p = max(E_p, min(D_{p-1}, c_p)), and functions x -> max(e, min(x, c)) compose, so D is a scan. The
 // leaf of key p is on level D_p + 1, it starts at p if c_p <= D_p, and the empty leaves between two keys' leaves are the
 // children that the paths between them pass by. A second scan, of the leaves that each key opens, places them.
-// Two reads of the keys and one host read, instead of a rebalance, a scan, a recount and a host read for every few
-// levels, with buffers that grew in between: 150,000 leaves of 4,000,037 clustered keys 2.6 -> 0.2 ms.
+// Three sweeps over the keys, a search per leaf boundary for the counts and one host read, instead of a rebalance, a
+// scan, a recount and a host read for every few levels, with buffers that grew in between: 150,000 leaves of 4,000,037
+// clustered keys 2.6 -> 0.2 ms.
 // ------------------------------------------------------------------------------------------------------------------
 namespace sphb
 {

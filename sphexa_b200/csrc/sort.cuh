@@ -41,8 +41,8 @@ struct LeafSortScratch
 /*! The same stable sort (values = 0..n-1 first) with the help of a cornerstone leaf array that held few keys per leaf
  *  for keys close to these, the tree of the previous step: every key finds its leaf, a scan of the leaf counts places
  *  the leaves, and one warp sorts each leaf, a block one of more than 128 keys. One host read, of whether anything is out
- *  of order and whether a leaf grew past 2,048 keys (then the radix sort runs, in place). It reads and writes the keys twice whatever the particles'
- *  motion is, where the radix sort takes eight passes. */
+ *  of order and whether a leaf grew past 2,048 keys (then the radix sort runs, in place). It reads and writes the keys
+ *  twice whatever the particles' motion is, where the radix sort takes four passes of that, eight if the keys crowd. */
 int sortByLeaves(uint64_t* keys, uint64_t* keysOut, uint32_t* values, size_t n, const uint64_t* leaves, int numLeaves,
                  LeafSortScratch& ls, void* scratch, size_t scratchBytes, LeafSort* result, cudaStream_t stream);
 

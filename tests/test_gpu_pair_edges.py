@@ -35,9 +35,10 @@ def contrast(side, keep=None, coincident=0, seed=5):
 
 @pytest.mark.parametrize("side,keep,coincident", [(8, None, 0), (8, 481, 0), (9, 720, 3), (13, 2177, 0), (13, None, 5)])
 def test_fp64_forces_against_the_restatement(cuda_device, side, keep, coincident):
-    """One force computation against the C restatement. Both sum the same terms in the same order; a term's rounding
-    differs by a few 1e-16 (reciprocals for divisions), the sums' by sqrt(100) of that, and divv, curlv, du and the
-    accelerations are differences of larger terms: 1e-12 of a field's largest magnitude leaves a factor 100."""
+    """One force computation against the C restatement, which sums neighbour by neighbour; the pair loops sum eight at a
+    time and add the partial sums. A term's rounding differs by a few 1e-16 (reciprocals for divisions). Either order of
+    100 additions is off by at most sqrt(100) of that for rounding errors that are independent, and divv, curlv, du and
+    the accelerations are differences of larger terms: 1e-12 of a field's largest magnitude leaves a factor 100."""
     from oracle import restated
     from sphexa_b200.simulation import Simulation
     ic = contrast(side, keep, coincident)
