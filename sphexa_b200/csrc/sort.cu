@@ -74,12 +74,12 @@ constexpr int kHistThreads = 1024;
 constexpr int kSamples     = 4096;
 constexpr int kSampleSlots = 2 * kSamples;
 
-/*! *verdict = 1 if many keys probably lie in runs that no block sorts, else 0: counts the samples (spread evenly,
+/*! *crowded = 1 if many keys probably lie in runs that no block sorts, else 0: counts the samples (spread evenly,
  *  up to kSamples) that agree in the upper digits with an earlier, different one. A hash table holds 8 bits of a fingerprint, the
  *  first sample and the count of each. A run of kRunBlockCap keys holds kRunBlockCap samples / n of them; three of spread
  *  keys hardly ever agree. Equal keys, which are in order, do not count. The upper digits are the kUpperPasses highest
  *  ones in which the samples differ. By one block of kHistThreads. */
-__device__ void sampleRuns(const uint64_t* __restrict__ keys, size_t n, uint32_t* slots, uint32_t* verdict)
+__device__ void sampleRuns(const uint64_t* __restrict__ keys, size_t n, uint32_t* slots, uint32_t* crowded)
 {
     __shared__ uint32_t differ; // the digits in which the samples differ
     if (threadIdx.x == 0) { differ = 0; }
@@ -140,22 +140,22 @@ __device__ void sampleRuns(const uint64_t* __restrict__ keys, size_t n, uint32_t
         }
     }
     bool many = __syncthreads_or(most >= limit);
-    if (threadIdx.x == 0) { *verdict = many ? 1u : 0u; }
+    if (threadIdx.x == 0) { *crowded = many ? 1u : 0u; }
 }
 
-//! digit histograms of all 8 byte positions in one sweep over the keys; with verdict set, the first block takes a sample
+//! digit histograms of all 8 byte positions in one sweep over the keys; with crowded set, the first block takes a sample
 //! instead (sampleRuns), which costs nothing beside the sweep
 __global__ void __launch_bounds__(kHistThreads) histogramKernel(const uint64_t* __restrict__ keys, size_t n,
                                                                 uint32_t* __restrict__ hist, const uint32_t* gate,
-                                                                uint32_t* verdict = nullptr)
+                                                                uint32_t* crowded = nullptr)
 {
     if (gate && *gate == 0) { return; }
     __shared__ uint32_t sh[kSampleSlots];
-    const unsigned blocks = verdict ? gridDim.x - 1 : gridDim.x;
-    const unsigned block  = verdict ? blockIdx.x - 1 : blockIdx.x;
-    if (verdict && blockIdx.x == 0)
+    const unsigned blocks = crowded ? gridDim.x - 1 : gridDim.x;
+    const unsigned block  = crowded ? blockIdx.x - 1 : blockIdx.x;
+    if (crowded && blockIdx.x == 0)
     {
-        sampleRuns(keys, n, sh, verdict);
+        sampleRuns(keys, n, sh, crowded);
         return;
     }
     for (int t = threadIdx.x; t < kPasses * kRadix; t += kHistThreads)
@@ -630,7 +630,7 @@ int sortByKey(uint64_t* keys, uint32_t* values, size_t n, bool initValues, void*
                                                                                 sample ? s.status : nullptr);
     SPHB_CUDA_TRY(cudaGetLastError());
 
-    // decide on the host which passes are trivial (one digit holds every key); the word behind is the sample's verdict
+    // decide on the host which passes are trivial (one digit holds every key); the word behind tells the sample's finding
     uint32_t h[kPasses * kRadix + 1];
     SPHB_CUDA_TRY(cudaMemcpyAsync(h, s.hist, sizeof(h), cudaMemcpyDeviceToHost, stream));
     SPHB_CUDA_TRY(cudaStreamSynchronize(stream));
